@@ -86,6 +86,12 @@ EXPORTS = {
                                    c_void_p, c_size_t, c_void_p]),
     "cobalt_linear_host_async": (c_int, [POINTER(CobaltMat), c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p,
                                    c_void_p, c_size_t, c_void_p]),
+    "cobalt_compress_state_bytes": (c_size_t, []),
+    "cobalt_score_rows": (c_int, [c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_int, c_uint32, c_void_p, c_void_p, c_void_p, c_void_p]),
+    "cobalt_keep_from_scores": (c_int, [c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p]),
+    "cobalt_quantize_groups": (c_int, [c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p]),
+    "cobalt_pack_plan": (c_int, [c_void_p, c_void_p, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p]),
+    "cobalt_pack_tiles": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p]),
     "cobalt_add_rmsnorm": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_float, c_int, c_void_p,
                                    c_void_p]),
     "cobalt_rope_kv": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int,

@@ -13,8 +13,8 @@ import sys
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libcobalt_b200.so")
-SOURCES = ["cobalt_abi.cu"]
-HEADERS = ["common.cuh", "decode_core.cuh", "walk_kernels.cuh", "gemv_kernel.cuh", "gemm_kernel.cuh", "glue_kernels.cuh", "staged_input.cuh",
+SOURCES = ["cobalt_abi.cu", "compress_abi.cu"]
+HEADERS = ["common.cuh", "decode_core.cuh", "walk_kernels.cuh", "gemv_kernel.cuh", "gemm_kernel.cuh", "glue_kernels.cuh", "staged_input.cuh", "compress_kernels.cuh",
            os.path.join("..", "..", "include", "cobalt_b200.h")]
 
 
@@ -38,7 +38,7 @@ def build(force: bool = False, verbose: bool = False) -> str:
     if not force and not needs_build():
         return LIB
     cmd = [_nvcc(), "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
-           "--expt-relaxed-constexpr", "-shared", "-Xcompiler", "-fPIC",
+           "--expt-relaxed-constexpr", "--threads", "0", "-shared", "-Xcompiler", "-fPIC",
            "-o", LIB] + [os.path.join(CSRC, s) for s in SOURCES]
     if verbose:
         cmd.insert(1, "-Xptxas")

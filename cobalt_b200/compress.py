@@ -19,6 +19,7 @@ from dataclasses import dataclass
 
 import torch
 
+from . import _lib
 from .format import GROUP
 
 
@@ -66,11 +67,51 @@ def _global_kth_smallest(flat: torch.Tensor, k: int) -> torch.Tensor:
     return below.max() if below.numel() else hi
 
 
+_W_TYPES = {torch.float32: 0, torch.float16: 1, torch.bfloat16: 2}
+
+
+def _dense_for_kernel(weight: torch.Tensor) -> torch.Tensor:
+    """``weight`` as the compression kernels read it: contiguous, 16-byte aligned, fp32 / fp16 / bf16 (same values)."""
+    w = weight if weight.dtype in _W_TYPES else weight.float()
+    w = w.contiguous()
+    return w if w.data_ptr() % 16 == 0 else w.clone()
+
+
+def _keep_mask_cuda(weight: torch.Tensor, act_norm: torch.Tensor, sparsity: float, beta: float) -> torch.Tensor:
+    """``keep_mask`` in CUDA kernels (csrc/compress_kernels.cuh), equal bit for bit: torch's kthvalue works a single slice with
+    a single thread block, which for the global threshold of a 4096 x 4096 matrix takes 96 ms."""
+    K, N = weight.shape
+    n_row, n_col, k = int(N * sparsity), int(K * sparsity), int(K * N * sparsity)
+    if beta <= 0:
+        n_col = 0
+    lib = _lib.load()
+    with torch.cuda.device(weight.device):
+        w = _dense_for_kernel(weight)
+        norm = act_norm.float().reshape(-1).contiguous()
+        if norm.data_ptr() % 16:
+            norm = norm.clone()
+        scores = torch.empty(K, N, dtype=torch.float32, device=w.device)
+        col_kth = torch.empty(N, dtype=torch.float32, device=w.device) if n_col else None
+        state = torch.empty(lib.cobalt_compress_state_bytes(), dtype=torch.uint8, device=w.device)
+        keep = torch.empty(K, N, dtype=torch.uint8, device=w.device)
+        stream = torch.cuda.current_stream().cuda_stream
+        _lib.check("cobalt_score_rows", lib.cobalt_score_rows(
+            w.data_ptr(), _W_TYPES[w.dtype], norm.data_ptr(), K, N, n_row, n_col, k, scores.data_ptr(),
+            None if col_kth is None else col_kth.data_ptr(), state.data_ptr(), stream))
+        div = None if col_kth is None else col_kth.clamp(min=1e-30).pow(beta)
+        _lib.check("cobalt_keep_from_scores", lib.cobalt_keep_from_scores(
+            scores.data_ptr(), None if div is None else div.data_ptr(), K, N, int(n_row > 0), int(K * N > 32_000_000),
+            state.data_ptr(), keep.data_ptr(), stream))
+    return keep.view(torch.bool)
+
+
 def keep_mask(weight: torch.Tensor, act_norm: torch.Tensor, sparsity: float, beta: float) -> torch.Tensor:
     """bool ``[K, N]`` keep mask (True = survivor)."""
     K, N = weight.shape
     if sparsity <= 0.0:
         return torch.ones(K, N, dtype=torch.bool, device=weight.device)
+    if weight.is_cuda and act_norm.is_cuda and N % GROUP == 0 and act_norm.numel() == N and int(K * N * sparsity) >= 1:
+        return _keep_mask_cuda(weight, act_norm, sparsity, beta)
     score = weight.float().abs() * act_norm.float().view(1, -1)
     n_row, n_col = int(N * sparsity), int(K * sparsity)
     if n_row > 0:
@@ -91,6 +132,18 @@ def quantize_survivors(weight: torch.Tensor, keep: torch.Tensor, bits: int, grou
     if N % group_size:
         raise ValueError(f"in_features {N} is not a multiple of group_size {group_size}")
     G = N // group_size
+    if weight.is_cuda and keep.is_cuda and keep.dtype == torch.bool and keep.shape == weight.shape and group_size == GROUP:
+        lib = _lib.load()
+        with torch.cuda.device(weight.device):
+            w, kb = _dense_for_kernel(weight), keep.contiguous()
+            if kb.data_ptr() % 16:
+                kb = kb.clone()
+            q = torch.empty(K, N, dtype=torch.uint8, device=w.device)
+            scale, zero = (torch.empty(K, G, dtype=torch.float16, device=w.device) for _ in range(2))
+            _lib.check("cobalt_quantize_groups", lib.cobalt_quantize_groups(
+                w.data_ptr(), _W_TYPES[w.dtype], kb.data_ptr(), K, N, bits, q.data_ptr(), scale.data_ptr(), zero.data_ptr(),
+                torch.cuda.current_stream().cuda_stream))
+        return q, scale, zero
     top_code = (1 << bits) - 1
     wg = weight.float().view(K, G, group_size)
     kg = keep.view(K, G, group_size)

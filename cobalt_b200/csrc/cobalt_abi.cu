@@ -651,7 +651,7 @@ int cobalt_dequant(const CobaltMat* w, void* w_bf16, void* stream) {
     rc = device_info(&sms);
     if (rc) return rc;
     MatView V = make_view(w);
-    unpack_kernel<<<dim3(V.CT, V.RB), 64, 0, (cudaStream_t)stream>>>(V, nullptr, nullptr, (uint16_t*)w_bf16);
+    unpack_kernel<<<dim3(V.CT, V.RB), UNPACK_THREADS, 0, (cudaStream_t)stream>>>(V, nullptr, nullptr, (uint16_t*)w_bf16, ((uintptr_t)w_bf16 & 7) == 0);
     return cudaGetLastError() == cudaSuccess ? COBALT_OK : COBALT_ELAUNCH;
 }
 
@@ -663,7 +663,7 @@ int cobalt_unpack(const CobaltMat* w, uint8_t* codes, uint8_t* keep, void* strea
     rc = device_info(&sms);
     if (rc) return rc;
     MatView V = make_view(w);
-    unpack_kernel<<<dim3(V.CT, V.RB), 64, 0, (cudaStream_t)stream>>>(V, codes, keep, nullptr);
+    unpack_kernel<<<dim3(V.CT, V.RB), UNPACK_THREADS, 0, (cudaStream_t)stream>>>(V, codes, keep, nullptr, (((uintptr_t)codes | (uintptr_t)keep) & 3) == 0);
     return cudaGetLastError() == cudaSuccess ? COBALT_OK : COBALT_ELAUNCH;
 }
 

@@ -41,33 +41,74 @@ __device__ __forceinline__ SegCtx open_segment(const MatView& W, int rb, int ct,
     return c;
 }
 
-// codes u8[K,N] (0 at pruned), keep u8[K,N], dense bf16[K,N]; any output may be null
-__global__ void __launch_bounds__(64) unpack_kernel(MatView W, uint8_t* codes, uint8_t* keep, uint16_t* dense) {
-    __shared__ uint32_t sh_cnt[64];
-    const int ct = blockIdx.x, rb = blockIdx.y;
-    SegCtx c = open_segment(W, rb, ct, sh_cnt);
-    const int r = threadIdx.x >> 2, gi = threadIdx.x & 3;
-    const int row = rb * TILE_ROWS + r;
-    if (!c.active || row >= W.K) return;
-    const int col0 = (ct * TILE_GROUPS + gi) * GROUP;
-    const float s = half_bits_to_float(c.sz & 0xFFFFu), z = half_bits_to_float(c.sz >> 16);
-    uint32_t bitpos = c.first * (uint32_t)W.bits;
-    for (int j = 0; j < 4; ++j) {
-        const uint32_t m = c.mask[j];
-        for (int b = 0; b < 32; ++b) {
-            const int col = col0 + 32 * j + b;
-            const uint32_t kept = (m >> b) & 1u;
-            uint32_t code = 0;
-            if (kept) { code = extract_code(c.stream, bitpos, W.bits); bitpos += W.bits; }
-            const size_t o = (size_t)row * W.N + col;
-            if (codes) codes[o] = (uint8_t)code;
-            if (keep) keep[o] = (uint8_t)kept;
-            if (dense) {
-                const float cs = W.col_scale ? half_bits_to_float(W.col_scale[col]) : 1.0f;
-                // literal reference order: ((q - z) * s) * col_scale, then * keep, then one cast
-                dense[o] = float_to_bf16(__fmul_rn(dequant_fp32((float)code, z, s, cs), (float)kept));
+// codes u8[K,N] (0 at pruned), keep u8[K,N], dense bf16[K,N]; any output may be null.
+// One block of 8 warps per tile, a warp per segment, a lane per four columns: a warp writes whole 128-byte lines (256 for the
+// dense weight), which is what bounds it.  4096 x 4096: 31 us; a thread per segment with byte stores took 223.
+constexpr int UNPACK_THREADS = 256;
+__global__ void __launch_bounds__(UNPACK_THREADS) unpack_kernel(MatView W, uint8_t* codes, uint8_t* keep, uint16_t* dense, int wide) {
+    __shared__ uint32_t first_s[TILE_ROWS * TILE_GROUPS];
+    const int ct = blockIdx.x, rb = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int w = tile_width(W, ct), nseg = TILE_ROWS * w;
+    const uint8_t* tile = W.tiles + (size_t)W.tile_off[(size_t)rb * W.CT + ct] * 16;
+    if (warp == 0) {                                                   // rank of every segment's first survivor, two segments per lane
+        uint32_t c[2];
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+            c[k] = 0;
+            if (2 * lane + k < nseg) {
+                const uint4 m = __ldg(reinterpret_cast<const uint4*>(tile) + 2 * lane + k);
+                c[k] = __popc(m.x) + __popc(m.y) + __popc(m.z) + __popc(m.w);
             }
         }
+        uint32_t inc = c[0] + c[1];
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) { const uint32_t up = __shfl_up_sync(0xFFFFFFFFu, inc, d); if (lane >= d) inc += up; }
+        first_s[2 * lane] = inc - c[0] - c[1];
+        first_s[2 * lane + 1] = inc - c[1];
+    }
+    __syncthreads();
+    const uint32_t* stream = reinterpret_cast<const uint32_t*>(tile + nseg * 20);
+    for (int seg = warp; seg < nseg; seg += UNPACK_THREADS / 32) {
+        const int row = rb * TILE_ROWS + seg / w;
+        if (row >= W.K) continue;
+        const int col = (ct * TILE_GROUPS + seg % w) * GROUP + 4 * lane;
+        const uint4 m = __ldg(reinterpret_cast<const uint4*>(tile) + seg);
+        const uint32_t sz = __ldg(reinterpret_cast<const uint32_t*>(tile + nseg * 16) + seg);
+        const int j = lane >> 3, sh = 4 * (lane & 7);
+        const uint32_t mj = j == 0 ? m.x : j == 1 ? m.y : j == 2 ? m.z : m.w;
+        uint32_t rank = first_s[seg] + __popc(mj & ((1u << sh) - 1u));
+        if (j > 0) rank += __popc(m.x);
+        if (j > 1) rank += __popc(m.y);
+        if (j > 2) rank += __popc(m.z);
+        const uint32_t nib = (mj >> sh) & 15u, bit = rank * (uint32_t)W.bits, cmask = (1u << W.bits) - 1u;
+        uint32_t v = funnel_r(__ldg(stream + (bit >> 5)), __ldg(stream + (bit >> 5) + 1), bit);       // the image ends in slack words
+        const float s = half_bits_to_float(sz & 0xFFFFu), z = half_bits_to_float(sz >> 16);
+        uint32_t code4 = 0, keep4 = 0, d[4];
+#pragma unroll
+        for (int b = 0; b < 4; ++b) {
+            const uint32_t kept = (nib >> b) & 1u, code = kept ? v & cmask : 0u;
+            if (kept) v >>= W.bits;
+            code4 |= code << (8 * b);
+            keep4 |= kept << (8 * b);
+            if (dense) {
+                const float cs = W.col_scale ? half_bits_to_float(W.col_scale[col + b]) : 1.0f;
+                // literal reference order: ((q - z) * s) * col_scale, then * keep, then one cast
+                d[b] = float_to_bf16(__fmul_rn(dequant_fp32((float)code, z, s, cs), (float)kept));
+            }
+        }
+        const size_t o = (size_t)row * W.N + col;
+        if (!wide) {                                                   // outputs at odd addresses: one element at a time
+#pragma unroll
+            for (int b = 0; b < 4; ++b) {
+                if (codes) codes[o + b] = (uint8_t)(code4 >> (8 * b));
+                if (keep) keep[o + b] = (uint8_t)(keep4 >> (8 * b));
+                if (dense) dense[o + b] = (uint16_t)d[b];
+            }
+            continue;
+        }
+        if (codes) *reinterpret_cast<uint32_t*>(codes + o) = code4;
+        if (keep) *reinterpret_cast<uint32_t*>(keep + o) = keep4;
+        if (dense) *reinterpret_cast<uint2*>(dense + o) = make_uint2(d[0] | (d[1] << 16), d[2] | (d[3] << 16));
     }
 }
 

@@ -24,9 +24,12 @@ runs on whatever device the inputs live on.
 """
 from __future__ import annotations
 
+import struct
 from dataclasses import dataclass
 
 import torch
+
+from . import _lib
 
 GROUP = 128
 TILE_ROWS = 16
@@ -94,6 +97,8 @@ def pack_tiles(keep: torch.Tensor, q: torch.Tensor, scale: torch.Tensor, zero: t
     CT = (G + TILE_GROUPS - 1) // TILE_GROUPS
     Kp, Gp = RB * TILE_ROWS, CT * TILE_GROUPS
 
+    if keep.is_cuda and q.is_cuda and q.shape == keep.shape and RB <= 65535:         # row blocks are a grid dimension there
+        return _pack_tiles_cuda(keep, q, scale.reshape(K, G), zero.reshape(K, G), bits)
     keep_b = keep != 0
     qi = q.to(torch.int64)
     if bool(((qi < 0) | (qi >= (1 << bits)))[keep_b].any()):
@@ -177,6 +182,49 @@ def pack_tiles(keep: torch.Tensor, q: torch.Tensor, scale: torch.Tensor, zero: t
     return TileImage(blob=blob8, K=K, N=N, bits=bits, nnz=nnz, n_row_blocks=RB, n_col_tiles=CT,
                      header_bytes=header_bytes, max_tile_bytes=int(tb_flat.max()),
                      max_tile_nnz=int(nnz_tile.max()))
+
+
+def _pack_tiles_cuda(keep: torch.Tensor, q: torch.Tensor, scale: torch.Tensor, zero: torch.Tensor, bits: int) -> TileImage:
+    """``pack_tiles`` in CUDA kernels (csrc/compress_kernels.cuh), byte for byte the same image.  One synchronisation: the size of
+    the image depends on the mask."""
+    K, N = keep.shape
+    dev = keep.device
+    RB = (K + TILE_ROWS - 1) // TILE_ROWS
+    CT = (N // GROUP + TILE_GROUPS - 1) // TILE_GROUPS
+    n_tiles = RB * CT
+    header_bytes = _round_up(4 * (n_tiles + 1), HEADER_ALIGN)
+    lib = _lib.load()
+
+    def ready(t):
+        t = t.contiguous()
+        return t if t.data_ptr() % 16 == 0 else t.clone()
+
+    with torch.cuda.device(dev):
+        kb = ready(keep if keep.dtype in (torch.bool, torch.uint8) else keep != 0)
+        if q.dtype != torch.uint8:
+            qi = q.to(torch.int64)
+            if bool(((qi < 0) | (qi >= (1 << bits)))[keep != 0].any()):
+                raise ValueError("code outside [0, 2**bits) at a surviving position")
+            q = qi.to(torch.uint8)
+        qb, sc, zr = ready(q), scale.to(device=dev, dtype=torch.float16).contiguous(), zero.to(device=dev, dtype=torch.float16).contiguous()
+        stream = torch.cuda.current_stream().cuda_stream
+        plan = torch.empty(2 * n_tiles + 1, dtype=torch.int32, device=dev)           # survivors per tile, then the offsets
+        info = torch.empty(24, dtype=torch.uint8, device=dev)
+        off = plan[n_tiles:]
+        _lib.check("cobalt_pack_plan", lib.cobalt_pack_plan(kb.data_ptr(), qb.data_ptr(), K, N, bits, plan.data_ptr(), off.data_ptr(),
+                                                            info.data_ptr(), stream))
+        nnz, total16, max_bytes, max_nnz, bad = struct.unpack("<QIIII", info.cpu().numpy().tobytes())
+        if bad:
+            raise ValueError("code outside [0, 2**bits) at a surviving position")
+        end = header_bytes + total16 * 16
+        blob = torch.empty(end + TAIL_SLACK, dtype=torch.uint8, device=dev)
+        blob[: 4 * (n_tiles + 1)] = off.view(torch.uint8)
+        blob[4 * (n_tiles + 1): header_bytes] = 0
+        blob[end:] = 0
+        _lib.check("cobalt_pack_tiles", lib.cobalt_pack_tiles(kb.data_ptr(), qb.data_ptr(), sc.data_ptr(), zr.data_ptr(), K, N, bits,
+                                                              off.data_ptr(), blob.data_ptr() + header_bytes, stream))
+    return TileImage(blob=blob, K=K, N=N, bits=bits, nnz=nnz, n_row_blocks=RB, n_col_tiles=CT, header_bytes=header_bytes,
+                     max_tile_bytes=max_bytes, max_tile_nnz=max_nnz)
 
 
 def bytes_to_keep(mask_u8: torch.Tensor, N: int) -> torch.Tensor:

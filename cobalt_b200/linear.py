@@ -218,7 +218,7 @@ class CobaltSparseLinear(nn.Module):
         rc = lib.cobalt_unpack(ctypes.byref(self._descriptor()), codes.data_ptr(), keep.data_ptr(),
                                torch.cuda.current_stream(dev).cuda_stream)
         _lib.check("cobalt_unpack", rc)
-        return codes, keep.bool()
+        return codes, keep.view(torch.bool)                  # the kernel writes 0 and 1
 
     def device_status(self) -> int:
         """Status word of the last kernels that used this module's scratch buffer (0 = healthy)."""

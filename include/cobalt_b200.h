@@ -239,6 +239,33 @@ int cobalt_linear_host_async(const CobaltMat* w, const void* x_host, void* y_hos
 int cobalt_gemv_fused_host_async(int n_mats, const CobaltMat* const* w, const void* x_host, void* const* y_host, int M,
                                  void* dev_x, void* const* dev_y, void* scratch, size_t scratch_bytes, void* stream);
 
+/* Compression of a dense weight on the GPU (cobalt_b200/compress.py and format.py drive these; every result equals their torch
+ * form bit for bit; reference: src/cobaltkernel/cobalt_math.py:15-32, 144-168).  W [K, N] row-major, w_type 0 fp32 / 1 fp16 /
+ * 2 bf16, 16-byte aligned; N % 128 == 0, K * N < 2^34.
+ *   cobalt_score_rows        : scores [K, N] fp32 = |W| * norm, with n_row > 0 over the row's n_row-th smallest; with n_col > 0
+ *                              also col_kth [N] = the n_col-th smallest of every column (after the division by the maximum).
+ *                              `state` (cobalt_compress_state_bytes()) carries what the next call needs; k_keep = the number of
+ *                              positions to prune.
+ *   cobalt_keep_from_scores  : scores over col_div [N] (NULL: no column step), then keep [K, N] u8 = score > k_keep-th smallest;
+ *                              bracketed = the reference's bisection for matrices above 32 M elements.  Consumes `scores`.
+ *   cobalt_quantize_groups   : asymmetric min-max rounding of the survivors per 128-wide group: q u8 [K, N] (0 where pruned),
+ *                              scale and zero fp16 [K, N / 128].
+ *   cobalt_pack_plan         : tile_off [tiles + 1] of the tile image and, in `info`, { u64 survivors, u32 image size in 16-byte
+ *                              units, u32 largest tile in bytes, u32 largest survivor count of a tile, u32 1 if a surviving code
+ *                              does not fit `bits` }.  tile_nnz: u32 [tiles] of work space.
+ *   cobalt_pack_tiles        : the tiles (16-byte aligned, cleared by nobody: every byte of a tile is written). */
+size_t cobalt_compress_state_bytes(void);
+int cobalt_score_rows(const void* W, int w_type, const float* norm, int K, int N, int n_row, int n_col, uint32_t k_keep, float* scores,
+                      float* col_kth, void* state, void* stream);
+int cobalt_keep_from_scores(float* scores, const float* col_div, int K, int N, int rows_normalised, int bracketed, void* state,
+                            uint8_t* keep, void* stream);
+int cobalt_quantize_groups(const void* W, int w_type, const uint8_t* keep, int K, int N, int bits, uint8_t* q, void* scale, void* zero,
+                           void* stream);
+int cobalt_pack_plan(const uint8_t* keep, const uint8_t* q, int K, int N, int bits, uint32_t* tile_nnz, uint32_t* tile_off, void* info,
+                     void* stream);
+int cobalt_pack_tiles(const uint8_t* keep, const uint8_t* q, const void* scale, const void* zero, int K, int N, int bits,
+                      const uint32_t* tile_off, void* tiles, void* stream);
+
 /* Fused element-wise steps of a decoder block around the linears, with the dtype policy of the
  * reference's executable specs (src/cobaltkernel/ref_llama.py:82-97, 139-143; src/cobaltkernel/ref_gemma3.py:138-143,
  * 173-174, 225-228; in the reference they are phases of its megakernel: src/cobaltkernel/csrc/megakernel.cu:270-288,
