@@ -15,6 +15,7 @@ CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libcobalt_b200.so")
 SOURCES = ["cobalt_abi.cu", "compress_abi.cu"]
 HEADERS = ["common.cuh", "decode_core.cuh", "walk_kernels.cuh", "gemv_kernel.cuh", "gemm_kernel.cuh", "glue_kernels.cuh", "staged_input.cuh", "compress_kernels.cuh",
+           "prompt_attn.cuh",
            os.path.join("..", "..", "include", "cobalt_b200.h")]
 
 

@@ -9,6 +9,7 @@
 #include "gemv_kernel.cuh"
 #include "gemm_kernel.cuh"
 #include "glue_kernels.cuh"
+#include "prompt_attn.cuh"
 
 using namespace cb;
 
@@ -247,6 +248,32 @@ int launch_gemm(const GemmParams& P, const CUtensorMap& xmap, const GemmCfg& c, 
         configured[dev] = true;
     }
     gemm_tcgen05_kernel<BITS><<<c.grid, GEMM_THREADS, GEMM_SMEM_BYTES, st>>>(P, xmap);
+    return cudaGetLastError() == cudaSuccess ? COBALT_OK : COBALT_ELAUNCH;
+}
+
+// bf16 tensor of three dimensions, box 64 elements wide (one 128-byte swizzle row)
+int make_map_3d(CUtensorMap* map, const void* p, const cuuint64_t* dim, const cuuint64_t* stride, const cuuint32_t* box) {
+    TensorMapEncodeFn enc = tensor_map_encoder();
+    if (!enc) return COBALT_ELAUNCH;
+    const cuuint32_t estr[3] = {1, 1, 1};
+    CUresult r = enc(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(p), dim, stride, box, estr,
+                     CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                     CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    return r == CUDA_SUCCESS ? COBALT_OK : COBALT_EINVAL;
+}
+
+template <int D>
+int launch_prompt_attn(const PromptAttnParams& P, unsigned ctas, const CUtensorMap& qm, const CUtensorMap& km, const CUtensorMap& vm,
+                       cudaStream_t st) {
+    static bool configured[MAX_DEVICES];
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (!configured[dev]) {
+        if (cudaFuncSetAttribute(prompt_attn_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pa_smem_bytes(D)) != cudaSuccess)
+            return COBALT_ELAUNCH;
+        configured[dev] = true;
+    }
+    prompt_attn_kernel<D><<<ctas, PA_THREADS, pa_smem_bytes(D), st>>>(P, qm, km, vm);
     return cudaGetLastError() == cudaSuccess ? COBALT_OK : COBALT_ELAUNCH;
 }
 
@@ -867,6 +894,39 @@ int cobalt_attn_decode_fused(const void* q, const void* k_cache, const void* v_c
     const dim3 grid((unsigned)chunks, (unsigned)n_kv_heads, (unsigned)n_seq);
     return cudaLaunchCooperativeKernel((const void*)attn_decode_fused_kernel, grid, dim3(ATTN_THREADS), args, 0, (cudaStream_t)stream) == cudaSuccess
                ? COBALT_OK : COBALT_ELAUNCH;
+}
+
+int cobalt_attn_prompt(const void* q, const void* k_cache, const void* v_cache, const int64_t* positions, void* out, int T,
+                       int n_heads, int n_kv_heads, int head_dim, int n_slots, int max_ctx, int window, float scale, void* status,
+                       void* stream) {
+    if (!q || !k_cache || !v_cache || !positions || !out || T <= 0) return COBALT_EINVAL;
+    if (n_heads <= 0 || n_kv_heads <= 0 || n_heads % n_kv_heads != 0) return COBALT_EINVAL;
+    if (n_slots <= 0 || n_slots > max_ctx || max_ctx > (1 << 24) || window < 0) return COBALT_EINVAL;
+    if (((uintptr_t)q | (uintptr_t)k_cache | (uintptr_t)v_cache | (uintptr_t)out) & 15) return COBALT_EINVAL;
+    const int rep = n_heads / n_kv_heads;
+    if ((head_dim != 64 && head_dim != 128) || rep > PA_ROWS) return COBALT_EUNSUPPORTED;
+    int sms = 0;
+    int rc = device_info(&sms);
+    if (rc) return rc;
+    PromptAttnParams P;
+    P.positions = (const long long*)positions;
+    P.out = (uint16_t*)out;
+    P.T = T; P.n_kv = n_kv_heads; P.rep = rep; P.tok_per_cta = PA_ROWS / rep; P.S = n_slots; P.window = window;
+    P.scale = scale;
+    P.status = (uint32_t*)status;
+    const long tiles = ((long)T + P.tok_per_cta - 1) / P.tok_per_cta * n_kv_heads;
+    if (tiles > 0x7FFFFFFFl) return COBALT_ETOOBIG;
+    CUtensorMap qm, km, vm;
+    const cuuint64_t qdim[3] = {(cuuint64_t)head_dim, (cuuint64_t)n_heads, (cuuint64_t)T};
+    const cuuint64_t qstr[2] = {(cuuint64_t)head_dim * 2, (cuuint64_t)n_heads * head_dim * 2};
+    const cuuint32_t qbox[3] = {64, (cuuint32_t)rep, (cuuint32_t)P.tok_per_cta};
+    const cuuint64_t kdim[3] = {(cuuint64_t)head_dim, (cuuint64_t)n_slots, (cuuint64_t)n_kv_heads};   // slots beyond n_slots read as zero
+    const cuuint64_t kstr[2] = {(cuuint64_t)head_dim * 2, (cuuint64_t)max_ctx * head_dim * 2};
+    const cuuint32_t kbox[3] = {64, PA_KEYS, 1};
+    if ((rc = make_map_3d(&qm, q, qdim, qstr, qbox)) || (rc = make_map_3d(&km, k_cache, kdim, kstr, kbox)) ||
+        (rc = make_map_3d(&vm, v_cache, kdim, kstr, kbox))) return rc;
+    return head_dim == 64 ? launch_prompt_attn<64>(P, (unsigned)tiles, qm, km, vm, (cudaStream_t)stream)
+                          : launch_prompt_attn<128>(P, (unsigned)tiles, qm, km, vm, (cudaStream_t)stream);
 }
 
 int cobalt_swiglu(const void* gate, const void* up, void* out, int64_t n, int act, void* stream) {

@@ -154,6 +154,9 @@ class CobaltDecoder:
         need = _lib.load().cobalt_attn_decode_scratch_bytes(self.nh, D, max_ctx) * self.B
         self.att_scratch = torch.empty(need, dtype=torch.uint8, device=device) if self.nh // self.nkv <= 8 and D % 64 == 0 and D <= 256 \
             and max_ctx <= 65536 else None
+        # Prompts take the library's tcgen05 attention (128 / 64 wide heads), other head widths batched matmuls
+        self.prompt_kernel = D in (64, 128) and self.nh // self.nkv <= 128 and max_ctx <= 1 << 24
+        self.prompt_status = torch.zeros(1, dtype=torch.int32, device=device)          # non-zero: a bounded wait gave up
         # One-kernel attention (cooperative launch; its scratch starts zeroed; only while its whole grid fits on the GPU).
         # Off by default: bit-identical to the three kernels but slower inside the decode graph (4-layer 7B-shaped step
         # 0.574 ms against 0.524 ms) - a cooperative launch does not overlap its neighbours.  Set the flag before the
@@ -238,6 +241,17 @@ class CobaltDecoder:
                                           q.shape[0], self.seq_stride if seq is None else 0,
                                           torch.cuda.current_stream(self.dev).cuda_stream)
         _lib.check("cobalt_attn_decode", rc)
+        return ctx
+
+    def _attn_prompt(self, q, positions, layer, seq: int, n_slots: int):
+        """Attention of the T tokens of a prompt over cache slots [0, n_slots) of sequence ``seq``, one kernel."""
+        ctx = torch.empty_like(q)
+        window = int(self.cfg.get("sliding_window") or 0) if self.types[layer] == "sliding_attention" else 0
+        rc = self._lib.cobalt_attn_prompt(q.data_ptr(), self.k_cache[layer][seq].data_ptr(), self.v_cache[layer][seq].data_ptr(),
+                                          positions.data_ptr(), ctx.data_ptr(), q.shape[0], self.nh, self.nkv, self.cfg["head_dim"],
+                                          n_slots, self.max_ctx, window, self.scale, self.prompt_status.data_ptr(),
+                                          torch.cuda.current_stream(self.dev).cuda_stream)
+        _lib.check("cobalt_attn_prompt", rc)
         return ctx
 
     def _row_parallel(self, lin, x):
@@ -336,14 +350,15 @@ class CobaltDecoder:
         h = P["model.embed_tokens.weight"].index_select(0, ids)                        # [T, H]
         if self.gemma:
             h = h * self.embed_scale                                                   # scale rounded to bf16 first
-        causal = self.kv_pos[None, :S] <= positions[:, None]                           # [T, S]
         blocked, allowed_of = {}, {}
-        for lt in set(self.types):
-            allowed = causal
-            if lt == "sliding_attention" and cfg.get("sliding_window"):
-                allowed = allowed & (self.kv_pos[None, :S] > positions[:, None] - cfg["sliding_window"])
-            blocked[lt] = ~allowed[None, :, None, :]                                   # [1, T, 1, S]
-            allowed_of[lt] = allowed[None, None]                                       # [1, 1, T, S]
+        if seq is not None and (self.fused_prompt_attention or not self.prompt_kernel) and (T > 1 or self.att_scratch is None):
+            causal = self.kv_pos[None, :S] <= positions[:, None]                       # [T, S]
+            for lt in set(self.types):
+                allowed = causal
+                if lt == "sliding_attention" and cfg.get("sliding_window"):
+                    allowed = allowed & (self.kv_pos[None, :S] > positions[:, None] - cfg["sliding_window"])
+                blocked[lt] = ~allowed[None, :, None, :]                               # [1, T, 1, S]
+                allowed_of[lt] = allowed[None, None]                                   # [1, 1, T, S]
         scale = self.scale
         delta, delta_w = None, None                                                    # pending branch and (Gemma) its norm weight
         for i in range(cfg["num_hidden_layers"]):
@@ -358,7 +373,7 @@ class CobaltDecoder:
                 ctx = self._attn_one(q, positions, i, None)
             elif T == 1 and self.att_scratch is not None:
                 ctx = self._attn_one(q, positions, i, seq)
-            elif self.fused_prompt_attention and T > 16:
+            elif blocked and self.fused_prompt_attention and T > 16:
                 # opt-in for prompts: the library's fused attention (fp32 scores and softmax inside; no [T, S] score
                 # tensor in memory).  It skips the spec's bf16 rounding of scores and probabilities; on a small model the
                 # prefill logits then sit 7e-3 (rel-L2) from the spec against 2e-3 for a change of accumulation order,
@@ -366,8 +381,10 @@ class CobaltDecoder:
                 ctx = F.scaled_dot_product_attention(q.view(1, T, nh, D).transpose(1, 2), Kc.unsqueeze(0), Vc.unsqueeze(0),
                                                      attn_mask=allowed_of[self.types[i]], scale=scale, enable_gqa=True)
                 ctx = ctx.transpose(1, 2).reshape(T, nh * D)
+            elif self.prompt_kernel:
+                ctx = self._attn_prompt(q, positions, i, seq, S)
             elif T > 64:
-                # prompts: one KV head at a time, so that its [T * rep, S] scores (bf16), probabilities (fp32, then bf16)
+                # prompts of other head widths: one KV head at a time, so that its [T * rep, S] scores (bf16), probabilities (fp32, then bf16)
                 # stay in the L2 cache between the element-wise passes; same arithmetic as below
                 ctx = torch.empty(T, nkv, rep, D, dtype=q.dtype, device=q.device)
                 q4 = q.view(T, nkv, rep, D)

@@ -313,6 +313,14 @@ size_t cobalt_attn_decode_fused_scratch_bytes(int n_heads, int n_kv_heads, int h
 int cobalt_attn_decode_fused(const void* q, const void* k_cache, const void* v_cache, const int64_t* positions, void* scratch,
                              size_t scratch_bytes, void* out, int n_heads, int n_kv_heads, int head_dim, int max_ctx,
                              int window, float scale, int n_seq, int64_t cache_seq_stride, void* stream);
+/* Grouped-query attention of T tokens of one sequence (q and out [T][n_heads*D], q already rotated) over its caches
+ * [n_kv_heads][max_ctx][D]: token t attends the slots s < n_slots with s <= positions[t] (and s > positions[t] - window when
+ * window > 0).  Same rounding points as cobalt_attn_decode(); scores and probabilities stay on the chip.  D 64 or 128 and at
+ * most 128 query heads per KV head, else COBALT_EUNSUPPORTED (nothing launched).  q, caches and out 16-byte aligned.  status
+ * (may be NULL): a u32 that is set when a bounded wait gives up. */
+int cobalt_attn_prompt(const void* q, const void* k_cache, const void* v_cache, const int64_t* positions, void* out, int T,
+                       int n_heads, int n_kv_heads, int head_dim, int n_slots, int max_ctx, int window, float scale, void* status,
+                       void* stream);
 
 /* All-reduce (sum) of the fp32 partial outputs of a row-parallel layer over peer memory, for tensor-parallel decode
  * (the reference has no distributed code; this replaces the NCCL all-reduce that would follow cobalt_linear_f32).

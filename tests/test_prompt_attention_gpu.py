@@ -1,0 +1,76 @@
+"""Prompt attention (``cobalt_attn_prompt``, tcgen05) against the spec's arithmetic in fp64 (needs a B200).
+
+Reference: scores rounded to bf16, scaled and rounded again, fp32 softmax, probabilities rounded to bf16
+(src/cobaltkernel/ref_llama.py:117-137), every contraction in fp64.  Tolerance: the result is a bf16 rounding (at most 2^-9
+relative per element) of a sum whose bf16 scores and probabilities may fall on the other side of a rounding boundary (at most
+2^-8 relative each, for a small share of them): 2^-8 on the 2-norm, and 2^-6 of the largest value on a single element.
+"""
+import pytest
+import torch
+
+from cobalt_b200 import _lib
+
+pytestmark = pytest.mark.gpu
+
+
+def spec(q, k, v, pos, n_slots, window, scale, nh, nkv, D):
+    T, rep = q.shape[0], nh // nkv
+    slots = torch.arange(n_slots, device=q.device)
+    allowed = slots[None] <= pos[:, None]
+    if window > 0:
+        allowed &= slots[None] > pos[:, None] - window
+    out = torch.empty(T, nh, D, dtype=torch.float64, device=q.device)
+    for h in range(nh):
+        s = (q.view(T, nh, D)[:, h].double() @ k[h // rep, :n_slots].double().t()).to(torch.bfloat16) * scale
+        p = torch.softmax(s.float().masked_fill(~allowed, float("-inf")), -1).to(torch.bfloat16)
+        out[:, h] = p.double() @ v[h // rep, :n_slots].double()
+    return out.view(T, nh * D)
+
+
+def call(q, k, v, pos, n_slots, window, scale, nh, nkv, D):
+    out, status = torch.full_like(q, float("nan")), torch.zeros(1, dtype=torch.int32, device=q.device)
+    rc = _lib.load().cobalt_attn_prompt(q.data_ptr(), k.data_ptr(), v.data_ptr(), pos.data_ptr(), out.data_ptr(), q.shape[0], nh, nkv,
+                                        D, n_slots, k.shape[1], window, scale, status.data_ptr(),
+                                        torch.cuda.current_stream().cuda_stream)
+    return rc, out, status
+
+
+# one token, tiles of 128 rows minus / plus one, head groups that do not divide 128 rows, windows that end inside a
+# tile, a prompt that continues a filled cache, scores far from zero (the maximum is what keeps exp in range)
+@pytest.mark.parametrize("T,nh,nkv,D,ctx,window,start,gain", [
+    (1, 4, 2, 64, 40, 0, 0, 1.0), (2, 8, 2, 128, 40, 0, 0, 1.0), (31, 8, 2, 128, 40, 0, 0, 1.0), (33, 8, 2, 64, 64, 0, 0, 1.0),
+    (127, 1, 1, 128, 128, 0, 0, 1.0), (129, 1, 1, 64, 200, 0, 0, 1.0), (200, 6, 2, 128, 256, 0, 0, 1.0), (150, 7, 1, 64, 160, 64, 0, 1.0),
+    (300, 5, 1, 128, 300, 100, 0, 1.0), (100, 8, 2, 128, 700, 128, 500, 1.0), (77, 16, 1, 128, 500, 0, 333, 1.0), (640, 4, 2, 128, 640, 0, 0, 12.0)])
+def test_prompt_attention_matches_spec(T, nh, nkv, D, ctx, window, start, gain):
+    g = torch.Generator(device="cuda").manual_seed(T + nh)
+    n_slots = start + T
+    q = (torch.randn(T, nh * D, generator=g, device="cuda") * gain).bfloat16()
+    k, v = (torch.randn(nkv, ctx, D, generator=g, device="cuda").bfloat16() for _ in range(2))
+    pos = torch.arange(start, n_slots, device="cuda")
+    rc, out, status = call(q, k, v, pos, n_slots, window, D ** -0.5, nh, nkv, D)
+    ref = spec(q, k, v, pos, n_slots, window, D ** -0.5, nh, nkv, D)
+    assert rc == 0 and int(status) == 0
+    d = out.double() - ref
+    assert float(d.norm() / ref.norm()) <= 2.0 ** -8
+    assert float(d.abs().max()) <= 2.0 ** -6 * float(ref.abs().max())
+
+
+def test_slots_beyond_the_prompt_are_not_read():
+    """What an earlier, longer prompt left in the cache (here: NaN) does not reach the result."""
+    g = torch.Generator(device="cuda").manual_seed(3)
+    q = torch.randn(50, 4 * 64, generator=g, device="cuda").bfloat16()
+    k, v = (torch.randn(2, 300, 64, generator=g, device="cuda").bfloat16() for _ in range(2))
+    pos = torch.arange(50, device="cuda")
+    _, want, _ = call(q, k, v, pos, 50, 0, 0.125, 4, 2, 64)
+    k[:, 50:] = float("nan")
+    v[:, 50:] = float("nan")
+    _, got, _ = call(q, k, v, pos, 50, 0, 0.125, 4, 2, 64)
+    assert torch.equal(got, want)
+
+
+def test_unsupported_shapes_are_refused():
+    q = torch.zeros(4, 4 * 96, dtype=torch.bfloat16, device="cuda")
+    k = torch.zeros(2, 8, 96, dtype=torch.bfloat16, device="cuda")
+    pos = torch.arange(4, device="cuda")
+    assert call(q, k, k, pos, 4, 0, 0.1, 4, 2, 96)[0] == _lib.EUNSUPPORTED
+    assert call(q, k, k, pos, 9, 0, 0.1, 4, 2, 96)[0] != 0                       # more slots than the cache has
