@@ -2,6 +2,7 @@
 // See include/cobalt_b200.h for the contract of every entry point.
 #include <cuda_runtime.h>
 #include <stdint.h>
+#include <math.h>
 #include <stdlib.h>
 
 #include "common.cuh"
@@ -16,6 +17,7 @@ using namespace cb;
 namespace {
 
 constexpr size_t SMEM_LIMIT = 227 * 1024;
+constexpr size_t GEMM_SINGLE_SMEM = 113 * 1024;     // two CTAs on the 228 KB of an SM, 1 KB of each reserved by the system
 constexpr int MAX_DEVICES = 64;
 
 int g_num_sms[MAX_DEVICES];
@@ -27,6 +29,8 @@ bool g_dev_known[MAX_DEVICES];
 int g_tune_tiles_per_split = 0;     // 0 = heuristic
 int g_tune_gemv_stages = 0;
 int g_tune_gemm_stages = 0;
+int g_tune_gemm_form = 0;            // 1 = single CTAs, 2 = pairs
+int g_tune_gemm_tiles = 0;           // token tiles beyond the fewest, + 1
 int g_tune_gemv_mode = 0;           // 0 = heuristic, 1 = CTAs hold whole row blocks, 2 = balanced words
 #else
 constexpr int g_tune_tiles_per_split = 0, g_tune_gemv_stages = 0, g_tune_gemm_stages = 0, g_tune_gemv_mode = 0;
@@ -173,38 +177,85 @@ int launch_gemv(const GemvParams& P, const GemvCfg& c, cudaStream_t st) {
 
 // ----------------------------------------------------------------------------- GEMM configuration
 struct GemmCfg {
-    int splits, tok_per_cta;
+    bool pair;
+    int tok_per_cta, acc_tokens, splits, a_stages, b_stages;
+    uint32_t box_rows, b_acc_bytes, b_stage_bytes;
     dim3 grid;
-    size_t counters_off, partials_off, total;
+    size_t smem;
 };
 
-int gemm_config(const CobaltMat* w, int M, int num_sms, GemmCfg* c) {
-    const int row_tiles = (w->n_row_blocks + GEMM_RB - 1) / GEMM_RB;
-    // One token tile whenever the tokens fit one (M <= 512): a CTA decodes its 128-row slab of the weights whatever the
-    // number of tokens, so cutting the tokens would decode every weight tile several times.  SMs that such a grid
-    // leaves idle are filled by splitting the columns instead (split-K over whole column tiles, fp32 partial sums).
-    int tpc = 64;
-    while (tpc < GEMM_TOKENS && tpc < M) tpc *= 2;
-    c->tok_per_cta = tpc;
-    const int tok_tiles = (M + tpc - 1) / tpc;
-    const long units = (long)row_tiles * tok_tiles;
-    long splits = 1;
-    if (g_tune_gemm_stages > 0) splits = g_tune_gemm_stages;                 // tuning key 2 overrides the split-K factor
-    else if (units < (long)num_sms) splits = num_sms / units;
-    if (splits > 16) splits = 16;
-    if (splits > w->n_col_tiles) splits = w->n_col_tiles;
-    if (splits < 1) splits = 1;
-    {   // every split gets at least one column tile: the kernel hands out ceil(CT / splits) tiles per split
-        const long per = (w->n_col_tiles + splits - 1) / splits;
-        splits = (w->n_col_tiles + per - 1) / per;
+// Form (single CTAs, two per SM, or CTA pairs), token tile and split of one launch of `row_tiles` 128-row tiles: the cheapest
+// of all under a cost model in SM clocks, fitted to 770 timed launches (512 .. 28672 rows, 1024 .. 14336 columns, 20 .. 2048 tokens,
+// every form, one to four more token tiles than needed, 1 .. 8 splits; 8 % rms).  Over those shapes its choice is 2.5 % slower
+// than the best launch on average, 20 % at worst (1024 x 4096, 64 tokens: 22.5 us against 18.4).
+//   per 64-column stage, the largest of: expanding its weights (a CTA that has its SM to itself, one of two, a pair's); MMA
+//   per token; operands through shared memory (A written once and read once per accumulator, B written and read, half of it
+//   per SM in a pair; 128 bytes per clock)
+//   per tile: first loads, drain and epilogue, with the tokens;  split columns: cluster barriers and reduction
+//   clusters of many CTAs do not fill every SM of a GPC: the share that does
+constexpr double GEMM_CLK_ALONE = 1280, GEMM_CLK_SHARED = 990, GEMM_CLK_PAIR = 1150, GEMM_CLK_MMA_TOKEN = 2.74, GEMM_CLK_SMEM = 1.56 / 128;
+constexpr double GEMM_CLK_TILE = 12000, GEMM_CLK_TILE_TOKEN = 47, GEMM_CLK_SPLIT = 1700, GEMM_CLK_SPLIT_TOKEN = 9.5;
+
+int gemm_config(int row_tiles, int G, int M, int num_sms, GemmCfg* c) {
+    double best = 0;
+    c->tok_per_cta = 0;
+    for (int form = 0; form < 2; ++form) {
+        const bool pair = form == 1;
+#ifdef COBALT_TUNING_HOOKS
+        if (g_tune_gemm_form > 0 && g_tune_gemm_form != form + 1) continue;
+#endif
+        const int cap = pair ? GEMM_PAIR_TOKENS : GEMM_SINGLE_TOKENS, step = pair ? 32 : 16;
+        const long rows = pair ? (row_tiles + 1) / 2 * 2 : row_tiles;
+        for (int extra = 0, last = 0; extra < 8; ++extra) {
+#ifdef COBALT_TUNING_HOOKS
+            if (g_tune_gemm_tiles > 0 && g_tune_gemm_tiles != extra + 1) continue;
+#endif
+            const long tiles = ((long)M + cap - 1) / cap + extra;
+            int tpc = (int)(((long)M + tiles - 1) / tiles);
+            int accs = tpc > 256 ? 2 : 1;
+            const int acc = ((tpc + accs - 1) / accs + step - 1) / step * step;
+            tpc = acc * accs;
+            if (tpc == last) continue;
+            last = tpc;
+            const long tok_tiles = ((long)M + tpc - 1) / tpc;
+            for (int splits = 1; splits <= (pair ? GEMM_MAX_SPLITS / 2 : GEMM_MAX_SPLITS) && splits <= G; splits *= 2) {
+                if (g_tune_gemm_stages > 0 && splits != g_tune_gemm_stages) continue;      // tuning key 2 overrides the split-K factor
+                const double ctas = (double)rows * tok_tiles * splits;
+                const int cluster = pair ? 2 * splits : splits;
+                const double sms = num_sms * (pair ? (cluster >= 8 ? 0.75 : cluster >= 4 ? 0.9 : 1.0) : (cluster >= 8 ? 0.93 : cluster >= 4 ? 0.97 : 1.0));
+                const double smem = GEMM_CLK_SMEM * (pair ? 16384.0 * (1 + accs) + 128.0 * tpc : 32768.0 + 256.0 * tpc);
+                const bool alone = pair || ctas <= sms;
+                double clk = pair ? GEMM_CLK_PAIR : alone ? GEMM_CLK_ALONE : GEMM_CLK_SHARED;
+                if (clk < GEMM_CLK_MMA_TOKEN * tpc) clk = GEMM_CLK_MMA_TOKEN * tpc;
+                if (clk < smem) clk = smem;
+                const double stages = 2.0 * ((G + splits - 1) / splits), tile = GEMM_CLK_TILE + GEMM_CLK_TILE_TOKEN * tpc;
+                double cost = alone ? ceil(ctas / sms) * (stages * clk + tile) : ceil(ctas / (2.0 * sms)) * (2.0 * stages * clk + tile);
+                if (splits > 1) cost += GEMM_CLK_SPLIT * splits + GEMM_CLK_SPLIT_TOKEN * tpc;
+                if (c->tok_per_cta == 0 || cost < best) {
+                    best = cost;
+                    c->pair = pair; c->tok_per_cta = tpc; c->acc_tokens = acc; c->splits = splits;
+                    c->grid = dim3((unsigned)rows, (unsigned)tok_tiles, (unsigned)splits);
+                }
+            }
+        }
     }
-    c->splits = (int)splits;
-    c->grid = dim3((unsigned)row_tiles, (unsigned)tok_tiles, (unsigned)splits);
-    c->counters_off = SCRATCH_STATUS_BYTES;
-    c->partials_off = c->counters_off + round_up((size_t)units * 4, 256);
-    if (c->partials_off < SCRATCH_STATUS_BYTES + SCRATCH_COUNTER_BYTES) c->partials_off = SCRATCH_STATUS_BYTES + SCRATCH_COUNTER_BYTES;
-    c->total = c->partials_off + (splits > 1 ? (size_t)units * splits * GEMM_TOKENS * GEMM_ROWS * sizeof(float) : 0);
-    return COBALT_OK;
+    if (c->tok_per_cta == 0 || c->grid.y > 65535u) return COBALT_ETOOBIG;
+    c->box_rows = (uint32_t)(c->pair ? c->acc_tokens / 2 : c->acc_tokens);
+    c->b_acc_bytes = c->box_rows * GEMM_KS * 2;
+    c->b_stage_bytes = c->b_acc_bytes * (uint32_t)(c->tok_per_cta / c->acc_tokens);
+    // Operand stages in the CTA's share of the shared memory (one CTA per SM in a pair, else two): as many of B as leave the
+    // decode warps a free stage of A besides the ones they are writing (four groups of warps in a pair, two else), the rest to A
+    const size_t share = c->pair ? SMEM_LIMIT : GEMM_SINGLE_SMEM, fixed = GEMM_LUT_BYTES + GEMM_BAR_BYTES;
+    for (c->b_stages = 4; ; --c->b_stages) {
+        const long room = (long)share - (long)fixed - (long)c->b_stages * c->b_stage_bytes;
+        c->a_stages = room > 0 ? (int)(room / GEMM_A_BYTES) : 0;
+        if (c->a_stages > GEMM_MAX_STAGES) c->a_stages = GEMM_MAX_STAGES;
+        if (c->a_stages >= (c->pair ? 5 : 3) || c->b_stages == 2) break;
+    }
+    if (c->a_stages < (c->pair ? 4 : 2)) return COBALT_EINVAL;
+    c->smem = fixed + (size_t)c->a_stages * GEMM_A_BYTES + (size_t)c->b_stages * c->b_stage_bytes;
+    if (c->splits > 1 && c->smem < gemm_red_bytes(c->pair)) c->smem = gemm_red_bytes(c->pair);
+    return c->smem <= share ? COBALT_OK : COBALT_EINVAL;
 }
 
 typedef CUresult (*TensorMapEncodeFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
@@ -223,13 +274,13 @@ TensorMapEncodeFn tensor_map_encoder() {
     return fn;
 }
 
-// activations [M, N] bf16, row stride ldx elements: box = 64 columns x 256 tokens, 128-byte swizzle
-int make_x_map(CUtensorMap* map, const void* x, int64_t ldx, int M, int N) {
+// activations [M, N] bf16, row stride ldx elements: box = 64 columns x box_rows tokens, 128-byte swizzle
+int make_x_map(CUtensorMap* map, const void* x, int64_t ldx, int M, int N, uint32_t box_rows) {
     TensorMapEncodeFn enc = tensor_map_encoder();
     if (!enc) return COBALT_ELAUNCH;
     cuuint64_t gdim[2] = {(cuuint64_t)N, (cuuint64_t)M};
     cuuint64_t gstride[1] = {(cuuint64_t)ldx * 2};
-    cuuint32_t box[2] = {(cuuint32_t)GEMM_KS, (cuuint32_t)GEMM_NT};
+    cuuint32_t box[2] = {(cuuint32_t)GEMM_KS, (cuuint32_t)box_rows};
     cuuint32_t estr[2] = {1, 1};
     CUresult r = enc(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(x), gdim, gstride, box, estr,
                      CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
@@ -237,18 +288,36 @@ int make_x_map(CUtensorMap* map, const void* x, int64_t ldx, int M, int N) {
     return r == CUDA_SUCCESS ? COBALT_OK : COBALT_EINVAL;
 }
 
-template <int BITS>
+template <int BITS, bool PAIR, bool SCALED>
 int launch_gemm(const GemmParams& P, const CUtensorMap& xmap, const GemmCfg& c, cudaStream_t st) {
+    auto kernel = gemm_tcgen05_kernel<BITS, PAIR, SCALED>;
     static bool configured[MAX_DEVICES];
     int dev = 0;
     cudaGetDevice(&dev);
     if (!configured[dev]) {
-        if (cudaFuncSetAttribute(gemm_tcgen05_kernel<BITS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GEMM_SMEM_BYTES) != cudaSuccess)
+        if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(PAIR ? SMEM_LIMIT : GEMM_SINGLE_SMEM)) != cudaSuccess)
             return COBALT_ELAUNCH;
         configured[dev] = true;
     }
-    gemm_tcgen05_kernel<BITS><<<c.grid, GEMM_THREADS, GEMM_SMEM_BYTES, st>>>(P, xmap);
-    return cudaGetLastError() == cudaSuccess ? COBALT_OK : COBALT_ELAUNCH;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = c.grid;
+    cfg.blockDim = dim3((unsigned)gemm_threads(PAIR));
+    cfg.dynamicSmemBytes = c.smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = PAIR ? 2 : 1;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = (unsigned)c.splits;
+    cfg.attrs = attr;
+    cfg.numAttrs = PAIR || c.splits > 1 ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, kernel, P, xmap) == cudaSuccess ? COBALT_OK : COBALT_ELAUNCH;
+}
+
+template <int BITS>
+int launch_gemm(const GemmParams& P, const CUtensorMap& xmap, const GemmCfg& c, cudaStream_t st) {
+    if (P.col_scale) return c.pair ? launch_gemm<BITS, true, true>(P, xmap, c, st) : launch_gemm<BITS, false, true>(P, xmap, c, st);
+    return c.pair ? launch_gemm<BITS, true, false>(P, xmap, c, st) : launch_gemm<BITS, false, false>(P, xmap, c, st);
 }
 
 // bf16 tensor of three dimensions, box 64 elements wide (one 128-byte swizzle row)
@@ -469,7 +538,7 @@ const char* cobalt_strerror(int status) {
 
 #ifdef COBALT_TUNING_HOOKS
 // Experiment hook: key 0 = GEMV grid size, 1 = GEMV ring stages, 2 = GEMM split-K factor, 3 = GEMV partition
-// (1 = whole row blocks per CTA, 2 = balanced words); value 0 restores the heuristic.
+// (1 = whole row blocks per CTA, 2 = balanced words), 4 = GEMM form (1 = single CTAs, 2 = pairs), 5 = 1 + token tiles beyond the fewest; value 0 restores the heuristic.
 int cobalt_set_tuning(int key, int value) {
     if (value < 0) return COBALT_EINVAL;
     switch (key) {
@@ -477,6 +546,8 @@ int cobalt_set_tuning(int key, int value) {
         case 1: g_tune_gemv_stages = value; return COBALT_OK;
         case 2: g_tune_gemm_stages = value; return COBALT_OK;
         case 3: g_tune_gemv_mode = value; return COBALT_OK;
+        case 4: g_tune_gemm_form = value; return COBALT_OK;
+        case 5: g_tune_gemm_tiles = value; return COBALT_OK;
         default: return COBALT_EINVAL;
     }
 }
@@ -615,59 +686,87 @@ int cobalt_gemv_rowwalk(const CobaltMat* w, const void* x, int64_t ldx, void* y,
     return cudaGetLastError() == cudaSuccess ? COBALT_OK : COBALT_ELAUNCH;
 }
 
+// the GEMM keeps its partial sums on the chip: its scratch is the status word (and the counters of the GEMV it may share it with)
 size_t cobalt_gemm_scratch_bytes(const CobaltMat* w, int M) {
     int sms = 0;
     if (check_mat(w) != COBALT_OK || M <= 0) return 0;
     if (device_info(&sms) != COBALT_OK) return 0;
-    GemmCfg c;
-    if (gemm_config(w, M, sms, &c) != COBALT_OK) return 0;
-    return c.total;
+    return SCRATCH_STATUS_BYTES + SCRATCH_COUNTER_BYTES;
 }
 
-static int gemm_impl(const CobaltMat* w, const void* x, int64_t ldx, void* y, int64_t ldy, const void* bias, int M,
-                     void* scratch, size_t scratch_bytes, void* stream, bool fp32_out) {
-    int rc = check_mat(w);
-    if (rc) return rc;
-    rc = check_io(x, ldx, y, ldy, M, w->K, w->N);
-    if (rc) return rc;
+static int gemm_impl(int n, const CobaltMat* const* w, const GemvOut* out, const void* x, int64_t ldx, int M, void* scratch,
+                     size_t scratch_bytes, void* stream, bool fp32_out) {
+    if (n < 1 || n > GEMV_MAX_MATS || !w || !out) return COBALT_EINVAL;
+    GemmParams P = {};
+    int row_tiles = 0;
+    for (int i = 0; i < n; ++i) {
+        int rc = check_mat(w[i]);
+        if (rc) return rc;
+        rc = check_io(x, ldx, out[i].y, out[i].ldy, M, w[i]->K, w[i]->N);
+        if (rc) return rc;
+        if (i > 0 && (w[i]->N != w[0]->N || w[i]->bits != w[0]->bits || w[i]->col_scale || w[0]->col_scale)) return COBALT_EINVAL;
+        P.mat[i].tiles = (const uint8_t*)w[i]->tiles;
+        P.mat[i].tile_off = w[i]->tile_off;
+        P.mat[i].y = fp32_out ? nullptr : (uint16_t*)out[i].y;
+        P.mat[i].y32 = fp32_out ? (float*)out[i].y : nullptr;
+        P.mat[i].bias = (const uint16_t*)out[i].bias;
+        P.mat[i].ldy = out[i].ldy;
+        P.mat[i].K = w[i]->K; P.mat[i].RB = w[i]->n_row_blocks;
+        P.mat[i].rt_start = row_tiles;
+        row_tiles += (w[i]->n_row_blocks + GEMM_RB - 1) / GEMM_RB;
+    }
     int sms = 0;
-    rc = device_info(&sms);
+    int rc = device_info(&sms);
     if (rc) return rc;
     GemmCfg c;
-    rc = gemm_config(w, M, sms, &c);
+    rc = gemm_config(row_tiles, w[0]->N / GROUP, M, sms, &c);
     if (rc) return rc;
-    if (!scratch || ((uintptr_t)scratch & 255) || scratch_bytes < c.total) return COBALT_ESCRATCH;
+    if (!scratch || ((uintptr_t)scratch & 255) || scratch_bytes < SCRATCH_STATUS_BYTES + SCRATCH_COUNTER_BYTES) return COBALT_ESCRATCH;
     CUtensorMap xmap;
-    rc = make_x_map(&xmap, x, ldx, M, w->N);
+    rc = make_x_map(&xmap, x, ldx, M, w[0]->N, c.box_rows);
     if (rc) return rc;
-    GemmParams P;
-    P.W = make_view(w);
-    P.y = fp32_out ? nullptr : (uint16_t*)y; P.ldy = ldy;
-    P.y32 = fp32_out ? (float*)y : nullptr;
-    P.bias = (const uint16_t*)bias;
+    P.n_mats = n;
+    P.G = w[0]->N / GROUP; P.CT = w[0]->n_col_tiles;
+    P.col_scale = (const uint16_t*)w[0]->col_scale;
     P.M = M;
-    P.splits = c.splits;
-    P.tok_per_cta = c.tok_per_cta;
+    P.tok_per_cta = c.tok_per_cta; P.acc_tokens = c.acc_tokens; P.splits = c.splits;
+    P.a_stages = c.a_stages; P.b_stages = c.b_stages;
+    P.b_acc_bytes = c.b_acc_bytes; P.b_stage_bytes = c.b_stage_bytes;
     P.status = (uint32_t*)scratch;
-    P.counters = (uint32_t*)((uint8_t*)scratch + c.counters_off);
-    P.partials = c.splits > 1 ? (float*)((uint8_t*)scratch + c.partials_off) : nullptr;
     cudaStream_t st = (cudaStream_t)stream;
-    switch (w->bits) {
+    switch (w[0]->bits) {
         case 2: return launch_gemm<2>(P, xmap, c, st);
         case 3: return launch_gemm<3>(P, xmap, c, st);
         default: return launch_gemm<4>(P, xmap, c, st);
     }
 }
 
+size_t cobalt_gemm_fused_scratch_bytes(int n_mats, const CobaltMat* const* w, int M) {
+    if (n_mats < 1 || n_mats > GEMV_MAX_MATS || !w) return 0;
+    for (int i = 0; i < n_mats; ++i)
+        if (cobalt_gemm_scratch_bytes(w[i], M) == 0) return 0;
+    return SCRATCH_STATUS_BYTES + SCRATCH_COUNTER_BYTES;
+}
+
+int cobalt_gemm_fused(int n_mats, const CobaltMat* const* w, const void* x, int64_t ldx, void* const* y, const int64_t* ldy,
+                      const void* const* bias, int M, void* scratch, size_t scratch_bytes, void* stream) {
+    if (n_mats < 1 || n_mats > GEMV_MAX_MATS || !w || !y || !ldy) return COBALT_EINVAL;
+    GemvOut o[GEMV_MAX_MATS];
+    for (int i = 0; i < n_mats; ++i) { o[i].y = y[i]; o[i].ldy = ldy[i]; o[i].bias = bias ? bias[i] : nullptr; }
+    return gemm_impl(n_mats, w, o, x, ldx, M, scratch, scratch_bytes, stream, false);
+}
+
 int cobalt_gemm(const CobaltMat* w, const void* x, int64_t ldx, void* y, int64_t ldy, const void* bias, int M,
                 void* scratch, size_t scratch_bytes, void* stream) {
-    return gemm_impl(w, x, ldx, y, ldy, bias, M, scratch, scratch_bytes, stream, false);
+    const GemvOut o = {y, ldy, bias};
+    return gemm_impl(1, &w, &o, x, ldx, M, scratch, scratch_bytes, stream, false);
 }
 
 int cobalt_linear_f32(const CobaltMat* w, const void* x, int64_t ldx, float* y, int64_t ldy, int M, void* scratch,
                       size_t scratch_bytes, void* stream) {
     if (M <= MAX_GEMV_M) return gemv_impl(w, x, ldx, y, ldy, nullptr, M, scratch, scratch_bytes, false, stream, true);
-    return gemm_impl(w, x, ldx, y, ldy, nullptr, M, scratch, scratch_bytes, stream, true);
+    const GemvOut o = {y, ldy, nullptr};
+    return gemm_impl(1, &w, &o, x, ldx, M, scratch, scratch_bytes, stream, true);
 }
 
 int cobalt_dequant(const CobaltMat* w, void* w_bf16, void* stream) {

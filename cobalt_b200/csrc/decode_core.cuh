@@ -380,17 +380,48 @@ CB_HD uint32_t code_view(uint32_t w0) {
     return (u & 0x0F0F0F0Fu) | ((u << 1) & 0xF0F0F0F0u);
 }
 
-template <int BITS>
-CB_HD void decode8(uint32_t w0, uint32_t selA, uint32_t selB, uint32_t self, const SegParams& p, uint32_t out[4]) {
+// dq(e, i) turns the bf16x2 pattern {128 + c0, 128 + c1} of positions (2i, 2i+1) into their weights
+template <int BITS, class Dq>
+CB_HD void decode8_with(uint32_t w0, uint32_t selA, uint32_t selB, uint32_t self, uint32_t zq, Dq dq, uint32_t out[4]) {
     constexpr uint32_t HI_SHIFT = BITS == 2 ? 2u : 4u;
     constexpr uint32_t CM = ((1u << BITS) - 1u) * 0x00010001u;
     const uint32_t v = code_view<BITS>(w0);
-    const uint32_t hi = prmt(v >> HI_SHIFT, p.zq, self);      // byte 3 <- zero point unless all eight are kept
+    const uint32_t hi = prmt(v >> HI_SHIFT, zq, self);        // byte 3 <- zero point unless all eight are kept
     const uint32_t d0 = prmt(v, hi, selA), d1 = prmt(v, hi, selB);
-    out[0] = dq_pair(and_or(d0, CM, 0x43004300u), p);
-    out[1] = dq_pair(and_or(d0 >> 8, CM, 0x43004300u), p);
-    out[2] = dq_pair(and_or(d1, CM, 0x43004300u), p);
-    out[3] = dq_pair(and_or(d1 >> 8, CM, 0x43004300u), p);
+    out[0] = dq(and_or(d0, CM, 0x43004300u), 0);
+    out[1] = dq(and_or(d0 >> 8, CM, 0x43004300u), 1);
+    out[2] = dq(and_or(d1, CM, 0x43004300u), 2);
+    out[3] = dq(and_or(d1 >> 8, CM, 0x43004300u), 3);
+}
+
+template <int BITS>
+CB_HD void decode8(uint32_t w0, uint32_t selA, uint32_t selB, uint32_t self, const SegParams& p, uint32_t out[4]) {
+    decode8_with<BITS>(w0, selA, selB, self, p.zq, [&](uint32_t e, int) { return dq_pair(e, p); }, out);
+}
+
+// The same with a column scale: bf16( fp32(fp32(d * s) * c) ), the literal fp32 sequence on an integer zero point (d exact).
+// c[8] = fp32 column scales of the eight positions.  A pruned position decodes to d = 0, hence to 0 - unless its
+// column scale is not finite, which the literal path (decode32_slow) does not multiply by: those are cleared.
+CB_HD uint32_t dq_pair_scaled(uint32_t e, const SegParams& p, float c0, float c1) {
+    const uint32_t d = bf2_add(e, p.zb2);
+    const float w0 = dequant_fp32(u2f(d << 16), 0.0f, p.s, c0), w1 = dequant_fp32(u2f(d & 0xFFFF0000u), 0.0f, p.s, c1);
+#if CB_DEVICE_CODE
+    uint32_t r;
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(w1), "f"(w0));
+    return r;
+#else
+    return float_to_bf16_bits(w0) | (float_to_bf16_bits(w1) << 16);
+#endif
+}
+template <int BITS>
+CB_HD void decode8_scaled(uint32_t mask_byte, uint32_t w0, uint32_t selA, uint32_t selB, uint32_t self, const SegParams& p,
+                          const float c[8], uint32_t out[4]) {
+    decode8_with<BITS>(w0, selA, selB, self, p.zq, [&](uint32_t e, int i) { return dq_pair_scaled(e, p, c[2 * i], c[2 * i + 1]); }, out);
+    float f = 0.0f;                                            // stays 0 while every scale is finite
+    for (int i = 0; i < 8; ++i) f += c[i] * 0.0f;
+    if (!(f == 0.0f))
+        for (int i = 0; i < 4; ++i)
+            out[i] &= (((mask_byte >> (2 * i)) & 1u) ? 0x0000FFFFu : 0u) | (((mask_byte >> (2 * i + 1)) & 1u) ? 0xFFFF0000u : 0u);
 }
 
 // Literal fp32 path for 32 positions of any segment (off-grid zero point, column scale): codes are read

@@ -1,26 +1,36 @@
-// Prefill GEMM: Y[m, k] = sum_j bf16(W[k, j]) * X[m, j] with tcgen05.mma, accumulators in
-// tensor memory.
+// Prefill GEMM: Y[m, k] = sum_j bf16(W[k, j]) * X[m, j] with tcgen05.mma, accumulators in tensor memory.  Up to four
+// matrices that read the same activations (q|k|v, gate|up) go out as one launch: their 128-row tiles form one list.
 //
-// One CTA owns 128 weight rows and up to 512 tokens.  Per 64-column stage it forms
-//   D0[128 x n0] += A[128 x 64] * B0[n0 x 64]^T      D1[128 x n1] += A * B1[n1 x 64]^T
-// (n0, n1 <= 256 tokens; bf16 operands, fp32 accumulators in 2 x 256 TMEM columns), so a weight
-// tile is dequantised once per 512 tokens.  Both operands are K-major in shared memory with the
-// 128-byte swizzle.
+// A CTA owns 128 weight rows and one token tile and walks the 64-column stages of its range of 128-column groups:
 //
-//   warps 0-7  decode: two groups of four warps take alternate stages; thread r of a group owns
-//              weight row r.  It reads the row's bitmask words and code bits straight from the
-//              tile image in global memory (next stage prefetched into registers), expands the 64
-//              columns of the stage to bf16 (decode_core.cuh) and writes eight swizzled 16-byte
-//              chunks into the A stage.  After the main loop the same warps drain TMEM (warp w
-//              reads lanes 32*(w%4).., accumulator w/4) and store the outputs.
-//   warp 8     one elected lane issues the TMA loads of the activation stage (2-D tensor map,
-//              box 64 columns x 256 tokens, 128-byte swizzle, rows beyond M zero-filled).
-//   warp 9     one elected lane issues tcgen05.mma and tcgen05.commit.
+//   decode     sets of eight warps: the first four take the first 64 columns of a group, the others the second; thread r of
+//              either half owns weight row r.  It reads the row's bitmask words and code bits straight from the tile image
+//              in global memory (the next group's codes are requested before the current one is expanded; whole tiles are
+//              prefetched into the L2 two column tiles ahead), expands them to bf16 (decode_core.cuh) and writes eight
+//              swizzled 16-byte chunks into the A stage.  One set per CTA of the single form, two (on alternate groups) in
+//              a pair: 16 warps per SM, whose expansion is bound by latency more than by issue slots.  After the main
+//              loop the same warps drain TMEM.
+//   next warp  one elected lane issues the TMA loads of the activation stage (2-D tensor map, 128-byte swizzle, rows
+//              beyond M zero-filled; no multicast).
+//   last warp  one elected lane issues tcgen05.mma and tcgen05.commit.
 //
-// Generic-proxy writes to A stages are published with fence.proxy.async before the mbarrier
-// arrive.  Every wait is bounded: on expiry the kernel records a status code, stops issuing
-// work, frees its tensor memory and returns.  With split-K (small grids) every CTA writes its
-// fp32 tile to scratch and the last CTA of a tile adds the splits in order.
+// Two forms, picked per launch by a cost model (gemm_config() in cobalt_abi.cu):
+//   single  up to 256 tokens in one accumulator, two CTAs per SM: one CTA's load latencies, start-up and epilogue hide
+//           under the other's work.  Small and middling token counts, where expanding the weights is the cost.
+//   pair    two CTAs of a cluster form one 256-row tile (tcgen05.mma.cta_group::2) of up to 512 tokens in two
+//           accumulators.  With one CTA per tile the limit at many tokens was operand traffic through shared memory: per
+//           stage 16 KB of A written and read twice, 64 KB of B written and read = 176 KB against 1024 cycles of MMA (128
+//           bytes per cycle: 1375 cycles).  In a pair each SM holds and reads half of B: 112 KB, 875 cycles.
+//
+// Split-K (grids that leave SMs idle): the CTAs of a tile's column ranges form a cluster, park their fp32 sums in shared
+// memory and each adds its share of the tokens over the cluster in split order (distributed shared memory): no partial
+// sum goes through global memory and no CTA adds alone.
+// Measured (1965 MHz, cold L2, one CTA per tile with 512 tokens and partial sums in global memory -> this kernel): 4096 x 14336, 3 bit,
+// 2048 tokens 232 -> 172 us (1.40 PFLOP/s); 4096 x 4096, 2048 tokens 91 -> 68 us; 14336 x 4096, 2048 tokens 317 -> 238 us;
+// 4096 x 4096, 100 tokens 33 -> 26 us; q|k|v of a 7B block (one launch instead of three), 2048 tokens 241 -> 123 us.
+//
+// Generic-proxy writes to A stages are published with fence.proxy.async before the mbarrier arrive.  Every wait on an
+// mbarrier is bounded: on expiry the kernel records a status code, stops issuing work, frees its tensor memory and returns.
 //
 // Behaviour replaced: cbk::gemm_tile (mma.sync m16n8k16, per-fragment bf16x2 dequantisation,
 // src/cobaltkernel/csrc/cobalt_gemm.cuh:243-609) driven by gemm_phase
@@ -32,58 +42,109 @@
 
 namespace cb {
 
-constexpr int GEMM_ROWS = 128;            // UMMA M
-constexpr int GEMM_NT = 256;              // UMMA N (tokens per accumulator)
-constexpr int GEMM_ACCS = 2;              // accumulators per CTA -> 512 tokens
-constexpr int GEMM_TOKENS = GEMM_NT * GEMM_ACCS;
+constexpr int GEMM_ROWS = 128;            // weight rows per CTA
 constexpr int GEMM_KS = 64;               // columns per stage = one 128-byte swizzle row of bf16
 constexpr int GEMM_RB = GEMM_ROWS / TILE_ROWS;   // 8 row blocks per CTA
 constexpr int GEMM_LUT_COPIES = 8;
-constexpr int GEMM_A_STAGES = 3;
-constexpr int GEMM_B_STAGES = 2;
-constexpr int GEMM_DECODE_THREADS = 256;
-constexpr int GEMM_THREADS = GEMM_DECODE_THREADS + 64;
+constexpr int GEMM_MAX_STAGES = 8;
+constexpr int GEMM_MAX_SPLITS = 8;        // CTAs of a cluster along the columns (portable cluster size)
+constexpr int gemm_decode_warps(bool pair) { return pair ? 16 : 8; }     // 16 on an SM either way: singles come in twos
+constexpr int gemm_threads(bool pair) { return gemm_decode_warps(pair) * 32 + 64; }
+constexpr int gemm_red_tokens(bool pair) { return pair ? 256 : 128; }    // tokens per round of the split reduction
 constexpr uint32_t GEMM_LUT_BYTES = LUT_ENTRIES * GEMM_LUT_COPIES * 8;   // 16 KB
 constexpr uint32_t GEMM_A_BYTES = GEMM_ROWS * GEMM_KS * 2;               // 16 KB
-constexpr uint32_t GEMM_BHALF_BYTES = GEMM_NT * GEMM_KS * 2;             // 32 KB
-constexpr uint32_t GEMM_B_BYTES = GEMM_BHALF_BYTES * GEMM_ACCS;          // 64 KB
-constexpr uint32_t GEMM_BAR_BYTES = 256;
-constexpr uint32_t GEMM_SMEM_BYTES = GEMM_A_STAGES * GEMM_A_BYTES + GEMM_B_STAGES * GEMM_B_BYTES + GEMM_LUT_BYTES +
-                                     GEMM_BAR_BYTES + 1024;
+constexpr uint32_t gemm_red_bytes(bool pair) { return (uint32_t)gemm_red_tokens(pair) * GEMM_ROWS * 4; }   // laid over the operand stages
+constexpr uint32_t GEMM_BAR_BYTES = 4 * GEMM_MAX_STAGES * 8 + 64;
+constexpr int GEMM_SINGLE_TOKENS = 256, GEMM_PAIR_TOKENS = 512;          // accumulator columns a CTA may hold
 
-struct GemmParams {
-    MatView W;
-    uint16_t* y; int64_t ldy;
+struct GemmMat {
+    const uint8_t* tiles;
+    const uint32_t* tile_off;
+    uint16_t* y;
     float* y32;                 // when set, raw fp32 sums go here instead (no bias, no rounding)
     const uint16_t* bias;
+    int64_t ldy;
+    int K, RB;
+    int rt_start;               // first row tile of this matrix in the launch's list
+};
+
+struct GemmParams {
+    GemmMat mat[GEMV_MAX_MATS];
+    int n_mats;
+    int G, CT;
+    const uint16_t* col_scale;  // fp16 bits; the SCALED instantiation only (single-matrix launches)
     int M;
-    int tok_per_cta;            // tokens per CTA: 512, or less (multiple of 16) to spread a small problem over more SMs
-    int splits;                 // split-K factor (column tiles are divided among blockIdx.z)
-    float* partials;            // [tile][split][GEMM_TOKENS][GEMM_ROWS] fp32 (splits > 1)
-    uint32_t* counters;         // [tile]
+    int tok_per_cta;            // tokens per token tile
+    int acc_tokens;             // tokens per accumulator (tok_per_cta = one or two of these)
+    int splits;                 // column ranges = CTAs of the cluster along z
+    int a_stages, b_stages;     // operand stages in shared memory
+    uint32_t b_acc_bytes;       // B bytes of one accumulator's tokens that this CTA holds per stage
+    uint32_t b_stage_bytes;
     uint32_t* status;
 };
 
-// ---- tcgen05 / TMA wrappers
+// ---- tcgen05 / TMA / cluster wrappers
+template <bool PAIR>
 __device__ __forceinline__ void tmem_alloc(uint32_t smem_dst, uint32_t ncols) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_dst), "r"(ncols) : "memory");
+    if (PAIR) asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_dst), "r"(ncols) : "memory");
+    else asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_dst), "r"(ncols) : "memory");
 }
+template <bool PAIR>
 __device__ __forceinline__ void tmem_relinquish() {
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    if (PAIR) asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+    else asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
 }
+template <bool PAIR>
 __device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t ncols) {
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
+    if (PAIR) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
+    else asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
 }
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
+template <bool PAIR>
 __device__ __forceinline__ void umma_bf16(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-        ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
+    if (PAIR)
+        asm volatile(
+            "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+            "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+            ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
+    else
+        asm volatile(
+            "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+            "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+            ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
 }
-__device__ __forceinline__ void umma_commit(uint32_t bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
+// completion of the MMAs issued so far -> the barrier at this offset (pair: in both CTAs, `mask` = their cluster ranks)
+template <bool PAIR>
+__device__ __forceinline__ void umma_commit(uint32_t bar, uint16_t mask = 0) {
+    if (PAIR)
+        asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar), "h"(mask) : "memory");
+    else
+        asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
+}
+// One lane of a converged warp.  The loops around TMA and MMA instructions run on the whole warp and only the instruction
+// itself is elected: their operands are then known to be warp-uniform and live in uniform registers.  With the loop inside
+// "if (lane == 0)" every descriptor took moves to uniform registers and 64-bit adds in one thread's dependent chain, and issuing
+// the four MMAs and two commits of a stage took 650 clocks, more than the stage's arithmetic.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t e;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.b32 %0, 1, 0, p;\n\t}" : "=r"(e));
+    return e != 0;
+}
+__device__ __forceinline__ uint32_t cluster_rank() { uint32_t r; asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r)); return r; }
+__device__ __forceinline__ void cluster_sync_all() {       // every thread of every CTA of the cluster
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ uint32_t map_to_rank(uint32_t addr, uint32_t rank) {
+    uint32_t r; asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank)); return r;
+}
+__device__ __forceinline__ float4 ld_cluster_f4(uint32_t addr) {
+    float4 v;
+    asm volatile("ld.shared::cluster.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr) : "memory");
+    return v;
+}
+__device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
+    asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }
 __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&v)[32]) {
     asm volatile(
@@ -96,10 +157,16 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&v)[32]) {
         : "r"(taddr) : "memory");
 }
 __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
-// 2-D tiled TMA load (no multicast): box of the tensor map at (x = column, y = token) -> shared
+// 2-D tiled TMA load (no multicast): box of the tensor map at (x = column, y = token) -> this CTA's shared memory; the pair
+// form may count its bytes on a barrier of either CTA of the pair
+template <bool PAIR>
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, int x, int y, uint32_t bar) {
-    asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
-                 ::"r"(dst), "l"(map), "r"(x), "r"(y), "r"(bar) : "memory");
+    if (PAIR)
+        asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes.cta_group::2 [%0], [%1, {%2, %3}], [%4];"
+                     ::"r"(dst), "l"(map), "r"(x), "r"(y), "r"(bar) : "memory");
+    else
+        asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
+                     ::"r"(dst), "l"(map), "r"(x), "r"(y), "r"(bar) : "memory");
 }
 
 // K-major, 128-byte swizzle, 8-row groups 1024 B apart; descriptor version 1 (sm_100)
@@ -112,352 +179,429 @@ __device__ __forceinline__ uint64_t umma_smem_desc(uint32_t smem_addr) {
     d |= (uint64_t)2 << 61;                               // SWIZZLE_128B
     return d;
 }
-// D = f32, A = B = bf16, both K-major, M = 128, N = n
-__device__ __forceinline__ uint32_t umma_idesc(uint32_t n) {
-    return (1u << 4) | (1u << 7) | (1u << 10) | ((n >> 3) << 17) | ((GEMM_ROWS >> 4) << 24);
+// D = f32, A = B = bf16, both K-major, M = m rows, N = n
+__device__ __forceinline__ uint32_t umma_idesc(uint32_t n, uint32_t m = GEMM_ROWS) {
+    return (1u << 4) | (1u << 7) | (1u << 10) | ((n >> 3) << 17) | ((m >> 4) << 24);
 }
 
-// Nibble window (128 bits, first survivor in bits 0..3 of w0) of the 32-column word whose first
-// survivor has rank `rank` in the tile's code stream `codes` (global memory, 4-byte aligned).
+// What a thread needs to expand 64 columns of its row; requested one group ahead.  The rows of a warp lie about 128 bytes
+// apart in the code stream, so every load touches 32 lines whatever its width: the up to 256 bits come in as aligned
+// 16-byte chunks (only those that hold survivors of these columns) and the words are picked out of registers.  With one
+// 4-byte load per word that lookup was the limit: ten loads = 320 lines per warp and stage, 1600 clocks a stage per SM.
 template <int BITS>
-__device__ __forceinline__ void fetch_window(const uint32_t* codes, uint32_t rank, uint32_t (&raw)[5]) {
-    const uint32_t bitpos = rank * (uint32_t)BITS;
-    const uint32_t* p = codes + (bitpos >> 5);
-    constexpr int NW = BITS == 4 ? 5 : (BITS == 3 ? 4 : 3);
+struct GemmFetch {
+    static constexpr int NC = BITS == 2 ? 2 : 3;          // 64 codes at any bit offset of the first chunk
+    uint4 chunk[NC];
+    uint32_t mask[2];
+    uint32_t bit;                                         // offset of the first code in chunk[0]
+    uint32_t sz;
+};
+// the N words from word `first` on, out of W words in registers (barrel shift: no indexed registers)
+template <int W, int N, bool WIDE>
+__device__ __forceinline__ void pick_words(const uint32_t (&c)[W], uint32_t first, uint32_t (&out)[N]) {
+    uint32_t a[W];
 #pragma unroll
-    for (int i = 0; i < 5; ++i) raw[i] = i < NW ? __ldg(p + i) : 0u;
-}
-template <int BITS>
-__device__ __forceinline__ void align_window(const uint32_t (&raw)[5], uint32_t rank, uint32_t& w0, uint32_t& w1,
-                                             uint32_t& w2, uint32_t& w3) {
-    const uint32_t o = (rank * (uint32_t)BITS) & 31u;
-    const uint32_t a0 = funnel_r(raw[0], raw[1], o), a1 = funnel_r(raw[1], raw[2], o);
-    const uint32_t a2 = funnel_r(raw[2], raw[3], o), a3 = funnel_r(raw[3], raw[4], o);
-    if (BITS == 4) {
-        w0 = a0; w1 = a1; w2 = a2; w3 = a3;
-    } else if (BITS == 3) {                     // 96 bits = four 24-bit chunks of 8 codes
-        w0 = spread3(a0 & 0x00FFFFFFu);
-        w1 = spread3(funnel_r(a0, a1, 24) & 0x00FFFFFFu);
-        w2 = spread3(funnel_r(a1, a2, 16) & 0x00FFFFFFu);
-        w3 = spread3(a2 >> 8);
-    } else {                                    // 64 bits = four 16-bit chunks of 8 codes
-        w0 = spread2(a0); w1 = spread2(a0 >> 16); w2 = spread2(a1); w3 = spread2(a1 >> 16);
+    for (int i = 0; i < W; ++i) a[i] = c[i];
+#pragma unroll
+    for (int step = WIDE ? 4 : 2; step > 0; step >>= 1) {
+        const bool on = (first & (uint32_t)step) != 0;
+#pragma unroll
+        for (int i = 0; i < W; ++i)
+            if (i < N + step - 1) a[i] = on && i + step < W ? a[i + step] : a[i];
     }
+#pragma unroll
+    for (int i = 0; i < N; ++i) out[i] = i < W ? a[i] : 0u;
 }
 
-template <int BITS>
-__global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tcgen05_kernel(const GemmParams P,
-                                                                       const __grid_constant__ CUtensorMap xmap) {
+template <int BITS, bool PAIR, bool SCALED>
+__global__ void __launch_bounds__(gemm_threads(PAIR), PAIR ? 1 : 2) gemm_tcgen05_kernel(const __grid_constant__ GemmParams P,
+                                                                                  const __grid_constant__ CUtensorMap xmap) {
     extern __shared__ __align__(1024) uint8_t smem[];
-    const MatView& W = P.W;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t full_mask = 0xFFFFFFFFu;
+    constexpr int DW = gemm_decode_warps(PAIR);
 
-    // ---- shared memory carve-up (operand stages 1024-byte aligned)
-    const uint32_t s_raw = smem_u32(smem);
-    const uint32_t s0 = (s_raw + 1023u) & ~1023u;                         // the allocation carries 1 KB of slack
-    uint8_t* const sm = smem + (s0 - s_raw);
+    // ---- shared memory: A stages | B stages | expansion table | barriers.  The operand stages need 1024-byte alignment;
+    // the dynamic window starts on it (two CTAs of 113 KB leave no room for slack).
+    const uint32_t s0 = smem_u32(smem);
+    if (s0 & 1023u) {
+        if (threadIdx.x == 0 && P.status) atomicCAS(P.status, 0u, (uint32_t)DEV_TIMEOUT_STAGE);
+        return;
+    }
     const uint32_t a_base = s0;
-    const uint32_t b_base = a_base + GEMM_A_STAGES * GEMM_A_BYTES;
-    const uint32_t lut_addr = b_base + GEMM_B_STAGES * GEMM_B_BYTES;
+    const uint32_t b_base = a_base + GEMM_A_BYTES * (uint32_t)P.a_stages;
+    const uint32_t lut_addr = b_base + P.b_stage_bytes * (uint32_t)P.b_stages;
     const uint32_t bar_base = lut_addr + GEMM_LUT_BYTES;
-    auto bar_afull = [&](int s) { return bar_base + 8u * s; };             // 3
-    auto bar_aempty = [&](int s) { return bar_base + 24u + 8u * s; };      // 3
-    auto bar_bfull = [&](int s) { return bar_base + 48u + 8u * s; };       // 2
-    auto bar_bempty = [&](int s) { return bar_base + 64u + 8u * s; };      // 2
-    const uint32_t bar_acc = bar_base + 80u;
-    const uint32_t tmem_slot = bar_base + 96u;
+    auto bar_afull = [&](uint32_t s) { return bar_base + 8u * s; };
+    auto bar_aempty = [&](uint32_t s) { return bar_base + 8u * GEMM_MAX_STAGES + 8u * s; };
+    auto bar_bfull = [&](uint32_t s) { return bar_base + 16u * GEMM_MAX_STAGES + 8u * s; };
+    auto bar_bempty = [&](uint32_t s) { return bar_base + 24u * GEMM_MAX_STAGES + 8u * s; };
+    const uint32_t bar_acc = bar_base + 32u * GEMM_MAX_STAGES;
+    const uint32_t tmem_slot = bar_acc + 8u;
 
-    const int row_tile = blockIdx.x;
+    LutEntry* const lut_s = reinterpret_cast<LutEntry*>(smem + (lut_addr - s0));
+    const uint32_t rank = cluster_rank();
+    const uint32_t leader = PAIR ? rank & ~1u : rank;                   // the CTA that issues the MMAs of a pair
+    const uint32_t half_id = PAIR ? rank & 1u : 0u;
     const int m0 = blockIdx.y * P.tok_per_cta;
     int n_tok = P.M - m0;
     if (n_tok > P.tok_per_cta) n_tok = P.tok_per_cta;
-    const int n_half0 = n_tok < GEMM_NT ? n_tok : GEMM_NT;
-    const int n_half1 = n_tok - n_half0;
-    const uint32_t n_mma0 = (uint32_t)((n_half0 + 15) & ~15), n_mma1 = (uint32_t)((n_half1 + 15) & ~15);
-    const int rb0 = row_tile * GEMM_RB;
-    int n_rb = W.RB - rb0;
-    if (n_rb > GEMM_RB) n_rb = GEMM_RB;
-    // column tiles of this split
+    // tokens of the two accumulators, and the N of their MMAs (columns beyond n_tok are computed and never read)
+    const int n_acc0 = n_tok < P.acc_tokens ? n_tok : P.acc_tokens, n_acc1 = n_tok - n_acc0;
+    constexpr int N_STEP = PAIR ? 32 : 16;
+    const uint32_t n_mma0 = (uint32_t)((n_acc0 + N_STEP - 1) / N_STEP * N_STEP), n_mma1 = (uint32_t)((n_acc1 + N_STEP - 1) / N_STEP * N_STEP);
     const int split = blockIdx.z;
-    const int ct_per = (W.CT + P.splits - 1) / P.splits;
-    const int ct_begin = split * ct_per;
-    int ct_end = ct_begin + ct_per;
-    if (ct_end > W.CT) ct_end = W.CT;
-    int my_stages = 0;
-    for (int ct = ct_begin; ct < ct_end; ++ct) my_stages += 2 * tile_width(W, ct);
+    const int g_begin = (int)((long long)P.G * split / P.splits), g_end = (int)((long long)P.G * (split + 1) / P.splits);
+    const int my_stages = 2 * (g_end - g_begin);
+
+    // the matrix of this row tile, with compares over the (at most four) slots (see gemv_kernel.cuh)
+    const int row_tile = blockIdx.x;
+    int mi = 0;
+#pragma unroll
+    for (int k = 1; k < GEMV_MAX_MATS; ++k)
+        if (k < P.n_mats && row_tile >= P.mat[k].rt_start) mi = k;
+    const int local_rt = row_tile - MAT_FIELD(mi, rt_start);
+
+    // ---- the decode warps' first requests fly during the block set-up (they touch nothing that it prepares)
+    const int r = threadIdx.x & 127;                                    // weight row within the CTA tile
+    const int row = local_rt * GEMM_ROWS + r;
+    const uint32_t half = ((uint32_t)warp >> 2) & 1u;               // columns 64*half .. of a group
+    constexpr int STEP = DW / 8;                                    // two sets of decode warps take alternate groups
+    const int set = warp >> 3;
+    const int rr = r & 15;
+    const int rb = local_rt * GEMM_RB + (r >> 4);
+    const bool have_rb = warp < DW && rb < MAT_FIELD(mi, RB);
+    const uint8_t* const tiles = MAT_FIELD(mi, tiles);
+    const uint32_t* const tile_off = MAT_FIELD(mi, tile_off) + (size_t)(have_rb ? rb : 0) * P.CT;
+    const uint2* const lut_lane = reinterpret_cast<const uint2*>(lut_s) + (lane & (GEMM_LUT_COPIES - 1));
+    const uint32_t x7 = (uint32_t)(r & 7);
+    const uint32_t rowaddr = a_base + (uint32_t)(r >> 3) * 1024u + x7 * 128u;
+    // Weight bytes are read by per-thread loads whose addresses depend on each other (tile offset -> masks -> codes), so
+    // each is requested one step ahead of its use: offsets four column tiles ahead, a tile's masks when the last group of
+    // the tile before has been taken, a group's codes while the group before is expanded.  One thread per row block
+    // asks the L2 for whole tiles, two ahead of the one requested.
+    const int ct_begin = g_begin / TILE_GROUPS, ct_end = (g_end + TILE_GROUPS - 1) / TILE_GROUPS;
+    auto offset_of = [&](int ct) { return have_rb ? __ldg(tile_off + (ct < P.CT ? ct : P.CT)) : 0u; };
+    auto prefetch_l2 = [&](int ct, uint32_t from, uint32_t to) {
+        if (have_rb && rr == 0 && warp < 4 && ct < ct_end)
+            asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(tiles + (size_t)from * 16), "r"((to - from) * 16u) : "memory");
+    };
+    uint4 mk[TILE_GROUPS];                                          // masks and scale | zero of the tile's groups from `pos` on
+    uint32_t szv[TILE_GROUPS];
+    uint32_t o0 = offset_of(ct_begin), o1 = offset_of(ct_begin + 1), o2 = offset_of(ct_begin + 2), o3 = offset_of(ct_begin + 3);
+    uint32_t codes = 0, codes_cur = 0;                              // code stream of the tile in mk / being taken from, 16-byte units
+    uint32_t off = 0;                                               // rank of this row's next survivor within the tile
+    int pos = 0;
+    auto request_tile = [&](int ct) {
+        int w = P.G - TILE_GROUPS * ct;
+        if (w > TILE_GROUPS) w = TILE_GROUPS;
+        const uint8_t* tile = tiles + (size_t)o0 * 16;
+        codes = o0 + (uint32_t)(TILE_ROWS * 20 / 16) * (uint32_t)w;
+#pragma unroll
+        for (int gi = 0; gi < TILE_GROUPS; ++gi) {
+            mk[gi] = make_uint4(0, 0, 0, 0);
+            szv[gi] = 0;
+            if (have_rb && gi < w) {
+                mk[gi] = __ldg(reinterpret_cast<const uint4*>(tile) + rr * w + gi);
+                szv[gi] = __ldg(reinterpret_cast<const uint32_t*>(tile + TILE_ROWS * w * 16) + rr * w + gi);
+            }
+        }
+        prefetch_l2(ct + 2, o2, o3);
+        o0 = o1; o1 = o2; o2 = o3;
+        o3 = offset_of(ct + 4);
+    };
+    auto count = [&](const uint4& v) { return (uint32_t)(__popc(v.x) + __popc(v.y) + __popc(v.z) + __popc(v.w)); };
+    auto settle_tile = [&]() {                                      // the masks are there: where this row's codes start
+        uint32_t cnt = 0;
+#pragma unroll
+        for (int gi = 0; gi < TILE_GROUPS; ++gi) cnt += count(mk[gi]);
+        uint32_t inc = cnt;
+#pragma unroll
+        for (int d = 1; d < 16; d <<= 1) {
+            const uint32_t up = __shfl_up_sync(full_mask, inc, d, 16);
+            if ((lane & 15) >= d) inc += up;
+        }
+        off = inc - cnt;
+        codes_cur = codes;
+        pos = 0;
+    };
+    auto skip = [&]() {                                             // the next group moves into slot 0
+        off += count(mk[0]);
+#pragma unroll
+        for (int k2 = 0; k2 + 1 < TILE_GROUPS; ++k2) { mk[k2] = mk[k2 + 1]; szv[k2] = szv[k2 + 1]; }
+        ++pos;
+    };
+    int ct_cur = -1;
+    auto take = [&](GemmFetch<BITS>& f, int g) {                    // request the codes of group g (of the matrix)
+        if (g / TILE_GROUPS != ct_cur) { ct_cur = g / TILE_GROUPS; settle_tile(); }
+        while (pos < g % TILE_GROUPS) skip();
+        f.mask[0] = half ? mk[0].z : mk[0].x;
+        f.mask[1] = half ? mk[0].w : mk[0].y;
+        f.sz = szv[0];
+        const uint32_t first = (half ? off + __popc(mk[0].x) + __popc(mk[0].y) : off) * (uint32_t)BITS;
+        f.bit = first & 127u;
+        const uint32_t end = f.bit + (uint32_t)(__popc(f.mask[0]) + __popc(f.mask[1])) * (uint32_t)BITS;
+        const uint4* p = reinterpret_cast<const uint4*>(tiles) + codes_cur + (first >> 7);
+#pragma unroll
+        for (int i = 0; i < GemmFetch<BITS>::NC; ++i)
+            if (end > f.bit && end > 128u * i) f.chunk[i] = __ldg(p + i);
+        skip();
+        const int next = g + STEP;                                  // was this the last group taken from the tile?
+        if (next < g_end && next / TILE_GROUPS != ct_cur) request_tile(next / TILE_GROUPS);
+    };
+    prefetch_l2(ct_begin + 1, o1, o2);
+    request_tile(ct_begin);
+    if ((g_begin + set) / TILE_GROUPS != ct_begin) request_tile(ct_begin + 1);          // a set that starts in the second tile
 
     if (threadIdx.x == 0) {
-        for (int s = 0; s < GEMM_A_STAGES; ++s) { mbar_init(bar_afull(s), 128); mbar_init(bar_aempty(s), 1); }
-        for (int s = 0; s < GEMM_B_STAGES; ++s) { mbar_init(bar_bfull(s), 1); mbar_init(bar_bempty(s), 1); }
+        for (uint32_t s = 0; s < GEMM_MAX_STAGES; ++s) {
+            mbar_init(bar_afull(s), PAIR ? 8 : 4); mbar_init(bar_aempty(s), 1);      // afull: one arrival per decode warp
+            mbar_init(bar_bfull(s), 1); mbar_init(bar_bempty(s), 1);
+        }
         mbar_init(bar_acc, 1);
         mbar_fence_init();
         fence_proxy_async();
     }
-    {   // expansion table replicas
-        LutEntry* lut_s = reinterpret_cast<LutEntry*>(sm + (lut_addr - s0));
-        for (int i = threadIdx.x; i < LUT_ENTRIES * GEMM_LUT_COPIES; i += GEMM_THREADS) lut_s[i] = g_lut.e[i / GEMM_LUT_COPIES];
+    if (threadIdx.x < LUT_ENTRIES) {      // expansion table: .x = selector A | view selector << 16, .y = selector B | bits consumed << 16
+        const uint4 e = gemv_lut_entry(threadIdx.x, BITS);
+#pragma unroll
+        for (int c = 0; c < GEMM_LUT_COPIES; ++c) lut_s[threadIdx.x * GEMM_LUT_COPIES + c] = LutEntry{e.x | (e.z << 16), e.y | (e.w << 16)};
     }
-    if (warp == 9) { tmem_alloc(tmem_slot, 512); tmem_relinquish(); }
+    constexpr uint32_t TMEM_COLS = PAIR ? GEMM_PAIR_TOKENS : GEMM_SINGLE_TOKENS;
+    if (warp == DW + 1) { tmem_alloc<PAIR>(tmem_slot, TMEM_COLS); tmem_relinquish<PAIR>(); }
     tc_fence_before();
-    __syncthreads();
+    __syncwarp();
+    if (PAIR) cluster_sync_all();                                       // the other CTA's barriers are in place before anyone arrives on them
+    else __syncthreads();
     tc_fence_after();
     const uint32_t tmem_d = lds32(tmem_slot);
 
-    if (warp < 8) {
-        // =========================================================== decode + epilogue
-        const int group = warp >> 2;                      // takes stages with (q & 1) == group
-        const int r = threadIdx.x & 127;                  // weight row within the CTA tile
-        const int rbl = r >> 4, rr = r & 15;
-        const bool have_rb = rbl < n_rb;
-        const uint32_t lut_lane = lut_addr + (uint32_t)(lane & (GEMM_LUT_COPIES - 1)) * 8u;
-        const LutEntry* lut_lane_ptr = reinterpret_cast<const LutEntry*>(sm + (lut_addr - s0)) + (lane & (GEMM_LUT_COPIES - 1));
-        auto lut = [lut_lane](uint32_t idx) {
-            const uint2 e = lds64(lut_lane + idx * (GEMM_LUT_COPIES * 8u));
-            return LutEntry{e.x, e.y};
-        };
-        bool healthy = true;
-        int q = 0;                                        // stage counter of this CTA (both groups count every stage)
-        // Weight bytes are read by per-thread loads whose addresses depend on each other (tile offset -> masks -> code
-        // windows).  One thread per row block asks the L2 for whole tiles two column tiles ahead, so that those loads
-        // find their lines in the cache instead of paying a DRAM round trip each.
-        auto prefetch_tile = [&](int ct) {
-            if (have_rb && rr == 0 && group == 0 && ct < ct_end) {
-                const uint32_t* to = W.tile_off + (size_t)(rb0 + rbl) * W.CT + ct;
-                const uint32_t o0 = __ldg(to), o1 = __ldg(to + 1);
-                asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(W.tiles + (size_t)o0 * 16), "r"((o1 - o0) * 16u) : "memory");
+    bool healthy = true;
+    if (warp < DW) {
+        // =========================================================== decode
+        GemmFetch<BITS> cur = {};
+        if (g_begin + set < g_end) take(cur, g_begin + set);
+        uint32_t s = 2u * (uint32_t)set + half, ph = 0;                 // slot and phase of the stage: group n of the CTA is stages 2n, 2n + 1
+#pragma unroll 1
+        for (int g = g_begin + set; g < g_end; g += STEP) {
+            GemmFetch<BITS> nxt = {};
+            if (g + STEP < g_end) take(nxt, g + STEP);
+            const SegParams sp = make_seg_params(cur.sz, BITS, false);
+            uint32_t words[4 * GemmFetch<BITS>::NC];
+#pragma unroll
+            for (int i = 0; i < GemmFetch<BITS>::NC; ++i) {
+                words[4 * i] = cur.chunk[i].x; words[4 * i + 1] = cur.chunk[i].y;
+                words[4 * i + 2] = cur.chunk[i].z; words[4 * i + 3] = cur.chunk[i].w;
             }
-        };
-        prefetch_tile(ct_begin);
-        prefetch_tile(ct_begin + 1);
-        for (int ct = ct_begin; ct < ct_end && healthy; ++ct) {
-            const int w = tile_width(W, ct);
-            prefetch_tile(ct + 2);
-            // this row's segments, and where its codes start inside the tile
-            uint4 mk[TILE_GROUPS];
-            uint32_t szv[TILE_GROUPS];
-            uint32_t cnt = 0;
-            const uint32_t* codes = nullptr;
-            if (have_rb) {
-                const uint8_t* tile = W.tiles + (size_t)__ldg(W.tile_off + (size_t)(rb0 + rbl) * W.CT + ct) * 16;
-                codes = reinterpret_cast<const uint32_t*>(tile + TILE_ROWS * w * 20);
+            const uint32_t bit1 = cur.bit + (uint32_t)__popc(cur.mask[0]) * (uint32_t)BITS;
+            healthy = __all_sync(full_mask, mbar_wait_bounded(bar_aempty(s), ph ^ 1u, P.status, DEV_TIMEOUT_EMPTY));
+            if (!healthy) break;
+            const uint32_t dst = rowaddr + s * GEMM_A_BYTES;
+            const int col = g * GROUP + (int)half * 64;
 #pragma unroll
-                for (int gi = 0; gi < TILE_GROUPS; ++gi) {
-                    mk[gi] = make_uint4(0, 0, 0, 0);
-                    szv[gi] = 0;
-                    if (gi < w) {
-                        mk[gi] = __ldg(reinterpret_cast<const uint4*>(tile) + rr * w + gi);
-                        szv[gi] = __ldg(reinterpret_cast<const uint32_t*>(tile + TILE_ROWS * w * 16) + rr * w + gi);
-                        cnt += __popc(mk[gi].x) + __popc(mk[gi].y) + __popc(mk[gi].z) + __popc(mk[gi].w);
-                    }
-                }
-            } else {
-#pragma unroll
-                for (int gi = 0; gi < TILE_GROUPS; ++gi) { mk[gi] = make_uint4(0, 0, 0, 0); szv[gi] = 0; }
-            }
-            uint32_t inc = cnt;
-#pragma unroll
-            for (int d = 1; d < 16; d <<= 1) {
-                const uint32_t up = __shfl_up_sync(full_mask, inc, d, 16);
-                if ((lane & 15) >= d) inc += up;
-            }
-            uint32_t off = inc - cnt;                      // rank of this row's first survivor within the tile
-
-            const int nks = 2 * w;                         // 64-column stages in this column tile
-            for (int ks = 0; ks < nks; ++ks, ++q) {
-                const uint32_t m0w = (ks & 1) ? mk[0].z : mk[0].x;
-                const uint32_t m1w = (ks & 1) ? mk[0].w : mk[0].y;
-                const uint32_t sz_cur = szv[0];
-                const uint32_t off0 = off, off1 = off + __popc(m0w);
-                off = off1 + __popc(m1w);
-                if (ks & 1) {                              // group finished: rotate the next one into slot 0
-#pragma unroll
-                    for (int k2 = 0; k2 + 1 < TILE_GROUPS; ++k2) { mk[k2] = mk[k2 + 1]; szv[k2] = szv[k2 + 1]; }
-                }
-                if ((q & 1) != group) continue;            // the other group's stage
-                uint32_t raw0[5] = {0, 0, 0, 0, 0}, raw1[5] = {0, 0, 0, 0, 0};
-                if (have_rb) {
-                    fetch_window<BITS>(codes, off0, raw0);
-                    fetch_window<BITS>(codes, off1, raw1);
-                }
-                const SegParams sp = make_seg_params(sz_cur, BITS, W.col_scale != nullptr);
-                uint32_t e0[16], e1[16];
-                uint32_t w0, w1, w2, w3;
-                const int col = (ct * TILE_GROUPS + (ks >> 1)) * GROUP + (ks & 1) * 64;
+            for (int h = 0; h < 2; ++h) {
+                const uint32_t o = h ? bit1 : cur.bit;
                 if (sp.fast) {
-                    align_window<BITS>(raw0, off0, w0, w1, w2, w3);
-                    decode32_fast(m0w, w0, w1, w2, w3, sp, lut, e0);
-                    align_window<BITS>(raw1, off1, w0, w1, w2, w3);
-                    decode32_fast(m1w, w0, w1, w2, w3, sp, lut, e1);
-                } else {
+                    uint2 lut[4];                                       // table entries first: their latencies overlap
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) lut[c] = lut_lane[((cur.mask[h] >> (8 * c)) & 0xFFu) * GEMM_LUT_COPIES];
+                    uint32_t raw[BITS + 1], win[BITS];                  // codes of the word, first survivor in the low bits of win[0]
+                    if (h) pick_words<4 * GemmFetch<BITS>::NC, BITS + 1, true>(words, o >> 5, raw);
+                    else pick_words<4 * GemmFetch<BITS>::NC, BITS + 1, false>(words, o >> 5, raw);
+#pragma unroll
+                    for (int i = 0; i < BITS; ++i) win[i] = funnel_r(raw[i], raw[i + 1], o);
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) {
+                        const uint2 e = lut[c];
+                        uint32_t out[4];
+                        if (SCALED) {
+                            const uint4 cv = __ldg(reinterpret_cast<const uint4*>(P.col_scale + col + 32 * h) + c);
+                            const uint32_t cw[4] = {cv.x, cv.y, cv.z, cv.w};
+                            float cs[8];
+#pragma unroll
+                            for (int i = 0; i < 4; ++i) { cs[2 * i] = half_bits_to_float(cw[i]); cs[2 * i + 1] = half_bits_to_float(cw[i] >> 16); }
+                            decode8_scaled<BITS>((cur.mask[h] >> (8 * c)) & 0xFFu, win[0], e.x, e.y, e.x >> 16, sp, cs, out);
+                        } else {
+                            decode8<BITS>(win[0], e.x, e.y, e.x >> 16, sp, out);
+                        }
+                        sts128(dst + (((uint32_t)(4 * h + c) ^ x7) << 4), out[0], out[1], out[2], out[3]);
+                        if (c < 3) {
+                            const uint32_t amt = e.y >> 16;             // at most 32 bits
+#pragma unroll
+                            for (int i = 0; i + 1 < BITS; ++i) win[i] = funnel_rc(win[i], win[i + 1], amt);
+                            win[BITS - 1] = funnel_rc(win[BITS - 1], 0u, amt);
+                        }
+                    }
+                } else {                                                // literal fp32 path (off-grid zero point, scale not finite)
                     float cs[32];
-                    const float* csp = nullptr;
-                    if (W.col_scale != nullptr) {
-                        for (int i = 0; i < 32; ++i) cs[i] = half_bits_to_float(W.col_scale[col + i]);
-                        csp = cs;
-                    }
-                    align_window<BITS>(raw0, off0, w0, w1, w2, w3);
-                    decode32<GEMM_LUT_COPIES>(m0w, w0, w1, w2, w3, sp, lut_lane_ptr, csp, e0);
-                    if (W.col_scale != nullptr)
-                        for (int i = 0; i < 32; ++i) cs[i] = half_bits_to_float(W.col_scale[col + 32 + i]);
-                    align_window<BITS>(raw1, off1, w0, w1, w2, w3);
-                    decode32<GEMM_LUT_COPIES>(m1w, w0, w1, w2, w3, sp, lut_lane_ptr, csp, e1);
-                }
-                const int s = q % GEMM_A_STAGES;
-                healthy = __all_sync(full_mask, mbar_wait_bounded(bar_aempty(s), (((uint32_t)(q / GEMM_A_STAGES)) & 1u) ^ 1u,
-                                                                  P.status, DEV_TIMEOUT_EMPTY));
-                if (!healthy) break;
-                const uint32_t rowaddr = a_base + s * GEMM_A_BYTES + (uint32_t)(r >> 3) * 1024u + (uint32_t)(r & 7) * 128u;
-                const uint32_t x7 = (uint32_t)(r & 7);
-#pragma unroll
-                for (int c = 0; c < 4; ++c) {
-                    sts128(rowaddr + (((uint32_t)c ^ x7) << 4), e0[4 * c], e0[4 * c + 1], e0[4 * c + 2], e0[4 * c + 3]);
-                    sts128(rowaddr + (((uint32_t)(c + 4) ^ x7) << 4), e1[4 * c], e1[4 * c + 1], e1[4 * c + 2], e1[4 * c + 3]);
-                }
-                fence_proxy_async();
-                mbar_arrive(bar_afull(s));
-            }
-        }
-        // ---- epilogue: TMEM lane = weight row; warp w drains accumulator w/4
-        if (healthy && my_stages > 0) healthy = __all_sync(full_mask, mbar_wait_bounded(bar_acc, 0u, P.status, DEV_TIMEOUT_ACC));
-        tc_fence_after();
-        const int row = row_tile * GEMM_ROWS + r;
-        const int acc_id = group;
-        const int ntok_acc = acc_id ? n_half1 : n_half0;
-        const uint32_t nmma_acc = acc_id ? n_mma1 : n_mma0;
-        const int tok_base = m0 + acc_id * GEMM_NT;
-        const uint32_t tile_id = blockIdx.y * gridDim.x + blockIdx.x;
-        float* part = P.partials ? P.partials + ((size_t)tile_id * P.splits + split) * ((size_t)GEMM_TOKENS * GEMM_ROWS) : nullptr;
-        if (healthy) {
-            for (uint32_t c0 = 0; c0 < nmma_acc; c0 += 32) {
-                uint32_t v[32];
-                if (my_stages > 0) {
-                    tmem_ld32(tmem_d + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(acc_id * GEMM_NT) + c0, v);
-                    tmem_ld_wait();
-                } else {
-#pragma unroll
-                    for (int i = 0; i < 32; ++i) v[i] = 0u;
-                }
-                if (P.splits == 1) {
-                    if (row < W.K) {
-#pragma unroll
-                        for (int i = 0; i < 32; ++i) {
-                            const int tk = (int)c0 + i;
-                            if (tk < ntok_acc) {
-                                if (P.y32) P.y32[(size_t)(tok_base + tk) * P.ldy + row] = __uint_as_float(v[i]);
-                                else P.y[(size_t)(tok_base + tk) * P.ldy + row] = finish_output(__uint_as_float(v[i]), P.bias, row);
-                            }
-                        }
-                    }
-                } else {
-#pragma unroll
-                    for (int i = 0; i < 32; ++i) {
-                        const int tk = (int)c0 + i;
-                        if (tk < ntok_acc) part[(size_t)(acc_id * GEMM_NT + tk) * GEMM_ROWS + r] = __uint_as_float(v[i]);
-                    }
+                    if (SCALED)
+                        for (int i = 0; i < 32; ++i) cs[i] = half_bits_to_float(P.col_scale[col + 32 * h + i]);
+                    uint32_t e[16];
+                    decode32_slow(cur.mask[h], [&](uint32_t k) { return words[k]; }, o, BITS, sp, SCALED ? cs : nullptr, e);
+                    for (int c = 0; c < 4; ++c)
+                        sts128(dst + (((uint32_t)(4 * h + c) ^ x7) << 4), e[4 * c], e[4 * c + 1], e[4 * c + 2], e[4 * c + 3]);
                 }
             }
-        }
-        tc_fence_before();
-        if (P.splits > 1) {
-            // the last split to arrive adds all splits in order and writes the outputs
-            __threadfence();
-            asm volatile("bar.sync 1, 256;" ::: "memory");            // the 8 decode warps only
-            if (threadIdx.x == 0) sts32(bar_base + 104u, atomicAdd(&P.counters[tile_id], 1u));
-            asm volatile("bar.sync 1, 256;" ::: "memory");
-            if (lds32(bar_base + 104u) == (uint32_t)(P.splits - 1) && healthy) {
-                __threadfence();
-                const float* base = P.partials + (size_t)tile_id * P.splits * ((size_t)GEMM_TOKENS * GEMM_ROWS);
-                if (row < W.K) {
-                    // eight tokens x four splits of loads in flight per thread: one thread per row walks up to 256 tokens,
-                    // and a token at a time would be one L2 latency per token (the whole cost of a small-M launch)
-                    constexpr int TU = 8, KU = 4;
-                    const size_t split_stride = (size_t)GEMM_TOKENS * GEMM_ROWS;
-                    for (int tk0 = 0; tk0 < ntok_acc; tk0 += TU) {
-                        float sum[TU];
-#pragma unroll
-                        for (int j = 0; j < TU; ++j) sum[j] = 0.0f;
-                        for (int k0 = 0; k0 < P.splits; k0 += KU) {
-                            float v[KU][TU];
-#pragma unroll
-                            for (int kk = 0; kk < KU; ++kk)
-#pragma unroll
-                                for (int j = 0; j < TU; ++j) {
-                                    const int tk = tk0 + j < ntok_acc ? tk0 + j : ntok_acc - 1;
-                                    v[kk][j] = k0 + kk < P.splits
-                                        ? __ldcg(base + (size_t)(k0 + kk) * split_stride + (size_t)(acc_id * GEMM_NT + tk) * GEMM_ROWS + r) : 0.0f;
-                                }
-#pragma unroll
-                            for (int kk = 0; kk < KU; ++kk)             // splits in order: the sum does not depend on the grid
-#pragma unroll
-                                for (int j = 0; j < TU; ++j)
-                                    if (k0 + kk < P.splits) sum[j] += v[kk][j];
-                        }
-#pragma unroll
-                        for (int j = 0; j < TU; ++j) {
-                            const int tk = tk0 + j;
-                            if (tk < ntok_acc) {
-                                if (P.y32) P.y32[(size_t)(tok_base + tk) * P.ldy + row] = sum[j];
-                                else P.y[(size_t)(tok_base + tk) * P.ldy + row] = finish_output(sum[j], P.bias, row);
-                            }
-                        }
-                    }
-                }
-                if (threadIdx.x == 0) P.counters[tile_id] = 0u;
+            fence_proxy_async();
+            __syncwarp();
+            if (lane == 0) {
+                if (PAIR) mbar_arrive_cluster(map_to_rank(bar_afull(s), leader));
+                else mbar_arrive(bar_afull(s));
             }
+            s += 2 * STEP;                                              // a_stages >= 2 * STEP: at most one turn of the ring
+            if (s >= (uint32_t)P.a_stages) { s -= (uint32_t)P.a_stages; ph ^= 1u; }
+            cur = nxt;
         }
-    } else if (warp == 8) {
+        if (healthy) healthy = __all_sync(full_mask, mbar_wait_bounded(bar_acc, 0u, P.status, DEV_TIMEOUT_ACC));
+    } else if (warp == DW) {
         // =========================================================== activation loader (TMA)
-        if (lane == 0) {
-            bool healthy = true;
-            int q = 0;
-            const uint32_t bytes = (uint32_t)GEMM_BHALF_BYTES * (n_half1 > 0 ? 2u : 1u);
-            for (int ct = ct_begin; ct < ct_end && healthy; ++ct) {
-                const int w = tile_width(W, ct);
-                for (int ks = 0; ks < 2 * w; ++ks, ++q) {
-                    const int s = q % GEMM_B_STAGES;
-                    healthy = mbar_wait_bounded(bar_bempty(s), (((uint32_t)(q / GEMM_B_STAGES)) & 1u) ^ 1u, P.status, DEV_TIMEOUT_EMPTY);
-                    if (!healthy) break;
-                    const int col = ct * TILE_GROUPS * GROUP + ks * GEMM_KS;
-                    mbar_arrive_expect_tx(bar_bfull(s), bytes);
-                    tma_load_2d(b_base + s * GEMM_B_BYTES, &xmap, col, m0, bar_bfull(s));
-                    if (n_half1 > 0) tma_load_2d(b_base + s * GEMM_B_BYTES + GEMM_BHALF_BYTES, &xmap, col, m0 + GEMM_NT, bar_bfull(s));
-                }
+        bool good = true;
+        const uint32_t bytes = P.b_acc_bytes * (n_acc1 > 0 ? 2u : 1u);
+        uint32_t s = 0, ph = 0;
+        for (uint32_t q = 0; q < (uint32_t)my_stages; ++q) {
+            good = mbar_wait_bounded(bar_bempty(s), ph ^ 1u, P.status, DEV_TIMEOUT_EMPTY);
+            if (!__all_sync(full_mask, good)) break;
+            const int col = g_begin * GROUP + (int)q * GEMM_KS;
+            // pair: each CTA loads its half of every accumulator's tokens; both count on the leader's barrier
+            const uint32_t bar = PAIR ? map_to_rank(bar_bfull(s), leader) : bar_bfull(s);
+            const uint32_t dst = b_base + s * P.b_stage_bytes;
+            if (elect_one()) {
+                if (half_id == 0) mbar_arrive_expect_tx(bar_bfull(s), PAIR ? 2u * bytes : bytes);
+                tma_load_2d<PAIR>(dst, &xmap, col, m0 + (int)(half_id * (n_mma0 / 2u)), bar);
+                if (n_acc1 > 0) tma_load_2d<PAIR>(dst + P.b_acc_bytes, &xmap, col, m0 + P.acc_tokens + (int)(half_id * (n_mma1 / 2u)), bar);
             }
+            __syncwarp();
+            if (++s == (uint32_t)P.b_stages) { s = 0; ph ^= 1u; }
         }
-        __syncwarp();
     } else {
-        // =========================================================== MMA issuer
-        if (lane == 0) {
-            const uint32_t idesc0 = umma_idesc(n_mma0), idesc1 = umma_idesc(n_mma1 ? n_mma1 : 16);
-            bool healthy = true;
-            for (int q = 0; q < my_stages && healthy; ++q) {
-                const int sa = q % GEMM_A_STAGES, sb = q % GEMM_B_STAGES;
-                healthy = mbar_wait_bounded(bar_afull(sa), ((uint32_t)(q / GEMM_A_STAGES)) & 1u, P.status, DEV_TIMEOUT_FULL);
-                if (healthy) healthy = mbar_wait_bounded(bar_bfull(sb), ((uint32_t)(q / GEMM_B_STAGES)) & 1u, P.status, DEV_TIMEOUT_STAGE);
-                if (!healthy) break;
+        // =========================================================== MMA issuer (pair: of the leader)
+        if (half_id == 0) {
+            const uint32_t idesc0 = umma_idesc(n_mma0, PAIR ? 2 * GEMM_ROWS : GEMM_ROWS), idesc1 = umma_idesc(n_mma1 ? n_mma1 : 32, PAIR ? 2 * GEMM_ROWS : GEMM_ROWS);
+            const uint16_t both = (uint16_t)(3u << leader);
+            const uint32_t d0 = tmem_d, d1 = tmem_d + (uint32_t)P.acc_tokens;
+            bool good = true;
+            uint32_t sa = 0, pa = 0, sb = 0, pb = 0;
+            for (uint32_t q = 0; q < (uint32_t)my_stages; ++q) {
+                good = mbar_wait_bounded(bar_bfull(sb), pb, P.status, DEV_TIMEOUT_STAGE);
+                if (good) good = mbar_wait_bounded(bar_afull(sa), pa, P.status, DEV_TIMEOUT_FULL);
+                good = __all_sync(full_mask, good);
+                if (!good) break;
                 tc_fence_after();
                 const uint64_t ad = umma_smem_desc(a_base + sa * GEMM_A_BYTES);
-                const uint64_t bd0 = umma_smem_desc(b_base + sb * GEMM_B_BYTES);
-                const uint64_t bd1 = umma_smem_desc(b_base + sb * GEMM_B_BYTES + GEMM_BHALF_BYTES);
-#pragma unroll
-                for (int k = 0; k < GEMM_KS / 16; ++k)
-                    umma_bf16(tmem_d, ad + (uint64_t)(2 * k), bd0 + (uint64_t)(2 * k), idesc0, (q > 0 || k > 0) ? 1u : 0u);
-                if (n_mma1) {
+                const uint64_t bd0 = umma_smem_desc(b_base + sb * P.b_stage_bytes);
+                const uint64_t bd1 = umma_smem_desc(b_base + sb * P.b_stage_bytes + P.b_acc_bytes);
+                if (elect_one()) {
 #pragma unroll
                     for (int k = 0; k < GEMM_KS / 16; ++k)
-                        umma_bf16(tmem_d + GEMM_NT, ad + (uint64_t)(2 * k), bd1 + (uint64_t)(2 * k), idesc1, (q > 0 || k > 0) ? 1u : 0u);
+                        umma_bf16<PAIR>(d0, ad + (uint64_t)(2 * k), bd0 + (uint64_t)(2 * k), idesc0, (q > 0 || k > 0) ? 1u : 0u);
+                    if (PAIR && n_mma1) {
+#pragma unroll
+                        for (int k = 0; k < GEMM_KS / 16; ++k)
+                            umma_bf16<PAIR>(d1, ad + (uint64_t)(2 * k), bd1 + (uint64_t)(2 * k), idesc1, (q > 0 || k > 0) ? 1u : 0u);
+                    }
+                    umma_commit<PAIR>(bar_aempty(sa), both);
+                    umma_commit<PAIR>(bar_bempty(sb), both);
                 }
-                umma_commit(bar_aempty(sa));
-                umma_commit(bar_bempty(sb));
+                __syncwarp();
+                if (++sa == (uint32_t)P.a_stages) { sa = 0; pa ^= 1u; }
+                if (++sb == (uint32_t)P.b_stages) { sb = 0; pb ^= 1u; }
             }
-            if (healthy && my_stages > 0) umma_commit(bar_acc);
+            if (good && elect_one()) umma_commit<PAIR>(bar_acc, both);
+            __syncwarp();
         }
-        __syncwarp();
+    }
+
+    // ---- epilogue: TMEM lane = weight row, column = token; decode warp w drains lanes 32*(w%4).., every (DW / 4)-th 32 tokens
+    const uint32_t my_tmem = tmem_d + ((uint32_t)((warp & 3) * 32) << 16);
+    const bool stores = warp < DW && healthy && row < MAT_FIELD(mi, K);
+    uint16_t* const y = MAT_FIELD(mi, y);
+    float* const y32 = MAT_FIELD(mi, y32);
+    const uint16_t* const bias = MAT_FIELD(mi, bias);
+    const int64_t ldy = MAT_FIELD(mi, ldy);
+    if (P.splits == 1) {
+        if (warp < DW && healthy) {
+            tc_fence_after();
+            for (int c0 = 32 * (warp >> 2); c0 < n_tok; c0 += 8 * DW) {
+                uint32_t v[32];
+                tmem_ld32(my_tmem + (uint32_t)c0, v);
+                tmem_ld_wait();
+                if (stores) {
+                    if (y32) {
+#pragma unroll
+                        for (int i = 0; i < 32; ++i)
+                            if (c0 + i < n_tok) y32[(size_t)(m0 + c0 + i) * ldy + row] = __uint_as_float(v[i]);
+                    } else {
+#pragma unroll
+                        for (int i = 0; i < 32; ++i)
+                            if (c0 + i < n_tok) y[(size_t)(m0 + c0 + i) * ldy + row] = finish_output(__uint_as_float(v[i]), bias, row);
+                    }
+                }
+            }
+        }
+    } else {
+        // split-K, in rounds of RED tokens: every CTA of the cluster parks its sums (the operand stages are free by now) and adds
+        // its share of the tokens over all splits, in split order
+        constexpr int RED = gemm_red_tokens(PAIR);
+        float* red = reinterpret_cast<float*>(smem);
+        const int row0 = local_rt * GEMM_ROWS + 4 * lane, K = MAT_FIELD(mi, K);
+        const bool wide = row0 + 3 < K && (ldy & 3) == 0 && ((uintptr_t)y & 7) == 0 && ((uintptr_t)y32 & 15) == 0;
+        for (int t0 = 0; t0 < n_tok; t0 += RED) {
+            const int nt = n_tok - t0 < RED ? n_tok - t0 : RED;
+            if (warp < DW && healthy) {
+                tc_fence_after();
+                for (int c0 = 32 * (warp >> 2); c0 < nt; c0 += 8 * DW) {
+                    uint32_t v[32];
+                    tmem_ld32(my_tmem + (uint32_t)(t0 + c0), v);
+                    tmem_ld_wait();
+#pragma unroll
+                    for (int i = 0; i < 32; ++i) red[(c0 + i) * GEMM_ROWS + r] = __uint_as_float(v[i]);
+                }
+            }
+            __syncwarp();
+            cluster_sync_all();
+            if (warp < DW && healthy) {                                 // a lane takes four rows, a warp every DW-th token
+                const int per = (nt + P.splits - 1) / P.splits;
+                const int tk_end = min(nt, per * (split + 1));
+                uint32_t src[GEMM_MAX_SPLITS];
+#pragma unroll
+                for (int s = 0; s < GEMM_MAX_SPLITS; ++s)
+                    src[s] = map_to_rank(s0, s < P.splits ? (PAIR ? (rank & 1u) + 2u * s : (uint32_t)s) : rank) + (uint32_t)lane * 16u;
+#pragma unroll 2
+                for (int tk = per * split + warp; tk < tk_end; tk += DW) {
+                    float4 v[GEMM_MAX_SPLITS];
+#pragma unroll
+                    for (int s = 0; s < GEMM_MAX_SPLITS; ++s)
+                        if (s < P.splits) v[s] = ld_cluster_f4(src[s] + (uint32_t)tk * (GEMM_ROWS * 4u));
+                    float sum[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll
+                    for (int s = 0; s < GEMM_MAX_SPLITS; ++s)
+                        if (s < P.splits) { sum[0] += v[s].x; sum[1] += v[s].y; sum[2] += v[s].z; sum[3] += v[s].w; }
+                    const size_t at = (size_t)(m0 + t0 + tk) * ldy + row0;
+                    if (y32) {
+                        if (wide) *reinterpret_cast<float4*>(y32 + at) = make_float4(sum[0], sum[1], sum[2], sum[3]);
+                        else
+                            for (int i = 0; i < 4; ++i)
+                                if (row0 + i < K) y32[at + i] = sum[i];
+                    } else if (wide) {
+                        uint2 o;
+                        o.x = finish_output(sum[0], bias, row0) | ((uint32_t)finish_output(sum[1], bias, row0 + 1) << 16);
+                        o.y = finish_output(sum[2], bias, row0 + 2) | ((uint32_t)finish_output(sum[3], bias, row0 + 3) << 16);
+                        *reinterpret_cast<uint2*>(y + at) = o;
+                    } else {
+                        for (int i = 0; i < 4; ++i)
+                            if (row0 + i < K) y[at + i] = finish_output(sum[i], bias, row0 + i);
+                    }
+                }
+            }
+            __syncwarp();
+            cluster_sync_all();                                         // nobody overwrites or leaves while a neighbour still reads
+        }
     }
     tc_fence_before();
-    __syncthreads();
-    if (warp == 9) { tc_fence_after(); tmem_dealloc(tmem_d, 512); }
+    __syncwarp();
+    if (PAIR) cluster_sync_all();                                       // the pair frees its tensor memory together
+    else __syncthreads();
+    if (warp == DW + 1) { tc_fence_after(); tmem_dealloc<PAIR>(tmem_d, TMEM_COLS); }
 }
 
 }  // namespace cb

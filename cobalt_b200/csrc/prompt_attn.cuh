@@ -118,7 +118,7 @@ __global__ void __launch_bounds__(PA_THREADS, 1) prompt_attn_kernel(const Prompt
         mbar_fence_init();
         fence_proxy_async();
     }
-    if (warp == 9) { tmem_alloc(tmem_slot, 512); tmem_relinquish(); }
+    if (warp == 9) { tmem_alloc<false>(tmem_slot, 512); tmem_relinquish<false>(); }
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -233,76 +233,84 @@ __global__ void __launch_bounds__(PA_THREADS, 1) prompt_attn_kernel(const Prompt
         tc_fence_before();
     } else if (warp == 8) {
         // =========================================================== TMA
-        if (lane == 0) {
+        // (loops on the whole warp, the instructions elected: see elect_one())
+        if (elect_one()) {
             mbar_arrive_expect_tx(bar_q, (uint32_t)(P.rep * P.tok_per_cta) * 128u * SUBS);
             for (int c = 0; c < SUBS; ++c) tma_load_3d(q_base + c * PA_SUB, &qmap, 64 * c, kvh * P.rep, tok0, bar_q);
-            bool healthy = true;
-            int slot = 0;
-            auto load = [&](const CUtensorMap* map, int jt) {
-                const int s = slot % PA_RING;
-                healthy = healthy && mbar_wait_bounded(bar_empty(s), ((uint32_t)(slot / PA_RING) & 1u) ^ 1u, P.status, DEV_TIMEOUT_EMPTY);
-                if (!healthy) return;
-                mbar_arrive_expect_tx(bar_full(s), TILE);
-                for (int c = 0; c < SUBS; ++c) tma_load_3d(ring + s * TILE + c * PA_SUB, map, 64 * c, jt * PA_KEYS, kvh, bar_full(s));
-                ++slot;
-            };
-            for (int j = 0; j < n && healthy; ++j) load(&kmap, t_lo + j);
-            for (int j = 0; j <= n && healthy; ++j) {                   // K0, K1, V0, K2, V1, ..., V(n-1)
-                if (j < n) load(&kmap, t_lo + j);
-                if (j > 0) load(&vmap, t_lo + j - 1);
-            }
         }
         __syncwarp();
+        bool healthy = true;
+        uint32_t s = 0, ph = 0;
+        auto load = [&](const CUtensorMap* map, int jt) {
+            healthy = __all_sync(full_mask, healthy && mbar_wait_bounded(bar_empty(s), ph ^ 1u, P.status, DEV_TIMEOUT_EMPTY));
+            if (!healthy) return;
+            if (elect_one()) {
+                mbar_arrive_expect_tx(bar_full(s), TILE);
+#pragma unroll
+                for (int c = 0; c < SUBS; ++c) tma_load_3d(ring + s * TILE + c * PA_SUB, map, 64 * c, jt * PA_KEYS, kvh, bar_full(s));
+            }
+            __syncwarp();
+            if (++s == PA_RING) { s = 0; ph ^= 1u; }
+        };
+        for (int j = 0; j < n && healthy; ++j) load(&kmap, t_lo + j);
+        for (int j = 0; j <= n && healthy; ++j) {                       // K0, K1, V0, K2, V1, ..., V(n-1)
+            if (j < n) load(&kmap, t_lo + j);
+            if (j > 0) load(&vmap, t_lo + j - 1);
+        }
     } else {
         // =========================================================== MMA
-        if (lane == 0) {
-            const uint32_t idesc_s = umma_idesc(PA_KEYS);
-            const uint32_t idesc_o = umma_idesc(D) | (1u << 16);        // B (= V) is N-major
-            bool healthy = mbar_wait_bounded(bar_q, 0u, P.status, DEV_TIMEOUT_STAGE);
-            int slot = 0;
-            auto take = [&]() {                                         // next tile of the ring
-                const int s = slot % PA_RING;
-                healthy = healthy && mbar_wait_bounded(bar_full(s), (uint32_t)(slot / PA_RING) & 1u, P.status, DEV_TIMEOUT_STAGE);
-                ++slot;
-                return s;
-            };
-            auto issue_scores = [&](int g) {
-                const int s = take();
-                healthy = healthy && mbar_wait_bounded(bar_sempty(g & 1), ((uint32_t)(g >> 1) & 1u) ^ 1u, P.status, DEV_TIMEOUT_EMPTY);
-                if (!healthy) return;
-                tc_fence_after();
+        const uint32_t idesc_s = umma_idesc(PA_KEYS);
+        const uint32_t idesc_o = umma_idesc(D) | (1u << 16);            // B (= V) is N-major
+        bool healthy = __all_sync(full_mask, mbar_wait_bounded(bar_q, 0u, P.status, DEV_TIMEOUT_STAGE));
+        uint32_t s = 0, ph = 0;
+        const uint64_t qd = umma_smem_desc(q_base);
+        auto issue_scores = [&](int g) {
+            healthy = healthy && mbar_wait_bounded(bar_full(s), ph, P.status, DEV_TIMEOUT_STAGE);
+            healthy = __all_sync(full_mask, healthy && mbar_wait_bounded(bar_sempty(g & 1), ((uint32_t)(g >> 1) & 1u) ^ 1u, P.status, DEV_TIMEOUT_EMPTY));
+            if (!healthy) return;
+            tc_fence_after();
+            const uint64_t kd = umma_smem_desc(ring + s * TILE);
+            const uint32_t d = tmem + (uint32_t)((g & 1) * PA_KEYS);
+            if (elect_one()) {
 #pragma unroll
                 for (int k = 0; k < D / 16; ++k) {
-                    const uint32_t off = (uint32_t)(k / 4) * PA_SUB + (uint32_t)(k % 4) * 32u;
-                    umma_bf16(tmem + (uint32_t)((g & 1) * PA_KEYS), umma_smem_desc(q_base + off), umma_smem_desc(ring + s * TILE + off), idesc_s, k > 0 ? 1u : 0u);
+                    const uint64_t off = (uint64_t)((k / 4) * (PA_SUB >> 4) + (k % 4) * 2);
+                    umma_bf16<false>(d, qd + off, kd + off, idesc_s, k > 0 ? 1u : 0u);
                 }
-                umma_commit(bar_empty(s));
-                umma_commit(bar_sfull(g & 1));
-            };
-            auto issue_context = [&](int j) {
-                const int s = take();
-                healthy = healthy && mbar_wait_bounded(bar_pfull(j & 1), (uint32_t)(j >> 1) & 1u, P.status, DEV_TIMEOUT_FULL);
-                if (!healthy) return;
-                tc_fence_after();
+                umma_commit<false>(bar_empty(s));
+                umma_commit<false>(bar_sfull(g & 1));
+            }
+            __syncwarp();
+            if (++s == PA_RING) { s = 0; ph ^= 1u; }
+        };
+        auto issue_context = [&](int j) {
+            healthy = healthy && mbar_wait_bounded(bar_full(s), ph, P.status, DEV_TIMEOUT_STAGE);
+            healthy = __all_sync(full_mask, healthy && mbar_wait_bounded(bar_pfull(j & 1), (uint32_t)(j >> 1) & 1u, P.status, DEV_TIMEOUT_FULL));
+            if (!healthy) return;
+            tc_fence_after();
+            const uint64_t pd = umma_smem_desc(p_base + (uint32_t)(j & 1) * PA_P_BYTES), vd = umma_smem_desc_mn(ring + s * TILE, PA_SUB);
+            if (elect_one()) {
 #pragma unroll
                 for (int k = 0; k < PA_KEYS / 16; ++k)
-                    umma_bf16(tmem_o, umma_smem_desc(p_base + (uint32_t)(j & 1) * PA_P_BYTES + (uint32_t)(k / 4) * PA_SUB + (uint32_t)(k % 4) * 32u),
-                              umma_smem_desc_mn(ring + s * TILE + (uint32_t)k * 2048u, PA_SUB), idesc_o, (j > 0 || k > 0) ? 1u : 0u);
-                umma_commit(bar_empty(s));
-                umma_commit(bar_pempty(j & 1));
-            };
-            for (int g = 0; g < n && healthy; ++g) issue_scores(g);
-            for (int j = 0; j <= n && healthy; ++j) {
-                if (j < n) issue_scores(n + j);
-                if (j > 0) issue_context(j - 1);
+                    umma_bf16<false>(tmem_o, pd + (uint64_t)((k / 4) * (PA_SUB >> 4) + (k % 4) * 2), vd + (uint64_t)(k * (2048 >> 4)), idesc_o,
+                                     (j > 0 || k > 0) ? 1u : 0u);
+                umma_commit<false>(bar_empty(s));
+                umma_commit<false>(bar_pempty(j & 1));
             }
-            if (healthy) umma_commit(bar_o);
+            __syncwarp();
+            if (++s == PA_RING) { s = 0; ph ^= 1u; }
+        };
+        for (int g = 0; g < n && healthy; ++g) issue_scores(g);
+        for (int j = 0; j <= n && healthy; ++j) {
+            if (j < n) issue_scores(n + j);
+            if (j > 0) issue_context(j - 1);
         }
+        if (healthy && elect_one()) umma_commit<false>(bar_o);
         __syncwarp();
     }
     tc_fence_before();
     __syncthreads();
-    if (warp == 9) { tc_fence_after(); tmem_dealloc(tmem, 512); }
+    if (warp == 9) { tc_fence_after(); tmem_dealloc<false>(tmem, 512); }
 }
 
 }  // namespace cb

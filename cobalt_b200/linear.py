@@ -285,8 +285,8 @@ class CobaltSparseLinear(nn.Module):
 
 class FusedProjections:
     """Several ``CobaltSparseLinear`` that read the same activations (q|k|v, gate|up), evaluated with one
-    GEMV launch for up to 16 tokens (``cobalt_gemv_fused``) and one call each above that.  The reference
-    reaches the same goal by concatenating the matrices row-wise at pack time (docs/FORMAT.md:126-151)."""
+    launch: the decode GEMV for up to 16 tokens (``cobalt_gemv_fused``), the tcgen05 GEMM above that
+    (``cobalt_gemm_fused``).  The reference reaches the same goal by concatenating the matrices row-wise at pack time (docs/FORMAT.md:126-151)."""
 
     def __init__(self, mods):
         mods = list(mods)
@@ -303,7 +303,8 @@ class FusedProjections:
         lib = _lib.load()
         n = len(self.mods)
         descs = (ctypes.POINTER(_lib.CobaltMat) * n)(*[ctypes.pointer(m._descriptor()) for m in self.mods])
-        need = lib.cobalt_gemv_fused_scratch_bytes(n, descs, GEMV_MAX_TOKENS)   # fixed size: the address survives graph capture
+        # fixed size: the address survives graph capture; one buffer serves the GEMV and the GEMM (status word, counters)
+        need = max(lib.cobalt_gemv_fused_scratch_bytes(n, descs, GEMV_MAX_TOKENS), lib.cobalt_gemm_fused_scratch_bytes(n, descs, max(M, 1)))
         if need == 0:
             raise _lib.CobaltError("cobalt_gemv_fused_scratch_bytes", -1, "could not size the scratch buffer")
         if self._scratch is None or self._scratch.numel() < need + 256 or self._scratch.device != device:
@@ -314,9 +315,11 @@ class FusedProjections:
         lead = x.shape[:-1]
         x2 = x.reshape(-1, self.mods[0].in_features)
         M = x2.shape[0]
-        if M > GEMV_MAX_TOKENS or M == 0:
+        if M == 0:
             return [m(x) for m in self.mods]
         if not x2.is_cuda or x2.dtype != torch.bfloat16:
+            if M > GEMV_MAX_TOKENS:
+                return [m(x) for m in self.mods]             # raises what a module raises
             raise TypeError("FusedProjections needs a bf16 CUDA tensor")
         if x2.stride(-1) != 1 or x2.stride(0) % 8 or x2.data_ptr() % 16:
             x2 = x2.contiguous()
@@ -327,10 +330,11 @@ class FusedProjections:
         yp = (ctypes.c_void_p * n)(*[y.data_ptr() for y in ys])
         ld = (ctypes.c_int64 * n)(*[y.stride(0) for y in ys])
         sp = (self._scratch.data_ptr() + 255) // 256 * 256
-        rc = lib.cobalt_gemv_fused(n, descs, x2.data_ptr(), x2.stride(0), yp, ld, None, M, sp,
-                                   self._scratch.numel() - (sp - self._scratch.data_ptr()),
-                                   torch.cuda.current_stream(x.device).cuda_stream)
-        _lib.check("cobalt_gemv_fused", rc)
+        name = "cobalt_gemv_fused" if M <= GEMV_MAX_TOKENS else "cobalt_gemm_fused"
+        rc = getattr(lib, name)(n, descs, x2.data_ptr(), x2.stride(0), yp, ld, None, M, sp,
+                                self._scratch.numel() - (sp - self._scratch.data_ptr()),
+                                torch.cuda.current_stream(x.device).cuda_stream)
+        _lib.check(name, rc)
         return [y.reshape(*lead, m.out_features) for y, m in zip(ys, self.mods)]
 
     def staged(self, kind: int, a: torch.Tensor, b: Optional[torch.Tensor], flavor: int, w: Optional[torch.Tensor] = None,

@@ -197,6 +197,13 @@ int cobalt_gemm(const CobaltMat* w, const void* x, int64_t ldx, void* y, int64_t
                 const void* bias, int M, void* scratch, size_t scratch_bytes, void* stream);
 size_t cobalt_gemm_scratch_bytes(const CobaltMat* w, int M);
 
+/* Prefill GEMM of up to four matrices that read the same activations (q|k|v, gate|up) as one launch: equal in_features and
+ * bit width, no column scale; y[i], ldy[i], bias[i] (bias or its entries may be NULL) per matrix.  Same results as cobalt_gemm()
+ * up to the order in which fp32 sums are added; the 128-row tiles of all matrices fill the GPU together. */
+int cobalt_gemm_fused(int n_mats, const CobaltMat* const* w, const void* x, int64_t ldx, void* const* y, const int64_t* ldy,
+                      const void* const* bias, int M, void* scratch, size_t scratch_bytes, void* stream);
+size_t cobalt_gemm_fused_scratch_bytes(int n_mats, const CobaltMat* const* w, int M);
+
 /* Same product with the raw fp32 sums as output (no bias, no rounding): M <= 16 runs the GEMV,
  * larger M the GEMM.  For row-parallel tensor-parallel layers, whose partial outputs are added
  * across GPUs before the single rounding to bf16.  Scratch as for the kernel that runs.

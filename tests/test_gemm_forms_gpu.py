@@ -1,0 +1,87 @@
+"""Both forms of the prompt GEMM (single CTAs and CTA pairs), its split columns and its fused launch (needs a B200).
+
+Reference: the fp64 product with ``dequantize()`` (bit-exact against the oracle in test_kernels_gpu.py).  Tolerance, per element: one
+bf16 spacing (2^-7 of the magnitude at most) for every rounding - of the product, and with a bias of the sum with it, whose
+magnitudes differ when the bias cancels the product - plus 1e-4 of the largest value for fp32 sums in another order (5e-5
+seen over 14336 columns).
+"""
+import pytest
+import torch
+
+from cobalt_b200 import CobaltSparseLinear
+from cobalt_b200.compress import quantize_survivors
+from cobalt_b200.linear import FusedProjections
+
+pytestmark = pytest.mark.gpu
+
+
+def module(K, N, bits, sparsity=0.5, scale2=None, bias=False, seed=0, zero_shift=0.0):
+    g = torch.Generator(device="cuda").manual_seed(seed + K + N)
+    W = (torch.randn(K, N, generator=g, device="cuda") * 0.02).half().float()
+    keep = torch.rand(K, N, generator=g, device="cuda") > sparsity
+    q, s, z = quantize_survivors(W, keep, bits)
+    z = z.clone()
+    z[::3, ::2] += zero_shift                                    # 0.5: zero points off the integer grid
+    b = (torch.randn(K, generator=g, device="cuda") * 0.1).bfloat16() if bias else None
+    return CobaltSparseLinear(q, s, z, keep, scale2, b, {"nbits": bits})
+
+
+def check(m, x, y):
+    exact = x.double() @ m.dequantize().double().t()
+    bound = exact.abs() * 2.0 ** -7 + exact.abs().max() * 1e-4
+    if m.bias is not None:
+        exact = exact.to(torch.bfloat16).double() + m.bias.double()
+        bound = bound + exact.abs() * 2.0 ** -7
+    d = (y.double() - exact).abs()
+    assert m.device_status() == 0
+    assert bool((d <= bound).all()), float((d - bound).max())
+    assert float(d.norm() / exact.norm()) <= 2.0 ** -8
+
+
+def tokens(M, N, seed=1):
+    return torch.randn(M, N, generator=torch.Generator(device="cuda").manual_seed(seed + M), device="cuda").bfloat16()
+
+
+# rows: less than a tile, tiles minus / plus 16 rows, an odd number of tiles (a pair with an empty half); columns: one group, a tile
+# plus one group, ragged tiles; tokens: 17, accumulators minus / plus one, a ragged last tile
+@pytest.mark.parametrize("K,N,bits", [(16, 128, 4), (100, 640, 3), (144, 512, 2), (384, 1152, 4), (1000, 4096, 3), (4096, 2048, 4)])
+@pytest.mark.parametrize("M", [17, 32, 255, 257, 513, 1500])
+def test_forms_match_fp64(K, N, bits, M):
+    m, x = module(K, N, bits, bias=K == 384), tokens(M, N)
+    check(m, x, m(x))
+    assert torch.equal(m(x), m(x))                                # split sums are added in a fixed order
+
+
+@pytest.mark.parametrize("M", [3, 16, 40, 300, 1100])
+@pytest.mark.parametrize("bits", [2, 3, 4])
+def test_column_scale(M, bits):
+    s2 = torch.exp(torch.randn(1152, generator=torch.Generator(device="cuda").manual_seed(5), device="cuda") * 0.25).half()
+    m, x = module(272, 1152, bits, scale2=s2, bias=True), tokens(M, 1152)
+    check(m, x, m(x))
+
+
+@pytest.mark.parametrize("M", [2, 40, 600])
+@pytest.mark.parametrize("scaled", [False, True])
+def test_zero_points_off_the_grid(M, scaled):
+    s2 = (torch.rand(640, generator=torch.Generator(device="cuda").manual_seed(6), device="cuda") + 0.5).half() if scaled else None
+    m, x = module(272, 640, 4, scale2=s2, zero_shift=0.5), tokens(M, 640)
+    check(m, x, m(x))
+
+
+@pytest.mark.parametrize("M", [2, 40, 600])
+def test_infinite_column_scale_leaves_pruned_positions_alone(M):
+    """A column whose scale is infinite only reaches the rows that keep it."""
+    s2 = torch.ones(640, device="cuda").half()
+    s2[37], s2[300] = float("inf"), 0.5
+    m, x = module(64, 640, 3, scale2=s2), tokens(M, 640)
+    _, keep = m.unpack()
+    y = m(x).float()
+    assert bool(torch.isfinite(y[:, ~keep[:, 37]]).all()) and int((~keep[:, 37]).sum()) > 0
+
+
+@pytest.mark.parametrize("M", [17, 90, 400, 1500])
+def test_fused_launch(M):
+    mods = [module(K, 1024, 4, seed=i) for i, K in enumerate((512, 128, 200))]
+    x = tokens(M, 1024)
+    for m, y in zip(mods, FusedProjections(mods)(x)):
+        check(m, x, y)
