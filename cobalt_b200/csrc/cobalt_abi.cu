@@ -148,16 +148,18 @@ int gemv_config(const GemvGeom& g, int N, int M, int num_sms, GemvCfg* c) {
 
 template <int BITS, int MT, bool XS>
 int launch_gemv(const GemvParams& P, const GemvCfg& c, cudaStream_t st) {
-    // two kernels per shape class: the common launch, and the one that also carries the staged-input and push modes
-    const bool special = P.mode != 0;
-    void (*kernel)(const GemvParams) = special ? gemv_mma_special_kernel<BITS, MT, XS> : gemv_mma_kernel<BITS, MT, XS>;
-    static bool configured[MAX_DEVICES][2];
+    // three kernels per shape class: the common launch, the one that also carries the staged-input and push modes, and the
+    // one for a column scale
+    const int kind = P.mode != 0 ? 1 : P.col_scale != nullptr ? 2 : 0;
+    void (*kernel)(const GemvParams) = kind == 1 ? gemv_mma_special_kernel<BITS, MT, XS> : kind == 2 ? gemv_mma_scaled_kernel<BITS, MT, XS>
+                                                                                                    : gemv_mma_kernel<BITS, MT, XS>;
+    static bool configured[MAX_DEVICES][3];
     int dev = 0;
     cudaGetDevice(&dev);
-    if (!configured[dev][special ? 1 : 0]) {
+    if (!configured[dev][kind]) {
         if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_LIMIT) != cudaSuccess)
             return COBALT_ELAUNCH;
-        configured[dev][special ? 1 : 0] = true;
+        configured[dev][kind] = true;
     }
     // programmatic stream serialisation: the prologue of this kernel (barrier set-up, table fill, first weight
     // tiles) may overlap the tail of the previous kernel in the stream; the kernel itself waits before it

@@ -389,17 +389,20 @@ __device__ __noinline__ void gemv_push_publish(const GemvParams& P, uint32_t* s_
 }
 
 // what one unit (16 columns of both rows of a lane) reads from memory; requested one unit ahead
-template <int MT>
+template <int MT, bool SCALED>
 struct GemvUnit {
     uint32_t ra0, ra1, ra2, rb0, rb1, rb2;     // code-stream words at the unit's bit offset, rows A and B
     uint4 ea0, ea1, eb0, eb1;                  // table entries of the unit's mask bytes
     uint4 x[MT][2];                            // activations: 16 columns x token g (+8)
+    uint4 c[SCALED ? 2 : 1];                   // fp16 column scales of the 16 columns
+    uint32_t mA, mB;                           // the mask bytes themselves (column-scaled launches)
 };
 
 // SPECIAL = the launch computes its activations while staging them, adds pushed partial sums, or pushes its own
 // (GemvParams::mode != 0).  The common launch is a kernel of its own without any of that code, so that the
-// less common modes cost it neither a start-up test nor a register.
-template <int BITS, int MT, bool XS, bool SPECIAL>
+// less common modes cost it neither a start-up test nor a register.  SCALED = the matrix has a column scale: its weights
+// are expanded like the others and finished in fp32 (decode8_scaled), a kernel of its own for the same reason.
+template <int BITS, int MT, bool XS, bool SPECIAL, bool SCALED>
 __device__ __forceinline__ void gemv_mma_body(const GemvParams& P) {
     extern __shared__ __align__(1024) uint8_t smem[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -725,8 +728,9 @@ __device__ __forceinline__ void gemv_mma_body(const GemvParams& P) {
             staged = true;
             if (!healthy) continue;
         }
-        const SegParams pA = make_seg_params(szA, BITS, P.col_scale != nullptr);
-        const SegParams pB = make_seg_params(szB, BITS, P.col_scale != nullptr);
+        const bool literal_scale = SPECIAL && P.col_scale != nullptr;  // the special launch has no scaled expansion
+        const SegParams pA = make_seg_params(szA, BITS, literal_scale);
+        const SegParams pB = make_seg_params(szB, BITS, literal_scale);
         const bool all_fast = __all_sync(full, pA.fast && pB.fast);
         const int col0 = active ? (ct * TILE_GROUPS + t) * GROUP : 0;  // first column of this lane's group; lanes beyond a
                                                                        // partial tile read column 0, their zero weights cancel it
@@ -743,7 +747,7 @@ __device__ __forceinline__ void gemv_mma_body(const GemvParams& P) {
         if (all_fast) {
             // ---- request everything unit `u` (16 columns: half h of mask word j) needs
             auto load_unit = [&](uint32_t m16A, uint32_t m16B, uint32_t bA, uint32_t bB, int j, int h) {
-                GemvUnit<MT> Un;
+                GemvUnit<MT, SCALED> Un;
                 const uint32_t pa = cw + ((bA >> 5) << 2), pb = cw + ((bB >> 5) << 2);
                 Un.ra0 = lds32(pa); Un.ra1 = lds32(pa + 4); Un.ra2 = BITS == 2 ? 0u : lds32(pa + 8);
                 Un.rb0 = lds32(pb); Un.rb1 = lds32(pb + 4); Un.rb2 = BITS == 2 ? 0u : lds32(pb + 8);
@@ -764,19 +768,39 @@ __device__ __forceinline__ void gemv_mma_body(const GemvParams& P) {
                         Un.x[b][1] = __ldg(xp + MT * 32);
                     }
                 }
+                if (SCALED) {
+                    const uint4* cp = reinterpret_cast<const uint4*>(P.col_scale + col0 + 32 * (j & 3) + 16 * h);
+                    Un.c[0] = __ldg(cp);
+                    Un.c[SCALED ? 1 : 0] = __ldg(cp + 1);
+                    Un.mA = m16A; Un.mB = m16B;
+                }
                 return Un;
             };
             // ---- expand one unit and feed the tensor cores
-            auto compute_unit = [&](const GemvUnit<MT>& Un, uint32_t bA, uint32_t bB) {
+            auto compute_unit = [&](const GemvUnit<MT, SCALED>& Un, uint32_t bA, uint32_t bB) {
                 uint32_t oa[8], ob[8];
+                float cs[SCALED ? 16 : 1];
+                if (SCALED) {
+                    const uint32_t cw[8] = {Un.c[0].x, Un.c[0].y, Un.c[0].z, Un.c[0].w, Un.c[SCALED ? 1 : 0].x, Un.c[SCALED ? 1 : 0].y,
+                                            Un.c[SCALED ? 1 : 0].z, Un.c[SCALED ? 1 : 0].w};
+#pragma unroll
+                    for (int k = 0; k < 8; ++k) { cs[SCALED ? 2 * k : 0] = half_bits_to_float(cw[k]); cs[SCALED ? 2 * k + 1 : 0] = half_bits_to_float(cw[k] >> 16); }
+                }
+                auto expand = [&](uint32_t w0, const uint4& e, const SegParams& sp, uint32_t mb, int first, uint32_t* o) {
+                    uint32_t t4[4];
+                    if (SCALED) decode8_scaled<BITS>(mb, w0, e.x, e.y, e.z, sp, cs + (SCALED ? first : 0), t4);
+                    else decode8<BITS>(w0, e.x, e.y, e.z, sp, t4);
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) o[k] = t4[k];
+                };
                 const uint32_t a0 = funnel_r(Un.ra0, Un.ra1, bA);
                 const uint32_t a1 = BITS == 2 ? a0 >> Un.ea0.w : funnel_rc(a0, funnel_r(Un.ra1, Un.ra2, bA), Un.ea0.w);
-                decode8<BITS>(a0, Un.ea0.x, Un.ea0.y, Un.ea0.z, pA, oa);
-                decode8<BITS>(a1, Un.ea1.x, Un.ea1.y, Un.ea1.z, pA, oa + 4);
+                expand(a0, Un.ea0, pA, Un.mA & 0xFFu, 0, oa);
+                expand(a1, Un.ea1, pA, Un.mA >> 8, 8, oa + 4);
                 const uint32_t b0 = funnel_r(Un.rb0, Un.rb1, bB);
                 const uint32_t b1 = BITS == 2 ? b0 >> Un.eb0.w : funnel_rc(b0, funnel_r(Un.rb1, Un.rb2, bB), Un.eb0.w);
-                decode8<BITS>(b0, Un.eb0.x, Un.eb0.y, Un.eb0.z, pB, ob);
-                decode8<BITS>(b1, Un.eb1.x, Un.eb1.y, Un.eb1.z, pB, ob + 4);
+                expand(b0, Un.eb0, pB, Un.mB & 0xFFu, 0, ob);
+                expand(b1, Un.eb1, pB, Un.mB >> 8, 8, ob + 4);
 #pragma unroll
                 for (int b = 0; b < MT; ++b) {
                     mma_bf16_16816(acc[b], oa[0], ob[0], oa[1], ob[1], Un.x[b][0].x, Un.x[b][0].y);
@@ -787,9 +811,9 @@ __device__ __forceinline__ void gemv_mma_body(const GemvParams& P) {
             };
 
             // one word (two units) of both rows; `cur` arrives requested, the first unit of the next word leaves requested
-            auto do_word = [&](GemvUnit<MT>& cur, uint32_t mAj, uint32_t mBj, uint32_t mAn, uint32_t mBn, int j) {
+            auto do_word = [&](GemvUnit<MT, SCALED>& cur, uint32_t mAj, uint32_t mBj, uint32_t mAn, uint32_t mBn, int j) {
                 const uint32_t bitA1 = bitA + BITS * __popc(mAj & 0xFFFFu), bitB1 = bitB + BITS * __popc(mBj & 0xFFFFu);
-                const GemvUnit<MT> nxt = load_unit(mAj >> 16, mBj >> 16, bitA1, bitB1, j, 1);
+                const GemvUnit<MT, SCALED> nxt = load_unit(mAj >> 16, mBj >> 16, bitA1, bitB1, j, 1);
                 compute_unit(cur, bitA, bitB);
                 const uint32_t bitA2 = bitA + BITS * __popc(mAj), bitB2 = bitB + BITS * __popc(mBj);
                 // after the last word this requests a unit that is never expanded (harmless in-bounds reads)
@@ -797,7 +821,7 @@ __device__ __forceinline__ void gemv_mma_body(const GemvParams& P) {
                 compute_unit(nxt, bitA1, bitB1);
                 bitA = bitA2; bitB = bitB2;
             };
-            GemvUnit<MT> cur = load_unit(mA.x & 0xFFFFu, mB.x & 0xFFFFu, bitA, bitB, ja, 0);
+            GemvUnit<MT, SCALED> cur = load_unit(mA.x & 0xFFFFu, mB.x & 0xFFFFu, bitA, bitB, ja, 0);
             if (ja == 0 && jb == TILE_WORDS) {                         // whole tile: straight-line code, no register rotation
                 do_word(cur, mA.x, mB.x, mA.y, mB.y, 0);
                 do_word(cur, mA.y, mB.y, mA.z, mB.z, 1);
@@ -813,7 +837,7 @@ __device__ __forceinline__ void gemv_mma_body(const GemvParams& P) {
                 }
             }
         } else {
-            // ---- literal fp32 path (off-grid zero points, column scale): one 32-column word at a time
+            // ---- literal fp32 path (off-grid zero points, scales that are not finite): one 32-column word at a time
             auto word_at = [&](uint32_t k) { return lds32(cw + 4u * k); };
 #pragma unroll 1
             for (int j = ja; j < jb; ++j) {
@@ -823,7 +847,7 @@ __device__ __forceinline__ void gemv_mma_body(const GemvParams& P) {
                 uint32_t ea[16], eb[16];
                 float cs[32];
                 const float* csp = nullptr;
-                if (P.col_scale != nullptr) {
+                if ((SPECIAL || SCALED) && P.col_scale != nullptr) {
 #pragma unroll
                     for (int q = 0; q < 32; ++q) cs[q] = half_bits_to_float(P.col_scale[col0 + 32 * j + q]);
                     csp = cs;
@@ -882,12 +906,17 @@ __device__ __forceinline__ void gemv_mma_body(const GemvParams& P) {
 
 template <int BITS, int MT, bool XS>
 __global__ void __launch_bounds__(GEMV_THREADS, 1) gemv_mma_kernel(const GemvParams P) {
-    gemv_mma_body<BITS, MT, XS, false>(P);
+    gemv_mma_body<BITS, MT, XS, false, false>(P);
+}
+// one matrix with a column scale: 4096 x 4096, 4 bit, 5 tokens 14 us; one position at a time (the literal path) it took 68 us
+template <int BITS, int MT, bool XS>
+__global__ void __launch_bounds__(GEMV_THREADS, 1) gemv_mma_scaled_kernel(const GemvParams P) {
+    gemv_mma_body<BITS, MT, XS, false, true>(P);
 }
 // parameters in place (their address is handed to the out-of-line staging and push functions)
 template <int BITS, int MT, bool XS>
 __global__ void __launch_bounds__(GEMV_THREADS, 1) gemv_mma_special_kernel(const __grid_constant__ GemvParams P) {
-    gemv_mma_body<BITS, MT, XS, true>(P);
+    gemv_mma_body<BITS, MT, XS, true, false>(P);
 }
 
 }  // namespace cb
