@@ -348,6 +348,7 @@ int launch_prompt_attn(const PromptAttnParams& P, unsigned ctas, const CUtensorM
     return cudaGetLastError() == cudaSuccess ? COBALT_OK : COBALT_ELAUNCH;
 }
 
+constexpr int ROPE_MIN_ROWS = 32;
 constexpr long STAGED_NORM_MAX_VALUES = 8192, STAGED_GLU_MAX_VALUES = 32768;     // M * in_features a staged input may compute
 constexpr size_t SCRATCH_PUSH_DONE_OFF = 128;            // CTA arrival counter of pushing launches, inside the status block
 
@@ -848,10 +849,11 @@ int cobalt_add_rmsnorm(const void* h, const void* delta, const void* w, void* h_
     if (rc) return rc;
     const bool vec = H % 256 == 0 && H <= 256 * ADDNORM_MAX_ITERS * (ADDNORM_THREADS / 32) && !(((uintptr_t)h | (uintptr_t)delta | (uintptr_t)w |
                      (uintptr_t)h_out | (uintptr_t)y | (uintptr_t)w_branch) & 15);
-    if (vec)
-        add_rmsnorm_kernel<<<T, ADDNORM_THREADS, 0, (cudaStream_t)stream>>>((const uint16_t*)h, (const uint16_t*)delta, (const uint16_t*)w,
-                                                                           (uint16_t*)h_out, (uint16_t*)y, H, eps, flavor, (const uint16_t*)w_branch);
-    else
+    if (vec) {
+        auto kernel = H <= 8 * ADDNORM_THREADS ? add_rmsnorm_kernel<1> : H <= 16 * ADDNORM_THREADS ? add_rmsnorm_kernel<2> : add_rmsnorm_kernel<ADDNORM_MAX_ITERS>;
+        kernel<<<T, ADDNORM_THREADS, 0, (cudaStream_t)stream>>>((const uint16_t*)h, (const uint16_t*)delta, (const uint16_t*)w,
+                                                               (uint16_t*)h_out, (uint16_t*)y, H, eps, flavor, (const uint16_t*)w_branch);
+    } else
         add_rmsnorm_generic_kernel<<<T, 256, 0, (cudaStream_t)stream>>>((const uint16_t*)h, (const uint16_t*)delta, (const uint16_t*)w,
                                                                        (uint16_t*)h_out, (uint16_t*)y, H, eps, flavor, (const uint16_t*)w_branch);
     return cudaGetLastError() == cudaSuccess ? COBALT_OK : COBALT_ELAUNCH;
@@ -866,6 +868,19 @@ int cobalt_rope_kv(void* q, const void* k, const void* v, const int64_t* positio
     int sms = 0;
     int rc = device_info(&sms);
     if (rc) return rc;
+    // a block per token once that fills a good part of the GPU; fewer tokens (a decode step) spread every head instead
+    const bool rows = T >= ROPE_MIN_ROWS && head_dim % 16 == 0 && head_dim <= 2 * ROPE_MAX_HALF && cache_seq_stride % 8 == 0 &&
+                      !(((uintptr_t)q | (uintptr_t)k | (uintptr_t)v | (uintptr_t)k_cache | (uintptr_t)v_cache) & 15);
+    if (rows) {
+        if (q_norm_w)
+            rope_kv_norm_rows_kernel<<<T, 256, 0, (cudaStream_t)stream>>>((uint16_t*)q, (const uint16_t*)k, (const uint16_t*)v, (const long long*)positions,
+                inv_freq, (uint16_t*)k_cache, (uint16_t*)v_cache, n_heads, n_kv_heads, head_dim, max_ctx, (const uint16_t*)q_norm_w,
+                (const uint16_t*)k_norm_w, eps, (long long)cache_seq_stride);
+        else
+            rope_kv_rows_kernel<<<T, 256, 0, (cudaStream_t)stream>>>((uint16_t*)q, (const uint16_t*)k, (const uint16_t*)v, (const long long*)positions,
+                inv_freq, (uint16_t*)k_cache, (uint16_t*)v_cache, n_heads, n_kv_heads, head_dim, max_ctx, (long long)cache_seq_stride);
+        return cudaGetLastError() == cudaSuccess ? COBALT_OK : COBALT_ELAUNCH;
+    }
     if (q_norm_w) {
         const long long warps = (long long)T * (n_heads + 2 * n_kv_heads);
         rope_kv_norm_kernel<<<(unsigned)((warps * 32 + 255) / 256), 256, 0, (cudaStream_t)stream>>>(
@@ -1035,8 +1050,23 @@ int cobalt_swiglu(const void* gate, const void* up, void* out, int64_t n, int ac
     int sms = 0;
     int rc = device_info(&sms);
     if (rc) return rc;
+    if (n % 8 == 0 && !(((uintptr_t)gate | (uintptr_t)up | (uintptr_t)out) & 15)) {
+        swiglu_chunks_kernel<<<(unsigned)((n / 8 + 255) / 256), 256, 0, (cudaStream_t)stream>>>((const uint4*)gate, (const uint4*)up, (uint4*)out,
+                                                                                               (long long)(n / 8), act);
+        return cudaGetLastError() == cudaSuccess ? COBALT_OK : COBALT_ELAUNCH;
+    }
     swiglu_kernel<<<(unsigned)((n + 255) / 256), 256, 0, (cudaStream_t)stream>>>((const uint16_t*)gate, (const uint16_t*)up,
                                                                                  (uint16_t*)out, (long long)n, act);
+    return cudaGetLastError() == cudaSuccess ? COBALT_OK : COBALT_ELAUNCH;
+}
+
+int cobalt_argmax(const void* logits, int64_t ld, int rows, int64_t V, int64_t* out, void* stream) {
+    if (!logits || !out || rows <= 0 || rows > 65535 || V <= 0 || V > 0xFFFFFFFFll || ld < V || ((uintptr_t)logits & 1)) return COBALT_EINVAL;
+    int sms = 0;
+    int rc = device_info(&sms);
+    if (rc) return rc;
+    argmax_kernel<<<dim3(ARGMAX_CTAS, (unsigned)rows), ARGMAX_THREADS, 0, (cudaStream_t)stream>>>((const uint16_t*)logits, (long long)ld,
+                                                                                                 (long long)V, (long long*)out);
     return cudaGetLastError() == cudaSuccess ? COBALT_OK : COBALT_ELAUNCH;
 }
 

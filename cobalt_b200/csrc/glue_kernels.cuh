@@ -73,18 +73,21 @@ __global__ void __launch_bounds__(256) add_rmsnorm_generic_kernel(const uint16_t
 // the order staged_input.cuh defines, which the decode GEMV reproduces when it applies this step while staging.
 constexpr int ADDNORM_THREADS = 512;
 constexpr int ADDNORM_MAX_ITERS = 4;                                   // chunks per thread: rows up to 16384 values
-__global__ void __launch_bounds__(ADDNORM_THREADS) add_rmsnorm_kernel(const uint16_t* h, const uint16_t* delta, const uint16_t* w,
+// ITERS = chunks a thread holds.  Sized for the longest row the registers left one block per SM, and a prompt's rows went
+// through 14 rounds of load - sum - barrier latency: 2048 rows of 4096 values 44 -> 28 us.
+template <int ITERS>
+__global__ void __launch_bounds__(ADDNORM_THREADS, ITERS == 1 ? 4 : ITERS == 2 ? 2 : 1) add_rmsnorm_kernel(const uint16_t* h, const uint16_t* delta, const uint16_t* w,
                                                                       uint16_t* h_out, uint16_t* y, int H, float eps, int flavor,
                                                                       const uint16_t* w_branch) {
-    __shared__ float tot_branch[ADDNORM_MAX_ITERS * ADDNORM_THREADS / 32], tot_joined[ADDNORM_MAX_ITERS * ADDNORM_THREADS / 32];
+    __shared__ float tot_branch[ITERS * ADDNORM_THREADS / 32], tot_joined[ITERS * ADDNORM_THREADS / 32];
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const size_t base = (size_t)blockIdx.x * H;
     const int cpr = H / 8, groups = cpr / 32;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const bool norm_branch = delta != nullptr && w_branch != nullptr;
-    float v[ADDNORM_MAX_ITERS][8], d[ADDNORM_MAX_ITERS][8];
+    float v[ITERS][8], d[ITERS][8];
 #pragma unroll
-    for (int q = 0; q < ADDNORM_MAX_ITERS; ++q) {
+    for (int q = 0; q < ITERS; ++q) {
         const int c = threadIdx.x + q * ADDNORM_THREADS;
         if (c < cpr) {
             chunk_to_floats(__ldg(reinterpret_cast<const uint4*>(h + base) + c), v[q]);
@@ -93,7 +96,7 @@ __global__ void __launch_bounds__(ADDNORM_THREADS) add_rmsnorm_kernel(const uint
     }
     if (norm_branch) {
 #pragma unroll
-        for (int q = 0; q < ADDNORM_MAX_ITERS; ++q) {
+        for (int q = 0; q < ITERS; ++q) {
             const int c = threadIdx.x + q * ADDNORM_THREADS;
             const float s = warp_butterfly_sum(c < cpr ? chunk_sumsq(d[q]) : 0.0f);
             if (lane == 0 && c < cpr) tot_branch[q * (ADDNORM_THREADS / 32) + warp] = s;
@@ -101,7 +104,7 @@ __global__ void __launch_bounds__(ADDNORM_THREADS) add_rmsnorm_kernel(const uint
         __syncthreads();
         const float rb = row_rsqrt(tot_branch, groups, H, eps);
 #pragma unroll
-        for (int q = 0; q < ADDNORM_MAX_ITERS; ++q) {
+        for (int q = 0; q < ITERS; ++q) {
             const int c = threadIdx.x + q * ADDNORM_THREADS;
             if (c < cpr) {
                 float wb[8];
@@ -112,7 +115,7 @@ __global__ void __launch_bounds__(ADDNORM_THREADS) add_rmsnorm_kernel(const uint
         }
     }
 #pragma unroll
-    for (int q = 0; q < ADDNORM_MAX_ITERS; ++q) {
+    for (int q = 0; q < ITERS; ++q) {
         const int c = threadIdx.x + q * ADDNORM_THREADS;
         if (c < cpr && delta) {
 #pragma unroll
@@ -125,7 +128,7 @@ __global__ void __launch_bounds__(ADDNORM_THREADS) add_rmsnorm_kernel(const uint
     __syncthreads();
     const float r = row_rsqrt(tot_joined, groups, H, eps);
 #pragma unroll
-    for (int q = 0; q < ADDNORM_MAX_ITERS; ++q) {
+    for (int q = 0; q < ITERS; ++q) {
         const int c = threadIdx.x + q * ADDNORM_THREADS;
         if (c < cpr) {
             float wn[8], o[8];
@@ -218,12 +221,167 @@ __global__ void __launch_bounds__(256) rope_kv_norm_kernel(uint16_t* q, const ui
     }
 }
 
+// The two kernels above for the tokens of a prompt (D a multiple of 16, at most 256; everything 16-byte aligned): one block per
+// token computes the D/2 cosines and sines once - they are the same for every head - and moves 16 bytes at a time.  Per
+// thread and value, as above, the sine and cosine were the cost: 2048 tokens, 48 heads of 128: 63 -> 24 us.
+constexpr int ROPE_MAX_HALF = 128;
+__device__ __forceinline__ void rope_table(const float* inv_freq, long long pos, int half, float* cs, float* sn) {
+    for (int d = threadIdx.x; d < half; d += blockDim.x) {
+        const float ang = (float)pos * inv_freq[d];
+        cs[d] = bf16_round(cosf(ang));
+        sn[d] = bf16_round(sinf(ang));
+    }
+    __syncthreads();
+}
+__global__ void __launch_bounds__(256) rope_kv_rows_kernel(uint16_t* q, const uint16_t* k, const uint16_t* v, const long long* positions,
+                                                           const float* inv_freq, uint16_t* k_cache, uint16_t* v_cache, int nh, int nkv,
+                                                           int D, int max_ctx, long long seq_stride) {
+    __shared__ float cs[ROPE_MAX_HALF], sn[ROPE_MAX_HALF];
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    const int t = blockIdx.x, half = D / 2, hc = half / 8;              // 16-byte chunks of half a head
+    const long long pos = positions[t];
+    const bool stored = pos >= 0 && pos < max_ctx;                      // a position outside the cache is never stored
+    rope_table(inv_freq, pos, half, cs, sn);
+    const int turns = (nh + nkv) * hc, items = turns + nkv * 2 * hc;
+    for (int i = threadIdx.x; i < items; i += blockDim.x) {
+        if (i >= turns) {                                               // v: plain copy
+            const int c = i - turns, hv = c / (2 * hc), d = (c - hv * 2 * hc) * 8;
+            if (stored)
+                *reinterpret_cast<uint4*>(v_cache + (size_t)t * seq_stride + ((size_t)hv * max_ctx + (size_t)pos) * D + d) =
+                    __ldg(reinterpret_cast<const uint4*>(v + ((size_t)t * nkv + hv) * D + d));
+            continue;
+        }
+        const int head = i / hc, d = (i - head * hc) * 8;
+        const bool is_q = head < nh;
+        if (!is_q && !stored) continue;
+        const uint16_t* src = is_q ? q + ((size_t)t * nh + head) * D : k + ((size_t)t * nkv + (head - nh)) * D;
+        uint16_t* dst = is_q ? q + ((size_t)t * nh + head) * D
+                             : k_cache + (size_t)t * seq_stride + ((size_t)(head - nh) * max_ctx + (size_t)pos) * D;
+        float x1[8], x2[8], o1[8], o2[8];
+        chunk_to_floats(*reinterpret_cast<const uint4*>(src + d), x1);
+        chunk_to_floats(*reinterpret_cast<const uint4*>(src + half + d), x2);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+            const float c = cs[d + e], s = sn[d + e];
+            o1[e] = bf16_round(x1[e] * c) + bf16_round(-x2[e] * s);
+            o2[e] = bf16_round(x2[e] * c) + bf16_round(x1[e] * s);
+        }
+        *reinterpret_cast<uint4*>(dst + d) = floats_to_chunk(o1);
+        *reinterpret_cast<uint4*>(dst + half + d) = floats_to_chunk(o2);
+    }
+}
+// with the per-head norm: one warp per head at a time, sums in the order of rope_kv_norm_kernel
+__global__ void __launch_bounds__(256) rope_kv_norm_rows_kernel(uint16_t* q, const uint16_t* k, const uint16_t* v, const long long* positions,
+                                                                const float* inv_freq, uint16_t* k_cache, uint16_t* v_cache, int nh,
+                                                                int nkv, int D, int max_ctx, const uint16_t* q_norm_w,
+                                                                const uint16_t* k_norm_w, float eps, long long seq_stride) {
+    __shared__ float cs[ROPE_MAX_HALF], sn[ROPE_MAX_HALF];
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    const int t = blockIdx.x, half = D / 2, lane = threadIdx.x & 31;
+    const long long pos = positions[t];
+    const bool stored = pos >= 0 && pos < max_ctx;
+    rope_table(inv_freq, pos, half, cs, sn);
+    for (int head = threadIdx.x >> 5; head < nh + 2 * nkv; head += blockDim.x >> 5) {
+        const bool is_q = head < nh;
+        if (!is_q && !stored) continue;
+        if (head >= nh + nkv) {
+            const int hv = head - nh - nkv;
+            const uint4* src = reinterpret_cast<const uint4*>(v + ((size_t)t * nkv + hv) * D);
+            uint4* dst = reinterpret_cast<uint4*>(v_cache + (size_t)t * seq_stride + ((size_t)hv * max_ctx + (size_t)pos) * D);
+            for (int c = lane; c < D / 8; c += 32) dst[c] = __ldg(src + c);
+            continue;
+        }
+        const uint16_t* src = is_q ? q + ((size_t)t * nh + head) * D : k + ((size_t)t * nkv + (head - nh)) * D;
+        const uint16_t* nw = is_q ? q_norm_w : k_norm_w;
+        uint16_t* dst = is_q ? q + ((size_t)t * nh + head) * D : k_cache + (size_t)t * seq_stride + ((size_t)(head - nh) * max_ctx + (size_t)pos) * D;
+        float x[2 * ROPE_MAX_HALF / 32], ss = 0.0f;
+#pragma unroll
+        for (int i = 0; i < 2 * ROPE_MAX_HALF / 32; ++i) {
+            x[i] = lane + 32 * i < D ? bf16_to_float(src[lane + 32 * i]) : 0.0f;
+            if (lane + 32 * i < D) ss += x[i] * x[i];
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xFFFFFFFFu, ss, o);
+        const float r = rsqrtf(ss / (float)D + eps);
+        for (int d = lane; d < half; d += 32) {
+            const float x1 = bf16_round(__fmul_rn(__fmul_rn(bf16_to_float(src[d]), r), __fadd_rn(1.0f, bf16_to_float(nw[d]))));
+            const float x2 = bf16_round(__fmul_rn(__fmul_rn(bf16_to_float(src[d + half]), r), __fadd_rn(1.0f, bf16_to_float(nw[d + half]))));
+            const float c = cs[d], s = sn[d];
+            dst[d] = float_to_bf16(bf16_round(x1 * c) + bf16_round(-x2 * s));
+            dst[d + half] = float_to_bf16(bf16_round(x2 * c) + bf16_round(x1 * s));
+        }
+    }
+}
+
 // out = bf16( bf16(act(g)) * u ); act 0 = SiLU, act 1 = GELU with the tanh approximation
 __global__ void swiglu_kernel(const uint16_t* g, const uint16_t* u, uint16_t* out, long long n, int act) {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     out[i] = float_to_bf16(glu_value(bf16_to_float(g[i]), bf16_to_float(u[i]), act));
+}
+
+// the same over 16-byte chunks (n a multiple of 8, everything 16-byte aligned): value by value the loads and stores were the cost,
+// 2048 x 14336 values 120 -> 67 us (exponential, division and rounding are left)
+__global__ void __launch_bounds__(256) swiglu_chunks_kernel(const uint4* __restrict__ g, const uint4* __restrict__ u, uint4* __restrict__ out,
+                                                            long long chunks, int act) {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < chunks) out[i] = glu_chunk(__ldg(g + i), __ldg(u + i), act);
+}
+
+// ----------------------------------------------------------------------------- greedy token
+// out[row] = index of the largest of V bf16 logits: the first of equal ones, a NaN above everything (torch.argmax).  One cluster
+// of ARGMAX_CTAS blocks per row, joined through distributed shared memory: one 16-byte load per thread at 32000
+// logits, where the reduction over fp32 copies took two kernels and 14 us.
+constexpr int ARGMAX_CTAS = 8, ARGMAX_THREADS = 512;
+__device__ __forceinline__ unsigned long long argmax_key(uint32_t b, long long index) {      // larger value first, then smaller index
+    if ((b & 0x7FFFu) == 0) b = 0;                                      // -0 equals +0
+    const uint32_t order = (b & 0x7FFFu) > 0x7F80u ? 0xFFFFu : (b & 0x8000u) ? (~b & 0xFFFFu) : (b | 0x8000u);
+    return ((unsigned long long)order << 32) | (0xFFFFFFFFu - (uint32_t)index);
+}
+__global__ void __cluster_dims__(ARGMAX_CTAS, 1, 1) __launch_bounds__(ARGMAX_THREADS) argmax_kernel(const uint16_t* logits, long long ld,
+                                                                                                    long long V, long long* out) {
+    __shared__ unsigned long long best_s[ARGMAX_THREADS / 32];
+    __shared__ unsigned long long cta_best;
+    const uint16_t* row = logits + (size_t)blockIdx.y * ld;
+    unsigned long long best = 0;
+    auto take = [&](uint32_t b, long long i) { const unsigned long long k = argmax_key(b, i); best = k > best ? k : best; };
+    const long long first = (long long)blockIdx.x * ARGMAX_THREADS + threadIdx.x, step = (long long)ARGMAX_CTAS * ARGMAX_THREADS;
+    long long done = 0;
+    if (((uintptr_t)row & 15) == 0) {
+        done = V / 8 * 8;
+        for (long long c = first; c < V / 8; c += step) {
+            const uint4 v = __ldg(reinterpret_cast<const uint4*>(row) + c);
+            const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+            for (int e = 0; e < 4; ++e) { take(w[e] & 0xFFFFu, 8 * c + 2 * e); take(w[e] >> 16, 8 * c + 2 * e + 1); }
+        }
+    }
+    for (long long i = done + first; i < V; i += step) take(row[i], i);
+    auto larger = [](unsigned long long a, unsigned long long b) { return a > b ? a : b; };
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) best = larger(best, __shfl_xor_sync(0xFFFFFFFFu, best, o));
+    if ((threadIdx.x & 31) == 0) best_s[threadIdx.x >> 5] = best;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < ARGMAX_THREADS / 32; ++w) best = larger(best, best_s[w]);
+        cta_best = best;
+    }
+    __syncwarp();
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        for (uint32_t c = 1; c < ARGMAX_CTAS; ++c) {
+            uint32_t a;
+            unsigned long long other;
+            asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_u32(&cta_best)), "r"(c));
+            asm volatile("ld.shared::cluster.u64 %0, [%1];" : "=l"(other) : "r"(a) : "memory");
+            best = larger(best, other);
+        }
+        out[blockIdx.y] = (long long)(0xFFFFFFFFu - (uint32_t)best);
+    }
+    __syncwarp();
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
 // ----------------------------------------------------------------------------- single-token attention

@@ -460,14 +460,15 @@ class CobaltDecoder:
     def step(self) -> torch.Tensor:
         """One decode step for the tokens in ``self.tok`` at ``self.pos`` (one per sequence); returns the logits
         (``[V]`` for a single sequence, else ``[B, V]``) and advances ``tok`` (greedy) and ``pos`` on the device."""
-        if self.B == 1:
-            logits = self._forward(self.tok, self.pos, self.max_ctx, seq=0)[0, 0]
-            self.tok.copy_(torch.argmax(logits.float(), dim=-1, keepdim=True))
+        rows = self._forward(self.tok, self.pos, self.max_ctx, seq=0 if self.B == 1 else None)[0]        # [B, V]
+        if rows.dtype == torch.bfloat16 and rows.stride(-1) == 1:
+            rc = self._lib.cobalt_argmax(rows.data_ptr(), rows.stride(0), self.B, rows.shape[-1], self.tok.data_ptr(),
+                                         torch.cuda.current_stream(self.dev).cuda_stream)
+            _lib.check("cobalt_argmax", rc)
         else:
-            logits = self._forward(self.tok, self.pos, self.max_ctx, seq=None)[0]
-            self.tok.copy_(torch.argmax(logits.float(), dim=-1))
+            self.tok.copy_(torch.argmax(rows.float(), dim=-1))
         self.pos.add_(1)
-        return logits
+        return rows[0] if self.B == 1 else rows
 
     @torch.no_grad()
     def generate(self, prompt: torch.Tensor, n_new: int, use_graph: bool = True, teacher: Optional[torch.Tensor] = None):
@@ -505,7 +506,7 @@ class CobaltDecoder:
                 lg = self._logits
             else:
                 lg = self.step()
-            toks.append(torch.argmax(lg.float(), dim=-1, keepdim=single).clone())
+            toks.append(self.tok.clone())                    # the step's greedy tokens
             all_logits.append(lg.clone())
             if teacher is not None:
                 self.tok.copy_(teacher[i].reshape(-1).to(self.dev))

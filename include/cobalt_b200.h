@@ -320,6 +320,10 @@ size_t cobalt_attn_decode_fused_scratch_bytes(int n_heads, int n_kv_heads, int h
 int cobalt_attn_decode_fused(const void* q, const void* k_cache, const void* v_cache, const int64_t* positions, void* scratch,
                              size_t scratch_bytes, void* out, int n_heads, int n_kv_heads, int head_dim, int max_ctx,
                              int window, float scale, int n_seq, int64_t cache_seq_stride, void* stream);
+/* Greedy token: out[r] = index of the largest of the V bf16 logits of row r (logits + r * ld), the first of equal ones; a NaN counts
+ * as larger than everything. */
+int cobalt_argmax(const void* logits, int64_t ld, int rows, int64_t V, int64_t* out, void* stream);
+
 /* Grouped-query attention of T tokens of one sequence (q and out [T][n_heads*D], q already rotated) over its caches
  * [n_kv_heads][max_ctx][D]: token t attends the slots s < n_slots with s <= positions[t] (and s > positions[t] - window when
  * window > 0).  Same rounding points as cobalt_attn_decode(); scores and probabilities stay on the chip.  D 64 or 128 and at
