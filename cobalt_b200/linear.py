@@ -23,6 +23,13 @@ from .format import GROUP, TileImage, bytes_to_keep, pack_tiles
 
 GEMV_MAX_TOKENS = 16
 FUSED_MAX = 4
+_raw_stream = torch._C._cuda_getCurrentRawStream             # handle of the device's current stream, without a Stream object
+
+
+def _scratch_span(buf: torch.Tensor):
+    """Aligned address and usable bytes of a scratch buffer."""
+    p = (buf.data_ptr() + 255) // 256 * 256
+    return p, buf.numel() - (p - buf.data_ptr())
 
 
 def _ptr(t: Optional[torch.Tensor]) -> Optional[int]:
@@ -58,6 +65,7 @@ class CobaltSparseLinear(nn.Module):
         self._scratch = None
         self._desc = None
         self._desc_key = None
+        self._launch = {}
 
     @classmethod
     def _blank(cls):
@@ -164,40 +172,51 @@ class CobaltSparseLinear(nn.Module):
             raise RuntimeError("CobaltSparseLinear.forward needs a CUDA tensor; there is no CPU path")
         if x.dtype != torch.bfloat16:
             raise TypeError(f"CobaltSparseLinear computes in bfloat16, got {x.dtype}")
-        lib = _lib.load()
-        lead = x.shape[:-1]
-        x2 = x.reshape(-1, self.in_features)
+        N, K = self.in_features, self.out_features
+        flat = x.dim() == 2 and x.shape[1] == N
+        x2 = x if flat else x.reshape(-1, N)
         if x2.stride(-1) != 1 or x2.stride(0) % 8 or x2.data_ptr() % 16:
             x2 = x2.contiguous()
         M = x2.shape[0]
-        want = torch.float32 if out_fp32 else torch.bfloat16
         if out is not None:
-            if out.dtype != want or out.numel() != M * self.out_features or not out.is_contiguous() or out.device != x.device:
+            want = torch.float32 if out_fp32 else torch.bfloat16
+            if out.dtype != want or out.numel() != M * K or not out.is_contiguous() or out.device != x.device:
                 raise ValueError("`out` must be a contiguous [M, out_features] tensor of the result dtype on x's device")
-            y = out.view(M, self.out_features)
+            y = out.view(M, K)
         else:
-            y = torch.empty(M, self.out_features, dtype=want, device=x.device)
-        if M == 0:
-            return y.reshape(*lead, self.out_features)
-        d = self._descriptor()
-        scratch = self._scratch_for(M)
-        sp = self._aligned(scratch)
-        sbytes = scratch.numel() - (sp - scratch.data_ptr())
-        stream = torch.cuda.current_stream(x.device).cuda_stream
-        bias = None if self.bias is None else self.bias.data.to(torch.bfloat16)
-        if out_fp32:
-            rc = lib.cobalt_linear_f32(ctypes.byref(d), x2.data_ptr(), x2.stride(0), y.data_ptr(), y.stride(0), M, sp, sbytes,
-                                       stream)
-            _lib.check("cobalt_linear_f32", rc)
-        elif M <= GEMV_MAX_TOKENS:
-            rc = lib.cobalt_gemv(ctypes.byref(d), x2.data_ptr(), x2.stride(0), y.data_ptr(), y.stride(0), _ptr(bias), M,
-                                 sp, sbytes, stream)
-            _lib.check("cobalt_gemv", rc)
-        else:
-            rc = lib.cobalt_gemm(ctypes.byref(d), x2.data_ptr(), x2.stride(0), y.data_ptr(), y.stride(0), _ptr(bias), M,
-                                 sp, sbytes, stream)
-            _lib.check("cobalt_gemm", rc)
-        return y.reshape(*lead, self.out_features)
+            y = x2.new_empty((M, K), dtype=torch.float32) if out_fp32 else x2.new_empty((M, K))
+        if M:
+            lib = _lib.load()
+            desc, sp, sbytes = self._launch_args(M)
+            stream = _raw_stream(x2.get_device())
+            if out_fp32:
+                rc = lib.cobalt_linear_f32(desc, x2.data_ptr(), x2.stride(0), y.data_ptr(), K, M, sp, sbytes, stream)
+                name = "cobalt_linear_f32"
+            else:
+                bias = self.bias
+                if bias is not None and bias.dtype is not torch.bfloat16:
+                    bias = bias.data.to(torch.bfloat16)
+                name = "cobalt_gemv" if M <= GEMV_MAX_TOKENS else "cobalt_gemm"
+                rc = (lib.cobalt_gemv if M <= GEMV_MAX_TOKENS else lib.cobalt_gemm)(
+                    desc, x2.data_ptr(), x2.stride(0), y.data_ptr(), K, None if bias is None else bias.data_ptr(), M, sp, sbytes, stream)
+            if rc:
+                _lib.check(name, rc)
+        return y if flat else y.reshape(*x.shape[:-1], K)
+
+    def _launch_args(self, M: int):
+        """``(descriptor reference, scratch address, scratch bytes)`` of a call with ``M`` tokens.  Worked out once per kernel
+        (both scratch buffers have a fixed size) and again when the packed image or the column scale is another tensor."""
+        kind = "gemv" if M <= GEMV_MAX_TOKENS else "gemm"
+        bufs = self._buffers
+        scale2 = bufs["scale2"]
+        key = (bufs["packed"].data_ptr(), None if scale2 is None else scale2.data_ptr())
+        args = self._launch.get(kind)
+        if args is None or args[0] != key:
+            desc = self._descriptor()
+            sp, sbytes = _scratch_span(self._scratch_for(M))
+            args = (key, (ctypes.byref(desc), sp, sbytes))
+            self._launch[kind] = args
+        return args[1]
 
     # ------------------------------------------------------------------ inspection
     def dequantize(self) -> torch.Tensor:
@@ -274,6 +293,7 @@ class CobaltSparseLinear(nn.Module):
         out = super()._apply(fn, *a, **k)
         self._desc = None
         self._scratch = None
+        self._launch = {}
         return out
 
     def extra_repr(self) -> str:
@@ -297,23 +317,32 @@ class FusedProjections:
             raise ValueError("fused projections need equal in_features and bit width, no column scale and no bias")
         self.mods = mods
         self._scratch = None
-        self._arrays = None
+        self._key = None
+        self._args = None
+        self._ptrs = ctypes.c_void_p * len(mods)
 
-    def _prepare(self, M, device):
+    def _prepare(self, device):
+        """``(descriptors, row strides, scratch address, scratch bytes)``, worked out again when a module's image is another one."""
+        if self._key is not None and self._scratch.device == device and all(
+                m._img_meta is meta and m._buffers["packed"].data_ptr() == p for m, (meta, p) in zip(self.mods, self._key)):
+            return self._args
         lib = _lib.load()
         n = len(self.mods)
         descs = (ctypes.POINTER(_lib.CobaltMat) * n)(*[ctypes.pointer(m._descriptor()) for m in self.mods])
         # fixed size: the address survives graph capture; one buffer serves the GEMV and the GEMM (status word, counters)
-        need = max(lib.cobalt_gemv_fused_scratch_bytes(n, descs, GEMV_MAX_TOKENS), lib.cobalt_gemm_fused_scratch_bytes(n, descs, max(M, 1)))
+        need = max(lib.cobalt_gemv_fused_scratch_bytes(n, descs, GEMV_MAX_TOKENS), lib.cobalt_gemm_fused_scratch_bytes(n, descs, GEMV_MAX_TOKENS + 1))
         if need == 0:
             raise _lib.CobaltError("cobalt_gemv_fused_scratch_bytes", -1, "could not size the scratch buffer")
         if self._scratch is None or self._scratch.numel() < need + 256 or self._scratch.device != device:
             self._scratch = torch.zeros(need + 256, dtype=torch.uint8, device=device)
-        return descs
+        self._args = (descs, (ctypes.c_int64 * n)(*[m.out_features for m in self.mods]), *_scratch_span(self._scratch))
+        self._key = [(m._img_meta, m._buffers["packed"].data_ptr()) for m in self.mods]      # held, so that neither can be reused
+        return self._args
 
     def __call__(self, x: torch.Tensor):
-        lead = x.shape[:-1]
-        x2 = x.reshape(-1, self.mods[0].in_features)
+        N = self.mods[0].in_features
+        flat = x.dim() == 2 and x.shape[1] == N
+        x2 = x if flat else x.reshape(-1, N)
         M = x2.shape[0]
         if M == 0:
             return [m(x) for m in self.mods]
@@ -324,18 +353,14 @@ class FusedProjections:
         if x2.stride(-1) != 1 or x2.stride(0) % 8 or x2.data_ptr() % 16:
             x2 = x2.contiguous()
         lib = _lib.load()
-        n = len(self.mods)
-        descs = self._prepare(M, x.device)
-        ys = [torch.empty(M, m.out_features, dtype=torch.bfloat16, device=x.device) for m in self.mods]
-        yp = (ctypes.c_void_p * n)(*[y.data_ptr() for y in ys])
-        ld = (ctypes.c_int64 * n)(*[y.stride(0) for y in ys])
-        sp = (self._scratch.data_ptr() + 255) // 256 * 256
-        name = "cobalt_gemv_fused" if M <= GEMV_MAX_TOKENS else "cobalt_gemm_fused"
-        rc = getattr(lib, name)(n, descs, x2.data_ptr(), x2.stride(0), yp, ld, None, M, sp,
-                                self._scratch.numel() - (sp - self._scratch.data_ptr()),
-                                torch.cuda.current_stream(x.device).cuda_stream)
-        _lib.check(name, rc)
-        return [y.reshape(*lead, m.out_features) for y, m in zip(ys, self.mods)]
+        descs, ld, sp, sbytes = self._prepare(x2.device)
+        ys = [x2.new_empty((M, m.out_features)) for m in self.mods]
+        rc = (lib.cobalt_gemv_fused if M <= GEMV_MAX_TOKENS else lib.cobalt_gemm_fused)(
+            len(ys), descs, x2.data_ptr(), x2.stride(0), self._ptrs(*[y.data_ptr() for y in ys]), ld, None, M, sp, sbytes,
+            _raw_stream(x2.get_device()))
+        if rc:
+            _lib.check("cobalt_gemv_fused" if M <= GEMV_MAX_TOKENS else "cobalt_gemm_fused", rc)
+        return ys if flat else [y.reshape(*x.shape[:-1], m.out_features) for y, m in zip(ys, self.mods)]
 
     def staged(self, kind: int, a: torch.Tensor, b: Optional[torch.Tensor], flavor: int, w: Optional[torch.Tensor] = None,
                w_branch: Optional[torch.Tensor] = None, h_out: Optional[torch.Tensor] = None, eps: float = 0.0,
@@ -355,11 +380,10 @@ class FusedProjections:
                 raise ValueError("a, b and h_out must have the same shape and strides")
         lib = _lib.load()
         n = len(self.mods)
-        descs = self._prepare(M, a.device)
+        descs, _, sp, sbytes = self._prepare(a.device)
         ptr = lambda t: None if t is None else t.data_ptr()
         inp = _lib.CobaltStagedInput(kind, flavor, a.data_ptr(), ptr(b), a.stride(0), ptr(w), ptr(w_branch), ptr(h_out), eps,
                                      None if delta_slots is None else ctypes.pointer(delta_slots.slots))
-        sp = (self._scratch.data_ptr() + 255) // 256 * 256
         if push is not None:
             ys, yp, ld, out_fp32 = [], None, None, True
         else:
@@ -369,7 +393,7 @@ class FusedProjections:
             ld = (ctypes.c_int64 * n)(*[m.out_features if y.dim() == 1 else y.stride(0) for y, m in zip(ys, self.mods)])
         rc = lib.cobalt_gemv_fused_staged(n, descs, ctypes.byref(inp), yp, ld, None, M, 1 if out_fp32 else 0,
                                           None if push is None else ctypes.byref(push.slots), sp,
-                                          self._scratch.numel() - (sp - self._scratch.data_ptr()),
+                                          sbytes,
                                           torch.cuda.current_stream(a.device).cuda_stream)
         if rc == _lib.EUNSUPPORTED:
             return None
