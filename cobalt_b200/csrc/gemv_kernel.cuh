@@ -213,7 +213,7 @@ __device__ __forceinline__ void gemv_stage_chunk(uint8_t* xs, int chunks_per_row
 }
 
 __device__ __noinline__ void gemv_stage_glu(const GemvParams& P, uint8_t* xs) {
-    constexpr int XPRE = 2;
+    constexpr int XPRE = 4;                                        // 16384 values with every load in flight at once
     const int chunks_per_row = P.N / 8, x_total = chunks_per_row * P.M;
     auto stage_chunk = [&](int m, int c, const uint4& v) { gemv_stage_chunk(xs, chunks_per_row, m, c, v); };
     // gated activation of the two halves of the previous projection, applied while staging
@@ -257,11 +257,15 @@ __device__ __noinline__ void gemv_stage_addnorm(const GemvParams& P, uint8_t* xs
         if (summed) return peer_sum_chunk(slot_row0, P.in_stride, P.in_world, (size_t)m * P.N + (size_t)c * 8);
         return __ldg(reinterpret_cast<const uint4*>(P.in_b + (size_t)m * P.in_ld) + c);
     };
-    uint4 hq[XPRE], dq[XPRE];
+    uint4 hq[XPRE], dq[XPRE], wq[XPRE];                            // the norm weights are requested with the rows, not after the sums
 #pragma unroll
     for (int q = 0; q < XPRE; ++q) {
         const int i = threadIdx.x + q * GEMV_THREADS;
-        if (i < x_total) { const int m = i / chunks_per_row; hq[q] = ld_h(m, i - m * chunks_per_row); }
+        if (i < x_total) {
+            const int m = i / chunks_per_row, c = i - m * chunks_per_row;
+            hq[q] = ld_h(m, c);
+            wq[q] = __ldg(reinterpret_cast<const uint4*>(P.in_w) + c);
+        }
     }
     if (summed) {                                                  // bounded wait for every rank's partial of this epoch
         const uint32_t e = *reinterpret_cast<const volatile uint32_t*>(P.in_flags + PEER_EPOCH_INDEX);
@@ -330,10 +334,10 @@ __device__ __noinline__ void gemv_stage_addnorm(const GemvParams& P, uint8_t* xs
         joined_total(i, v);
     }
     __syncthreads();
-    auto normed_chunk = [&](int m, int c, const float (&v)[8]) {
+    auto normed_chunk = [&](int m, int c, const float (&v)[8], const uint4& w) {
         const float r = row_rsqrt(tot_joined + m * groups, groups, P.N, P.in_eps);
         float wn[8], o[8];
-        chunk_to_floats(__ldg(reinterpret_cast<const uint4*>(P.in_w) + c), wn);
+        chunk_to_floats(w, wn);
 #pragma unroll
         for (int k = 0; k < 8; ++k) o[k] = normed_value(v[k], r, wn[k], P.in_flavor);
         stage_chunk(m, c, floats_to_chunk(o));
@@ -341,13 +345,13 @@ __device__ __noinline__ void gemv_stage_addnorm(const GemvParams& P, uint8_t* xs
 #pragma unroll
     for (int q = 0; q < XPRE; ++q) {
         const int i = threadIdx.x + q * GEMV_THREADS;
-        if (i < x_total) { const int m = i / chunks_per_row; normed_chunk(m, i - m * chunks_per_row, vk[q]); }
+        if (i < x_total) { const int m = i / chunks_per_row; normed_chunk(m, i - m * chunks_per_row, vk[q], wq[q]); }
     }
     for (int i = threadIdx.x + XPRE * GEMV_THREADS; i < x_total; i += GEMV_THREADS) {         // the rest is recomputed, not kept
         const int m = i / chunks_per_row, c = i - m * chunks_per_row;
         float v[8];
         joined_chunk(m, c, ld_h(m, c), has_delta2 ? ld_d(m, c) : make_uint4(0, 0, 0, 0), v);
-        normed_chunk(m, c, v);
+        normed_chunk(m, c, v, __ldg(reinterpret_cast<const uint4*>(P.in_w) + c));
     }
 }
 

@@ -63,10 +63,6 @@ __device__ __forceinline__ uint64_t umma_smem_desc_mn(uint32_t smem_addr, uint32
     return d;
 }
 __device__ __forceinline__ float exp2_approx(float x) { float y; asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x)); return y; }
-__device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
-    uint32_t d; asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(d) : "f"(hi), "f"(lo)); return d;
-}
-
 template <int D>
 __global__ void __launch_bounds__(PA_THREADS, 1) prompt_attn_kernel(const PromptAttnParams P, const __grid_constant__ CUtensorMap qmap,
                                                                     const __grid_constant__ CUtensorMap kmap,

@@ -17,7 +17,16 @@
 
 namespace cb {
 
-__device__ __forceinline__ float bf16_round(float f) { return bf16_to_float(float_to_bf16(f)); }
+// rounding to bf16 (nearest even) in one conversion; the integer form that keeps a NaN's payload took six operations per value,
+// three times per value of a gated activation
+__device__ __forceinline__ float bf16_round(float f) {
+    uint16_t h;
+    asm("cvt.rn.bf16.f32 %0, %1;" : "=h"(h) : "f"(f));
+    return bf16_to_float(h);
+}
+__device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
+    uint32_t d; asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(d) : "f"(hi), "f"(lo)); return d;
+}
 
 // ---- partial sums of a row-parallel layer exchanged over peer memory (layout shared by the GEMV's pushing epilogue,
 // its summing activation staging and the stand-alone kernels in glue_kernels.cuh).  Every rank owns one buffer:
@@ -88,10 +97,7 @@ __device__ __forceinline__ void chunk_to_floats(const uint4& c, float (&f)[8]) {
     }
 }
 __device__ __forceinline__ uint4 floats_to_chunk(const float (&f)[8]) {      // rounds to bf16 (nearest even)
-    uint32_t w[4];
-#pragma unroll
-    for (int k = 0; k < 4; ++k) w[k] = (uint32_t)float_to_bf16(f[2 * k]) | ((uint32_t)float_to_bf16(f[2 * k + 1]) << 16);
-    return make_uint4(w[0], w[1], w[2], w[3]);
+    return make_uint4(pack_bf16x2(f[0], f[1]), pack_bf16x2(f[2], f[3]), pack_bf16x2(f[4], f[5]), pack_bf16x2(f[6], f[7]));
 }
 __device__ __forceinline__ float chunk_sumsq(const float (&f)[8]) {
     float s = 0.0f;
