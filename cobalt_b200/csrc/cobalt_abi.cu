@@ -79,24 +79,27 @@ struct GemvCfg {
     int stages, mt, grid;
     bool xs;                           // activations staged in shared memory
     bool aligned;                      // every CTA holds whole row blocks
+    bool dense;                        // nothing pruned: tiles are copied row by row, 16 bytes apart
     uint32_t slot, xs_bytes, total_warps, part_q, part_r;
     size_t smem, counters_off, partials_off, xperm_off, total;
 };
 
 // geometry shared by the matrices of one (possibly fused) GEMV launch
-struct GemvGeom { int RB, CT, bits; uint32_t max_tile_bytes, max_tile_nnz; };
+struct GemvGeom { int RB, CT, bits; uint32_t max_tile_bytes, max_tile_nnz; bool dense; };
 
 GemvGeom geom_of(const CobaltMat* w) {
     GemvGeom g;
     g.RB = w->n_row_blocks; g.CT = w->n_col_tiles; g.bits = w->bits;
     g.max_tile_bytes = w->max_tile_bytes; g.max_tile_nnz = w->max_tile_nnz;
+    g.dense = w->nnz == (uint64_t)w->K * (uint64_t)w->N;
     return g;
 }
 
 int gemv_config(const GemvGeom& g, int N, int M, int num_sms, GemvCfg* c) {
     const int RB = g.RB, CT = g.CT;
     c->mt = M > 8 ? 2 : 1;
-    c->slot = (uint32_t)round_up((size_t)g.max_tile_bytes + 32, 128);
+    c->dense = g.dense;
+    c->slot = (uint32_t)round_up((size_t)g.max_tile_bytes + 32 + (g.dense ? TILE_ROWS * 16 : 0), 128);
     const size_t fixed = GEMV_LUT_BYTES + GEMV_BAR_BYTES + GEMV_REDCNT_BYTES + gemv_red_bytes(c->mt) + 64;
     // Two ring slots per warp keep one tile in flight behind the one being decoded.  The activations are staged in
     // shared memory when they fit beside such a ring (always for one token); what is left goes to deeper rings.
@@ -148,12 +151,15 @@ int gemv_config(const GemvGeom& g, int N, int M, int num_sms, GemvCfg* c) {
 
 template <int BITS, int MT, bool XS>
 int launch_gemv(const GemvParams& P, const GemvCfg& c, cudaStream_t st) {
-    // three kernels per shape class: the common launch, the one that also carries the staged-input and push modes, and the
-    // one for a column scale
-    const int kind = P.mode != 0 ? 1 : P.col_scale != nullptr ? 2 : 0;
-    void (*kernel)(const GemvParams) = kind == 1 ? gemv_mma_special_kernel<BITS, MT, XS> : kind == 2 ? gemv_mma_scaled_kernel<BITS, MT, XS>
-                                                                                                    : gemv_mma_kernel<BITS, MT, XS>;
-    static bool configured[MAX_DEVICES][3];
+    // kernels per shape class: the common launch, the one that also carries the staged-input and push modes, the one for a column
+    // scale, and the first two for matrices without pruned positions
+    const int kind = P.mode != 0 ? (c.dense ? 4 : 1) : P.col_scale != nullptr ? 2 : c.dense ? 3 : 0;
+    void (*kernel)(const GemvParams) = kind == 1   ? gemv_mma_special_kernel<BITS, MT, XS>
+                                       : kind == 2 ? gemv_mma_scaled_kernel<BITS, MT, XS>
+                                       : kind == 3 ? gemv_mma_dense_kernel<BITS, MT, XS>
+                                       : kind == 4 ? gemv_mma_dense_special_kernel<BITS, MT, XS>
+                                                   : gemv_mma_kernel<BITS, MT, XS>;
+    static bool configured[MAX_DEVICES][5];
     int dev = 0;
     cudaGetDevice(&dev);
     if (!configured[dev][kind]) {
@@ -402,6 +408,7 @@ int gemv_launch(int n, const CobaltMat* const* w, const GemvOut* out, const void
         else {
             if (w[i]->N != w[0]->N || w[i]->bits != w[0]->bits || w[i]->col_scale || w[0]->col_scale) return COBALT_EINVAL;
             g.RB += w[i]->n_row_blocks;
+            g.dense = g.dense && geom_of(w[i]).dense;
             if (w[i]->max_tile_bytes > g.max_tile_bytes) g.max_tile_bytes = w[i]->max_tile_bytes;
             if (w[i]->max_tile_nnz > g.max_tile_nnz) g.max_tile_nnz = w[i]->max_tile_nnz;
         }
@@ -608,6 +615,7 @@ size_t cobalt_gemv_fused_scratch_bytes(int n_mats, const CobaltMat* const* w, in
         if (i == 0) g = geom_of(w[0]);
         else {
             g.RB += w[i]->n_row_blocks;
+            g.dense = g.dense && geom_of(w[i]).dense;
             if (w[i]->max_tile_bytes > g.max_tile_bytes) g.max_tile_bytes = w[i]->max_tile_bytes;
             if (w[i]->max_tile_nnz > g.max_tile_nnz) g.max_tile_nnz = w[i]->max_tile_nnz;
         }

@@ -406,7 +406,10 @@ struct GemvUnit {
 // (GemvParams::mode != 0).  The common launch is a kernel of its own without any of that code, so that the
 // less common modes cost it neither a start-up test nor a register.  SCALED = the matrix has a column scale: its weights
 // are expanded like the others and finished in fp32 (decode8_scaled), a kernel of its own for the same reason.
-template <int BITS, int MT, bool XS, bool SPECIAL, bool SCALED>
+// DENSE = nothing is pruned (a compressed head).  Every row of a tile then has the same number of code bytes, a multiple of the 128
+// bytes of all banks at 4 bit: the code words of the 8 rows and 4 groups of a warp fall into two banks.  Full tiles are
+// copied row by row, 16 bytes apart, which spreads the rows over the banks: 32000 x 5376, 4 bit, 8 tokens 92 -> 56 us
+template <int BITS, int MT, bool XS, bool SPECIAL, bool SCALED, bool DENSE>
 __device__ __forceinline__ void gemv_mma_body(const GemvParams& P) {
     extern __shared__ __align__(1024) uint8_t smem[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -487,7 +490,11 @@ __device__ __forceinline__ void gemv_mma_body(const GemvParams& P) {
     const uint32_t lut_lane = smem_u32(lut_s) + (uint32_t)(lane & (GEMV_LUT_COPIES - 1)) * 16u;      // this lane's replica
     const uint32_t xs32 = smem_u32(xs);                               // 256-byte aligned: the swizzle is XORed into addresses
 
-    auto issue = [&](int i, int slot_idx, bool drained) {              // all lanes call; lane 0 acts
+    // a full-width tile in which every position (or all but what the rounding to 16 bytes hides) survives
+    constexpr uint32_t DENSE_HEAD = TILE_ROWS * TILE_GROUPS * 20, DENSE_ROW = TILE_GROUPS * GROUP * BITS / 8;
+    constexpr uint32_t DENSE_BYTES = DENSE_HEAD + TILE_ROWS * DENSE_ROW;
+    static_assert(DENSE_ROW % 16 == 0, "rows of a dense tile are copied one by one");
+    auto issue = [&](int i, int slot_idx, bool drained) {              // all lanes call; lane 0 acts (dense tiles: a lane per row)
         const uint8_t* base;
         uint32_t o0, o1;
         if (i < 32) {
@@ -496,6 +503,19 @@ __device__ __forceinline__ void gemv_mma_body(const GemvParams& P) {
             o1 = __shfl_sync(full, my_o1, i);
         } else {
             tile_offsets(tile_at(i), o0, o1, base);
+        }
+        if (DENSE && (o1 - o0) * 16u == DENSE_BYTES && (tile_at(i) + 1u) % (uint32_t)CT != 0u) {
+            const uint32_t bar = bar0 + 8 * slot_idx, dst = ring + slot_idx * P.slot_bytes;
+            if (lane == 0) {
+                if (drained) fence_proxy_async();
+                mbar_arrive_expect_tx(bar, DENSE_BYTES);
+                bulk_g2s_hint(dst, base + (size_t)o0 * 16, DENSE_HEAD, bar, pol_stream);
+            }
+            __syncwarp();
+            if (lane < TILE_ROWS)
+                bulk_g2s_hint(dst + DENSE_HEAD + (uint32_t)lane * (DENSE_ROW + 16u), base + (size_t)o0 * 16 + DENSE_HEAD + (uint32_t)lane * DENSE_ROW,
+                              DENSE_ROW, bar, pol_stream);
+            return;
         }
         if (lane == 0) {
             const uint32_t bar = bar0 + 8 * slot_idx;
@@ -721,6 +741,11 @@ __device__ __forceinline__ void gemv_mma_body(const GemvParams& P) {
         uint32_t bitA = (exc & 0xFFFFu) * BITS;                        // bit offset of the lane's first code, row A / row B
         uint32_t bitB = ((tot & 0xFFFFu) + (exc >> 16)) * BITS;
         const uint32_t cw = slot + TILE_ROWS * w * 20;                 // code stream of the tile
+        // copied row by row (the same test on the survivors as on the bytes when the copy was issued); `whole` when every row
+        // is full, else - a few codes short, same size - rows are read through the address map of the literal path
+        const bool by_rows = DENSE && ct + 1 != CT && ((tot & 0xFFFFu) + (tot >> 16)) * BITS + 127u >= (uint32_t)(TILE_ROWS * TILE_GROUPS * GROUP * BITS);
+        const bool whole = by_rows && (tot & 0xFFFFu) + (tot >> 16) == (uint32_t)(TILE_ROWS * TILE_GROUPS * GROUP);
+        const uint32_t cwA = DENSE && whole ? cw + 16u * (uint32_t)g : cw, cwB = DENSE && whole ? cw + 16u * (uint32_t)(g + 8) : cw;
         for (int r = 0; r < ja; ++r) {                                 // skip the words in front of the range
             bitA += BITS * __popc(mA.x); bitB += BITS * __popc(mB.x);
             mA.x = mA.y; mA.y = mA.z; mA.z = mA.w;
@@ -735,7 +760,7 @@ __device__ __forceinline__ void gemv_mma_body(const GemvParams& P) {
         const bool literal_scale = SPECIAL && P.col_scale != nullptr;  // the special launch has no scaled expansion
         const SegParams pA = make_seg_params(szA, BITS, literal_scale);
         const SegParams pB = make_seg_params(szB, BITS, literal_scale);
-        const bool all_fast = __all_sync(full, pA.fast && pB.fast);
+        const bool all_fast = __all_sync(full, pA.fast && pB.fast) && !(DENSE && by_rows && !whole);
         const int col0 = active ? (ct * TILE_GROUPS + t) * GROUP : 0;  // first column of this lane's group; lanes beyond a
                                                                        // partial tile read column 0, their zero weights cancel it
         // activations of this lane's group: staged copy (byte offset with the swizzle folded in) or global rows
@@ -752,7 +777,7 @@ __device__ __forceinline__ void gemv_mma_body(const GemvParams& P) {
             // ---- request everything unit `u` (16 columns: half h of mask word j) needs
             auto load_unit = [&](uint32_t m16A, uint32_t m16B, uint32_t bA, uint32_t bB, int j, int h) {
                 GemvUnit<MT, SCALED> Un;
-                const uint32_t pa = cw + ((bA >> 5) << 2), pb = cw + ((bB >> 5) << 2);
+                const uint32_t pa = cwA + ((bA >> 5) << 2), pb = cwB + ((bB >> 5) << 2);
                 Un.ra0 = lds32(pa); Un.ra1 = lds32(pa + 4); Un.ra2 = BITS == 2 ? 0u : lds32(pa + 8);
                 Un.rb0 = lds32(pb); Un.rb1 = lds32(pb + 4); Un.rb2 = BITS == 2 ? 0u : lds32(pb + 8);
                 Un.ea0 = lds128(lut_lane + (m16A & 0xFFu) * (GEMV_LUT_COPIES * 16u));
@@ -842,7 +867,7 @@ __device__ __forceinline__ void gemv_mma_body(const GemvParams& P) {
             }
         } else {
             // ---- literal fp32 path (off-grid zero points, scales that are not finite): one 32-column word at a time
-            auto word_at = [&](uint32_t k) { return lds32(cw + 4u * k); };
+            auto word_at = [&](uint32_t k) { return lds32(cw + 4u * k + (DENSE && by_rows ? 4u * k / DENSE_ROW * 16u : 0u)); };
 #pragma unroll 1
             for (int j = ja; j < jb; ++j) {
                 const uint32_t mAj = mA.x, mBj = mB.x;
@@ -910,17 +935,26 @@ __device__ __forceinline__ void gemv_mma_body(const GemvParams& P) {
 
 template <int BITS, int MT, bool XS>
 __global__ void __launch_bounds__(GEMV_THREADS, 1) gemv_mma_kernel(const GemvParams P) {
-    gemv_mma_body<BITS, MT, XS, false, false>(P);
+    gemv_mma_body<BITS, MT, XS, false, false, false>(P);
 }
 // one matrix with a column scale: 4096 x 4096, 4 bit, 5 tokens 15 us; one position at a time (the literal path) it took 70 us
 template <int BITS, int MT, bool XS>
 __global__ void __launch_bounds__(GEMV_THREADS, 1) gemv_mma_scaled_kernel(const GemvParams P) {
-    gemv_mma_body<BITS, MT, XS, false, true>(P);
+    gemv_mma_body<BITS, MT, XS, false, true, false>(P);
 }
 // parameters in place (their address is handed to the out-of-line staging and push functions)
 template <int BITS, int MT, bool XS>
 __global__ void __launch_bounds__(GEMV_THREADS, 1) gemv_mma_special_kernel(const __grid_constant__ GemvParams P) {
-    gemv_mma_body<BITS, MT, XS, true, false>(P);
+    gemv_mma_body<BITS, MT, XS, true, false, false>(P);
+}
+// matrices without pruned positions, plain and staged
+template <int BITS, int MT, bool XS>
+__global__ void __launch_bounds__(GEMV_THREADS, 1) gemv_mma_dense_kernel(const GemvParams P) {
+    gemv_mma_body<BITS, MT, XS, false, false, true>(P);
+}
+template <int BITS, int MT, bool XS>
+__global__ void __launch_bounds__(GEMV_THREADS, 1) gemv_mma_dense_special_kernel(const __grid_constant__ GemvParams P) {
+    gemv_mma_body<BITS, MT, XS, true, false, true>(P);
 }
 
 }  // namespace cb

@@ -85,3 +85,29 @@ def test_fused_launch(M):
     x = tokens(M, 1024)
     for m, y in zip(mods, FusedProjections(mods)(x)):
         check(m, x, y)
+
+
+@pytest.mark.parametrize("K,N,bits", [(64, 512, 4), (80, 1152, 4), (512, 2048, 3), (48, 640, 2), (2400, 1536, 4)])
+@pytest.mark.parametrize("M", [1, 5, 8, 16])
+def test_matrix_without_pruned_positions(K, N, bits, M):
+    """Full tiles copied row by row; a ragged last column tile, and rows beyond K (whose tiles are not full), are not."""
+    m, x = module(K, N, bits, sparsity=-1.0), tokens(M, N)
+    assert m._img_meta["nnz"] == K * N
+    check(m, x, m(x))
+
+
+@pytest.mark.parametrize("missing", [1, 31, 40])
+def test_almost_full_tile_in_a_launch_for_full_ones(missing):
+    """A tile a few codes short of full can have the bytes of a full one: the kernel must notice even if the survivor count of the
+    descriptor says that nothing is pruned."""
+    g = torch.Generator(device="cuda").manual_seed(missing)
+    W = torch.randn(48, 1024, generator=g, device="cuda") * 0.02
+    keep = torch.ones(48, 1024, dtype=torch.bool, device="cuda")
+    keep[19, 300:300 + missing] = False
+    q, s, z = quantize_survivors(W, keep, 4)
+    m, x = CobaltSparseLinear(q, s, z, keep, None, None, {"nbits": 4}), tokens(4, 1024)
+    W64 = m.dequantize()
+    m._img_meta["nnz"] = 48 * 1024
+    m._desc = None
+    exact = x.double() @ W64.double().t()
+    assert bool(((m(x).double() - exact).abs() <= exact.abs() * 2.0 ** -7 + exact.abs().max() * 1e-4).all())
