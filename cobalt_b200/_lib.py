@@ -78,7 +78,7 @@ EXPORTS = {
     "cobalt_gemm": (c_int, [POINTER(CobaltMat), c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_int, c_void_p,
                             c_size_t, c_void_p]),
     "cobalt_gemm_scratch_bytes": (c_size_t, [POINTER(CobaltMat), c_int]),
-    "cobalt_gemm_fused": (c_int, [c_int, c_void_p, c_void_p, c_int64, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_size_t,
+    "cobalt_gemm_fused": (c_int, [c_int, c_void_p, c_void_p, c_int64, c_void_p, c_void_p, c_void_p, c_int, c_int, c_void_p, c_size_t,
                                   c_void_p]),
     "cobalt_gemm_fused_scratch_bytes": (c_size_t, [c_int, c_void_p, c_int]),
     "cobalt_linear_f32": (c_int, [POINTER(CobaltMat), c_void_p, c_int64, c_void_p, c_int64, c_int, c_void_p, c_size_t,
@@ -105,7 +105,7 @@ EXPORTS = {
                                    c_int, c_float, c_int, c_int64, c_void_p]),
     "cobalt_argmax": (c_int, [c_void_p, c_int64, c_int, c_int64, c_void_p, c_void_p]),
     "cobalt_attn_prompt": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int,
-                                   c_float, c_void_p, c_void_p]),
+                                   c_float, c_int, c_int64, c_void_p, c_void_p]),
     "cobalt_attn_decode_fused": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_size_t, c_void_p, c_int, c_int, c_int,
                                          c_int, c_int, c_float, c_int, c_int64, c_void_p]),
     "cobalt_attn_decode_fused_scratch_bytes": (c_size_t, [c_int, c_int, c_int, c_int, c_int]),

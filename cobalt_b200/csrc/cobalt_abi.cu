@@ -204,7 +204,8 @@ struct GemmCfg {
 constexpr double GEMM_CLK_ALONE = 1280, GEMM_CLK_SHARED = 990, GEMM_CLK_PAIR = 1150, GEMM_CLK_MMA_TOKEN = 2.74, GEMM_CLK_SMEM = 1.56 / 128;
 constexpr double GEMM_CLK_TILE = 12000, GEMM_CLK_TILE_TOKEN = 47, GEMM_CLK_SPLIT = 1700, GEMM_CLK_SPLIT_TOKEN = 9.5;
 
-int gemm_config(int row_tiles, int G, int M, int num_sms, GemmCfg* c) {
+// `only_splits` > 0: that split, whatever it costs (the order of the sums is the caller's choice)
+int gemm_config(int row_tiles, int G, int M, int num_sms, GemmCfg* c, int only_splits = 0) {
     double best = 0;
     c->tok_per_cta = 0;
     for (int form = 0; form < 2; ++form) {
@@ -227,6 +228,7 @@ int gemm_config(int row_tiles, int G, int M, int num_sms, GemmCfg* c) {
             last = tpc;
             const long tok_tiles = ((long)M + tpc - 1) / tpc;
             for (int splits = 1; splits <= (pair ? GEMM_MAX_SPLITS / 2 : GEMM_MAX_SPLITS) && splits <= G; splits *= 2) {
+                if (only_splits > 0 && splits != only_splits) continue;
                 if (g_tune_gemm_stages > 0 && splits != g_tune_gemm_stages) continue;      // tuning key 2 overrides the split-K factor
                 const double ctas = (double)rows * tok_tiles * splits;
                 const int cluster = pair ? 2 * splits : splits;
@@ -328,19 +330,19 @@ int launch_gemm(const GemmParams& P, const CUtensorMap& xmap, const GemmCfg& c, 
     return c.pair ? launch_gemm<BITS, true, false>(P, xmap, c, st) : launch_gemm<BITS, false, false>(P, xmap, c, st);
 }
 
-// bf16 tensor of three dimensions, box 64 elements wide (one 128-byte swizzle row)
-int make_map_3d(CUtensorMap* map, const void* p, const cuuint64_t* dim, const cuuint64_t* stride, const cuuint32_t* box) {
+// bf16 tensor of up to four dimensions, box 64 elements wide (one 128-byte swizzle row)
+int make_map(CUtensorMap* map, const void* p, int rank, const cuuint64_t* dim, const cuuint64_t* stride, const cuuint32_t* box) {
     TensorMapEncodeFn enc = tensor_map_encoder();
     if (!enc) return COBALT_ELAUNCH;
-    const cuuint32_t estr[3] = {1, 1, 1};
-    CUresult r = enc(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(p), dim, stride, box, estr,
+    const cuuint32_t estr[4] = {1, 1, 1, 1};
+    CUresult r = enc(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, (cuuint32_t)rank, const_cast<void*>(p), dim, stride, box, estr,
                      CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                      CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     return r == CUDA_SUCCESS ? COBALT_OK : COBALT_EINVAL;
 }
 
 template <int D>
-int launch_prompt_attn(const PromptAttnParams& P, unsigned ctas, const CUtensorMap& qm, const CUtensorMap& km, const CUtensorMap& vm,
+int launch_prompt_attn(const PromptAttnParams& P, dim3 grid, const CUtensorMap& qm, const CUtensorMap& km, const CUtensorMap& vm,
                        cudaStream_t st) {
     static bool configured[MAX_DEVICES];
     int dev = 0;
@@ -350,7 +352,7 @@ int launch_prompt_attn(const PromptAttnParams& P, unsigned ctas, const CUtensorM
             return COBALT_ELAUNCH;
         configured[dev] = true;
     }
-    prompt_attn_kernel<D><<<ctas, PA_THREADS, pa_smem_bytes(D), st>>>(P, qm, km, vm);
+    prompt_attn_kernel<D><<<grid, PA_THREADS, pa_smem_bytes(D), st>>>(P, qm, km, vm);
     return cudaGetLastError() == cudaSuccess ? COBALT_OK : COBALT_ELAUNCH;
 }
 
@@ -706,7 +708,7 @@ size_t cobalt_gemm_scratch_bytes(const CobaltMat* w, int M) {
 }
 
 static int gemm_impl(int n, const CobaltMat* const* w, const GemvOut* out, const void* x, int64_t ldx, int M, void* scratch,
-                     size_t scratch_bytes, void* stream, bool fp32_out) {
+                     size_t scratch_bytes, void* stream, bool fp32_out, int sum_tokens = 0) {
     if (n < 1 || n > GEMV_MAX_MATS || !w || !out) return COBALT_EINVAL;
     GemmParams P = {};
     int row_tiles = 0;
@@ -730,7 +732,13 @@ static int gemm_impl(int n, const CobaltMat* const* w, const GemvOut* out, const
     int rc = device_info(&sms);
     if (rc) return rc;
     GemmCfg c;
-    rc = gemm_config(row_tiles, w[0]->N / GROUP, M, sms, &c);
+    int splits = 0;
+    if (sum_tokens > 0 && sum_tokens != M) {
+        rc = gemm_config(row_tiles, w[0]->N / GROUP, sum_tokens, sms, &c);
+        if (rc) return rc;
+        splits = c.splits;
+    }
+    rc = gemm_config(row_tiles, w[0]->N / GROUP, M, sms, &c, splits);
     if (rc) return rc;
     if (!scratch || ((uintptr_t)scratch & 255) || scratch_bytes < SCRATCH_STATUS_BYTES + SCRATCH_COUNTER_BYTES) return COBALT_ESCRATCH;
     CUtensorMap xmap;
@@ -760,11 +768,11 @@ size_t cobalt_gemm_fused_scratch_bytes(int n_mats, const CobaltMat* const* w, in
 }
 
 int cobalt_gemm_fused(int n_mats, const CobaltMat* const* w, const void* x, int64_t ldx, void* const* y, const int64_t* ldy,
-                      const void* const* bias, int M, void* scratch, size_t scratch_bytes, void* stream) {
-    if (n_mats < 1 || n_mats > GEMV_MAX_MATS || !w || !y || !ldy) return COBALT_EINVAL;
+                      const void* const* bias, int M, int sum_tokens, void* scratch, size_t scratch_bytes, void* stream) {
+    if (n_mats < 1 || n_mats > GEMV_MAX_MATS || !w || !y || !ldy || sum_tokens < 0) return COBALT_EINVAL;
     GemvOut o[GEMV_MAX_MATS];
     for (int i = 0; i < n_mats; ++i) { o[i].y = y[i]; o[i].ldy = ldy[i]; o[i].bias = bias ? bias[i] : nullptr; }
-    return gemm_impl(n_mats, w, o, x, ldx, M, scratch, scratch_bytes, stream, false);
+    return gemm_impl(n_mats, w, o, x, ldx, M, scratch, scratch_bytes, stream, false, sum_tokens);
 }
 
 int cobalt_gemm(const CobaltMat* w, const void* x, int64_t ldx, void* y, int64_t ldy, const void* bias, int M,
@@ -1021,9 +1029,11 @@ int cobalt_attn_decode_fused(const void* q, const void* k_cache, const void* v_c
 }
 
 int cobalt_attn_prompt(const void* q, const void* k_cache, const void* v_cache, const int64_t* positions, void* out, int T,
-                       int n_heads, int n_kv_heads, int head_dim, int n_slots, int max_ctx, int window, float scale, void* status,
-                       void* stream) {
+                       int n_heads, int n_kv_heads, int head_dim, int n_slots, int max_ctx, int window, float scale, int n_seq,
+                       int64_t cache_seq_stride, void* status, void* stream) {
     if (!q || !k_cache || !v_cache || !positions || !out || T <= 0) return COBALT_EINVAL;
+    if (n_seq < 1 || n_seq > 65535 || (int64_t)n_seq * T > 0x7FFFFFFFll || cache_seq_stride < 0 || (cache_seq_stride & 7)) return COBALT_EINVAL;
+    if (n_seq > 1 && cache_seq_stride == 0) return COBALT_EINVAL;
     if (n_heads <= 0 || n_kv_heads <= 0 || n_heads % n_kv_heads != 0) return COBALT_EINVAL;
     if (n_slots <= 0 || n_slots > max_ctx || max_ctx > (1 << 24) || window < 0) return COBALT_EINVAL;
     if (((uintptr_t)q | (uintptr_t)k_cache | (uintptr_t)v_cache | (uintptr_t)out) & 15) return COBALT_EINVAL;
@@ -1041,16 +1051,19 @@ int cobalt_attn_prompt(const void* q, const void* k_cache, const void* v_cache, 
     const long tiles = ((long)T + P.tok_per_cta - 1) / P.tok_per_cta * n_kv_heads;
     if (tiles > 0x7FFFFFFFl) return COBALT_ETOOBIG;
     CUtensorMap qm, km, vm;
-    const cuuint64_t qdim[3] = {(cuuint64_t)head_dim, (cuuint64_t)n_heads, (cuuint64_t)T};
+    const cuuint64_t qdim[3] = {(cuuint64_t)head_dim, (cuuint64_t)n_heads, (cuuint64_t)n_seq * T};
     const cuuint64_t qstr[2] = {(cuuint64_t)head_dim * 2, (cuuint64_t)n_heads * head_dim * 2};
     const cuuint32_t qbox[3] = {64, (cuuint32_t)rep, (cuuint32_t)P.tok_per_cta};
-    const cuuint64_t kdim[3] = {(cuuint64_t)head_dim, (cuuint64_t)n_slots, (cuuint64_t)n_kv_heads};   // slots beyond n_slots read as zero
-    const cuuint64_t kstr[2] = {(cuuint64_t)head_dim * 2, (cuuint64_t)max_ctx * head_dim * 2};
-    const cuuint32_t kbox[3] = {64, PA_KEYS, 1};
-    if ((rc = make_map_3d(&qm, q, qdim, qstr, qbox)) || (rc = make_map_3d(&km, k_cache, kdim, kstr, kbox)) ||
-        (rc = make_map_3d(&vm, v_cache, kdim, kstr, kbox))) return rc;
-    return head_dim == 64 ? launch_prompt_attn<64>(P, (unsigned)tiles, qm, km, vm, (cudaStream_t)stream)
-                          : launch_prompt_attn<128>(P, (unsigned)tiles, qm, km, vm, (cudaStream_t)stream);
+    // slots beyond n_slots read as zero
+    const cuuint64_t kdim[4] = {(cuuint64_t)head_dim, (cuuint64_t)n_slots, (cuuint64_t)n_kv_heads, (cuuint64_t)n_seq};
+    const cuuint64_t one_seq = (cuuint64_t)n_kv_heads * max_ctx * head_dim;
+    const cuuint64_t kstr[3] = {(cuuint64_t)head_dim * 2, (cuuint64_t)max_ctx * head_dim * 2, (n_seq > 1 ? (cuuint64_t)cache_seq_stride : one_seq) * 2};
+    const cuuint32_t kbox[4] = {64, PA_KEYS, 1, 1};
+    if ((rc = make_map(&qm, q, 3, qdim, qstr, qbox)) || (rc = make_map(&km, k_cache, 4, kdim, kstr, kbox)) ||
+        (rc = make_map(&vm, v_cache, 4, kdim, kstr, kbox))) return rc;
+    const dim3 grid((unsigned)tiles, (unsigned)n_seq);
+    return head_dim == 64 ? launch_prompt_attn<64>(P, grid, qm, km, vm, (cudaStream_t)stream)
+                          : launch_prompt_attn<128>(P, grid, qm, km, vm, (cudaStream_t)stream);
 }
 
 int cobalt_swiglu(const void* gate, const void* up, void* out, int64_t n, int act, void* stream) {

@@ -40,13 +40,17 @@ constexpr uint32_t pa_smem_bytes(int D) {
 static_assert(pa_smem_bytes(128) <= 227 * 1024, "the 128-wide head fills the shared memory of one SM");
 
 struct PromptAttnParams {
-    const long long* positions;            // [T]
-    uint16_t* out;                         // [T][n_kv * rep * D]
+    const long long* positions;            // [T], the same for every sequence (blockIdx.y)
+    uint16_t* out;                         // [sequence][T][n_kv * rep * D]
     int T, n_kv, rep, tok_per_cta, S, window;
     float scale;
     uint32_t* status;                      // may be null
 };
 
+__device__ __forceinline__ void tma_load_4d(uint32_t dst, const CUtensorMap* map, int x, int y, int z, int w, uint32_t bar) {
+    asm volatile("cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], [%6];"
+                 ::"r"(dst), "l"(map), "r"(x), "r"(y), "r"(z), "r"(w), "r"(bar) : "memory");
+}
 __device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* map, int x, int y, int z, uint32_t bar) {
     asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
                  ::"r"(dst), "l"(map), "r"(x), "r"(y), "r"(z), "r"(bar) : "memory");
@@ -215,7 +219,7 @@ __global__ void __launch_bounds__(PA_THREADS, 1) prompt_attn_kernel(const Prompt
                 tmem_ld32(tmem_o + my_lanes + (uint32_t)col, v);
                 tmem_ld_wait();
                 if (valid) {
-                    uint4* dst = reinterpret_cast<uint4*>(P.out + ((size_t)tok * P.n_kv * P.rep + (size_t)kvh * P.rep + head) * D + col);
+                    uint4* dst = reinterpret_cast<uint4*>(P.out + (((size_t)blockIdx.y * P.T + tok) * P.n_kv * P.rep + (size_t)kvh * P.rep + head) * D + col);
 #pragma unroll
                     for (int c = 0; c < 4; ++c) {
                         uint32_t o[4];
@@ -232,7 +236,7 @@ __global__ void __launch_bounds__(PA_THREADS, 1) prompt_attn_kernel(const Prompt
         // (loops on the whole warp, the instructions elected: see elect_one())
         if (elect_one()) {
             mbar_arrive_expect_tx(bar_q, (uint32_t)(P.rep * P.tok_per_cta) * 128u * SUBS);
-            for (int c = 0; c < SUBS; ++c) tma_load_3d(q_base + c * PA_SUB, &qmap, 64 * c, kvh * P.rep, tok0, bar_q);
+            for (int c = 0; c < SUBS; ++c) tma_load_3d(q_base + c * PA_SUB, &qmap, 64 * c, kvh * P.rep, (int)blockIdx.y * P.T + tok0, bar_q);
         }
         __syncwarp();
         bool healthy = true;
@@ -243,7 +247,7 @@ __global__ void __launch_bounds__(PA_THREADS, 1) prompt_attn_kernel(const Prompt
             if (elect_one()) {
                 mbar_arrive_expect_tx(bar_full(s), TILE);
 #pragma unroll
-                for (int c = 0; c < SUBS; ++c) tma_load_3d(ring + s * TILE + c * PA_SUB, map, 64 * c, jt * PA_KEYS, kvh, bar_full(s));
+                for (int c = 0; c < SUBS; ++c) tma_load_4d(ring + s * TILE + c * PA_SUB, map, 64 * c, jt * PA_KEYS, kvh, (int)blockIdx.y, bar_full(s));
             }
             __syncwarp();
             if (++s == PA_RING) { s = 0; ph ^= 1u; }

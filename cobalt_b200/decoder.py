@@ -243,13 +243,13 @@ class CobaltDecoder:
         _lib.check("cobalt_attn_decode", rc)
         return ctx
 
-    def _attn_prompt(self, q, positions, layer, seq: int, n_slots: int):
-        """Attention of the T tokens of a prompt over cache slots [0, n_slots) of sequence ``seq``, one kernel."""
+    def _attn_prompt(self, q, positions, layer, seq: int, n_slots: int, n_seq: int = 1):
+        """Attention of the prompts of ``n_seq`` sequences from ``seq`` on (``q [n_seq * T, nh*D]``) over cache slots [0, n_slots), one kernel."""
         ctx = torch.empty_like(q)
         window = int(self.cfg.get("sliding_window") or 0) if self.types[layer] == "sliding_attention" else 0
         rc = self._lib.cobalt_attn_prompt(q.data_ptr(), self.k_cache[layer][seq].data_ptr(), self.v_cache[layer][seq].data_ptr(),
-                                          positions.data_ptr(), ctx.data_ptr(), q.shape[0], self.nh, self.nkv, self.cfg["head_dim"],
-                                          n_slots, self.max_ctx, window, self.scale, self.prompt_status.data_ptr(),
+                                          positions.data_ptr(), ctx.data_ptr(), q.shape[0] // n_seq, self.nh, self.nkv, self.cfg["head_dim"],
+                                          n_slots, self.max_ctx, window, self.scale, n_seq, self.seq_stride, self.prompt_status.data_ptr(),
                                           torch.cuda.current_stream(self.dev).cuda_stream)
         _lib.check("cobalt_attn_prompt", rc)
         return ctx
@@ -436,6 +436,42 @@ class CobaltDecoder:
         torch.cuda.synchronize()
         return e0.elapsed_time(e1) / reps
 
+    def _prompts_at_once(self, T: int) -> int:
+        """How many sequences' prompts of ``T`` tokens run through the layers together: weights are expanded once for all of them.
+        Every row's sums are added as if its sequence ran alone (``sum_tokens``), so the logits do not depend on it.  Up to 8192 rows
+        (activations of a few GB at the widest MLPs); prompts that the decode GEMV takes, tensor parallelism and head
+        widths without the prompt kernel run one by one."""
+        if self.world > 1 or T <= 16 or not self.prompt_kernel or self.fused_prompt_attention:
+            return 1
+        return max(1, min(self.B, 8192 // T))
+
+    def _forward_prompts(self, ids: torch.Tensor, positions: torch.Tensor, first: int) -> torch.Tensor:
+        """``ids [n, T]``: the prompts of sequences ``first`` .. ``first + n - 1`` at the same ``positions [T]``; logits ``[n, T, V]``."""
+        cfg, P = self.cfg, self.P
+        n, T = ids.shape
+        h = P["model.embed_tokens.weight"].index_select(0, ids.reshape(-1))            # [n*T, H]
+        if self.gemma:
+            h = h * self.embed_scale
+        delta, delta_w = None, None
+        for i in range(cfg["num_hidden_layers"]):
+            p = f"model.layers.{i}."
+            h, x = self._add_rmsnorm(h, delta, P[p + "input_layernorm.weight"], delta_w if delta is not None else None)
+            q, k, v = self.qkv[i](x, T)
+            for b in range(n):
+                r = slice(b * T, (b + 1) * T)
+                self._rope_kv(q[r], k[r], v[r], positions, i, first + b)
+            (o,) = self.o_f[i](self._attn_prompt(q, positions, i, first, T, n), T)
+            if self.gemma:
+                h, x = self._add_rmsnorm(h, o, P[p + "pre_feedforward_layernorm.weight"], P[p + "post_attention_layernorm.weight"])
+                delta_w = P[p + "post_feedforward_layernorm.weight"]
+            else:
+                h, x = self._add_rmsnorm(h, o, P[p + "post_attention_layernorm.weight"])
+            (delta,) = self.down[i](self._swiglu(*self.gate_up[i](x, T)), T)
+        h, x = self._add_rmsnorm(h, delta, P["model.norm.weight"], delta_w)
+        if self.head_f is not None:
+            return self.head_f(x, T)[0].view(n, T, -1)
+        return torch.stack([self._head_logits(x[b * T:(b + 1) * T]) for b in range(n)])        # the library's GEMM, one shape for all
+
     def _check_room(self, n_tokens: int, start: int = 0):
         if start < 0 or start + n_tokens > self.max_ctx:
             raise ValueError(f"{n_tokens} tokens from position {start} do not fit the KV cache of {self.max_ctx} slots")
@@ -452,7 +488,13 @@ class CobaltDecoder:
         T = ids2.shape[1]
         self._check_room(T)
         pos = torch.arange(T, device=self.dev)
-        logits = torch.stack([self._forward(ids2[b], pos, T, seq=b)[0] for b in range(ids2.shape[0])])
+        n, at_once = ids2.shape[0], self._prompts_at_once(T)
+        if at_once > 1 and n > 1:
+            parts = [self._forward_prompts(ids2[b:b + at_once], pos, b) for b in range(0, n, at_once)]
+            logits = parts[0] if len(parts) == 1 else torch.cat(parts)
+        else:
+            parts = [self._forward(ids2[b], pos, T, seq=b) for b in range(n)]              # [1, T, V] each
+            logits = parts[0] if n == 1 else torch.cat(parts)
         self.pos.fill_(T)
         return logits[0] if single else logits
 

@@ -339,7 +339,8 @@ class FusedProjections:
         self._key = [(m._img_meta, m._buffers["packed"].data_ptr()) for m in self.mods]      # held, so that neither can be reused
         return self._args
 
-    def __call__(self, x: torch.Tensor):
+    def __call__(self, x: torch.Tensor, sum_tokens: int = 0):
+        """``sum_tokens``: above 16 tokens, add every sum in the order of a launch of that many tokens (0: the fastest)."""
         N = self.mods[0].in_features
         flat = x.dim() == 2 and x.shape[1] == N
         x2 = x if flat else x.reshape(-1, N)
@@ -355,9 +356,11 @@ class FusedProjections:
         lib = _lib.load()
         descs, ld, sp, sbytes = self._prepare(x2.device)
         ys = [x2.new_empty((M, m.out_features)) for m in self.mods]
-        rc = (lib.cobalt_gemv_fused if M <= GEMV_MAX_TOKENS else lib.cobalt_gemm_fused)(
-            len(ys), descs, x2.data_ptr(), x2.stride(0), self._ptrs(*[y.data_ptr() for y in ys]), ld, None, M, sp, sbytes,
-            _raw_stream(x2.get_device()))
+        yp, stream = self._ptrs(*[y.data_ptr() for y in ys]), _raw_stream(x2.get_device())
+        if M <= GEMV_MAX_TOKENS:
+            rc = lib.cobalt_gemv_fused(len(ys), descs, x2.data_ptr(), x2.stride(0), yp, ld, None, M, sp, sbytes, stream)
+        else:
+            rc = lib.cobalt_gemm_fused(len(ys), descs, x2.data_ptr(), x2.stride(0), yp, ld, None, M, sum_tokens, sp, sbytes, stream)
         if rc:
             _lib.check("cobalt_gemv_fused" if M <= GEMV_MAX_TOKENS else "cobalt_gemm_fused", rc)
         return ys if flat else [y.reshape(*x.shape[:-1], m.out_features) for y, m in zip(ys, self.mods)]

@@ -199,9 +199,11 @@ size_t cobalt_gemm_scratch_bytes(const CobaltMat* w, int M);
 
 /* Prefill GEMM of up to four matrices that read the same activations (q|k|v, gate|up) as one launch: equal in_features and
  * bit width, no column scale; y[i], ldy[i], bias[i] (bias or its entries may be NULL) per matrix.  Same results as cobalt_gemm()
- * up to the order in which fp32 sums are added; the 128-row tiles of all matrices fill the GPU together. */
+ * up to the order in which fp32 sums are added; the 128-row tiles of all matrices fill the GPU together.  sum_tokens > 0: the
+ * columns are split - hence every sum is added - as in a launch of that many tokens, so that the prompts of several
+ * sequences in one launch give each the bits it gets alone; 0: as is fastest for M. */
 int cobalt_gemm_fused(int n_mats, const CobaltMat* const* w, const void* x, int64_t ldx, void* const* y, const int64_t* ldy,
-                      const void* const* bias, int M, void* scratch, size_t scratch_bytes, void* stream);
+                      const void* const* bias, int M, int sum_tokens, void* scratch, size_t scratch_bytes, void* stream);
 size_t cobalt_gemm_fused_scratch_bytes(int n_mats, const CobaltMat* const* w, int M);
 
 /* Same product with the raw fp32 sums as output (no bias, no rounding): M <= 16 runs the GEMV,
@@ -328,10 +330,11 @@ int cobalt_argmax(const void* logits, int64_t ld, int rows, int64_t V, int64_t* 
  * [n_kv_heads][max_ctx][D]: token t attends the slots s < n_slots with s <= positions[t] (and s > positions[t] - window when
  * window > 0).  Same rounding points as cobalt_attn_decode(); scores and probabilities stay on the chip.  D 64 or 128 and at
  * most 128 query heads per KV head, else COBALT_EUNSUPPORTED (nothing launched).  q, caches and out 16-byte aligned.  status
- * (may be NULL): a u32 that is set when a bounded wait gives up. */
+ * (may be NULL): a u32 that is set when a bounded wait gives up.  n_seq > 1: that many sequences of T tokens at once, q and out
+ * [n_seq][T][n_heads*D], the same positions, sequence b's caches at k_cache/v_cache + b * cache_seq_stride elements (a multiple of 8). */
 int cobalt_attn_prompt(const void* q, const void* k_cache, const void* v_cache, const int64_t* positions, void* out, int T,
-                       int n_heads, int n_kv_heads, int head_dim, int n_slots, int max_ctx, int window, float scale, void* status,
-                       void* stream);
+                       int n_heads, int n_kv_heads, int head_dim, int n_slots, int max_ctx, int window, float scale, int n_seq,
+                       int64_t cache_seq_stride, void* status, void* stream);
 
 /* All-reduce (sum) of the fp32 partial outputs of a row-parallel layer over peer memory, for tensor-parallel decode
  * (the reference has no distributed code; this replaces the NCCL all-reduce that would follow cobalt_linear_f32).

@@ -30,7 +30,7 @@ def spec(q, k, v, pos, n_slots, window, scale, nh, nkv, D):
 def call(q, k, v, pos, n_slots, window, scale, nh, nkv, D):
     out, status = torch.full_like(q, float("nan")), torch.zeros(1, dtype=torch.int32, device=q.device)
     rc = _lib.load().cobalt_attn_prompt(q.data_ptr(), k.data_ptr(), v.data_ptr(), pos.data_ptr(), out.data_ptr(), q.shape[0], nh, nkv,
-                                        D, n_slots, k.shape[1], window, scale, status.data_ptr(),
+                                        D, n_slots, k.shape[1], window, scale, 1, 0, status.data_ptr(),
                                         torch.cuda.current_stream().cuda_stream)
     return rc, out, status
 
@@ -74,3 +74,26 @@ def test_unsupported_shapes_are_refused():
     pos = torch.arange(4, device="cuda")
     assert call(q, k, k, pos, 4, 0, 0.1, 4, 2, 96)[0] == _lib.EUNSUPPORTED
     assert call(q, k, k, pos, 9, 0, 0.1, 4, 2, 96)[0] != 0                       # more slots than the cache has
+
+
+@pytest.mark.parametrize("family,batch,T", [("llama", 3, 17), ("gemma", 8, 40), ("llama", 5, 150)])
+def test_prompts_together_equal_prompts_alone(family, batch, T):
+    """Prompts of several sequences through the layers at once: the logits and caches of each are those of its prompt alone."""
+    from cobalt_b200 import SparseQuantConfig
+    from cobalt_b200.decoder import build_random_decoder
+    from oracle import model_oracle as MO
+    if family == "gemma":
+        cfg = MO.gemma3_config(hidden=512, layers=2, heads=8, kv_heads=2, head_dim=64, inter=1024, vocab=1008, sliding_window=16, pattern=2,
+                               query_pre_attn_scalar=96, rope_scaling={"rope_type": "linear", "factor": 8.0})
+    else:
+        cfg = MO.llama_config(hidden=512, layers=2, heads=8, kv_heads=2, head_dim=64, inter=1024, vocab=1008)
+    dec = build_random_decoder(cfg, SparseQuantConfig(4, 0.5, 0.5), T + 8, torch.device("cuda"), batch=batch, head_bits=4)
+    ids = torch.randint(0, 1000, (batch, T), generator=torch.Generator().manual_seed(T))
+    assert dec._prompts_at_once(T) == batch
+    together = dec.prefill(ids)
+    kc, vc = dec.k_cache.clone(), dec.v_cache.clone()
+    pos = torch.arange(T, device="cuda")
+    for b in range(batch):
+        assert torch.equal(dec._forward(ids[b].cuda(), pos, T, seq=b)[0], together[b]), b
+    assert torch.equal(dec.k_cache, kc) and torch.equal(dec.v_cache, vc)
+    assert int(dec.prompt_status) == 0
