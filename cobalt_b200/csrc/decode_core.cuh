@@ -358,10 +358,10 @@ CB_HD void decode32_fast(uint32_t m, uint32_t w0, uint32_t w1, uint32_t w2, uint
 // One mask byte of a fast segment, decoded straight from the `BITS`-wide code stream (no re-pack to
 // nibbles).  `w0` holds the codes of this byte's survivors from bit 0 upwards (8 * BITS bits are looked
 // at).  code_view() turns them into a word whose byte k carries rank 2k in its low bits and whose copy
-// shifted right by HI_SHIFT carries rank 2k+1 there; bits above the code width are junk and are masked
+// shifted right by HI_SHIFT = BITS carries rank 2k+1 there; bits above the code width are junk and are masked
 // off when the bf16 pattern is formed.
 //   4 bit: the stream itself (nibbles);
-//   3 bit: three shift-and-select steps spread the eight 3-bit fields to nibbles (bit 3 of each is junk);
+//   3 bit: two shift-and-select steps put the four 6-bit pairs into bytes (a third one, to nibbles, cost the GEMV 5 %);
 //   2 bit: one byte permute puts ranks 0,2,4,6 into bits 0..1 of bytes 0..3 and ranks 1,3,5,7 into bits 2..3.
 // selA / selB / self are the table fields of the mask byte (see Lut4), out[i] = bf16x2 weights of
 // positions (2i, 2i+1).
@@ -376,14 +376,13 @@ CB_HD uint32_t code_view(uint32_t w0) {
     if (BITS == 4) return w0;
     if (BITS == 2) return prmt(w0, w0 >> 4, 0x5140u);
     const uint32_t t = (w0 & 0x0000FFFFu) | ((w0 << 4) & 0xFFFF0000u);
-    const uint32_t u = (t & 0x00FF00FFu) | ((t << 2) & 0xFF00FF00u);
-    return (u & 0x0F0F0F0Fu) | ((u << 1) & 0xF0F0F0F0u);
+    return (t & 0x00FF00FFu) | ((t << 2) & 0xFF00FF00u);
 }
 
 // dq(e, i) turns the bf16x2 pattern {128 + c0, 128 + c1} of positions (2i, 2i+1) into their weights
 template <int BITS, class Dq>
 CB_HD void decode8_with(uint32_t w0, uint32_t selA, uint32_t selB, uint32_t self, uint32_t zq, Dq dq, uint32_t out[4]) {
-    constexpr uint32_t HI_SHIFT = BITS == 2 ? 2u : 4u;
+    constexpr uint32_t HI_SHIFT = (uint32_t)BITS;
     constexpr uint32_t CM = ((1u << BITS) - 1u) * 0x00010001u;
     const uint32_t v = code_view<BITS>(w0);
     const uint32_t hi = prmt(v >> HI_SHIFT, zq, self);        // byte 3 <- zero point unless all eight are kept
