@@ -227,6 +227,7 @@ int gemm_config(int row_tiles, int G, int M, int num_sms, GemmCfg* c, int only_s
             if (tpc == last) continue;
             last = tpc;
             const long tok_tiles = ((long)M + tpc - 1) / tpc;
+            if (tok_tiles > 65535) continue;
             for (int splits = 1; splits <= (pair ? GEMM_MAX_SPLITS / 2 : GEMM_MAX_SPLITS) && splits <= G; splits *= 2) {
                 if (only_splits > 0 && splits != only_splits) continue;
                 if (g_tune_gemm_stages > 0 && splits != g_tune_gemm_stages) continue;      // tuning key 2 overrides the split-K factor
@@ -249,7 +250,7 @@ int gemm_config(int row_tiles, int G, int M, int num_sms, GemmCfg* c, int only_s
             }
         }
     }
-    if (c->tok_per_cta == 0 || c->grid.y > 65535u) return COBALT_ETOOBIG;
+    if (c->tok_per_cta == 0) return COBALT_ETOOBIG;
     c->box_rows = (uint32_t)(c->pair ? c->acc_tokens / 2 : c->acc_tokens);
     c->b_acc_bytes = c->box_rows * GEMM_KS * 2;
     c->b_stage_bytes = c->b_acc_bytes * (uint32_t)(c->tok_per_cta / c->acc_tokens);

@@ -39,6 +39,8 @@ def _ptr(t: Optional[torch.Tensor]) -> Optional[int]:
 class CobaltSparseLinear(nn.Module):
     """y = x @ dequant(W).T (+ bias), weights held as bitmask + low-bit survivors."""
 
+    _launch = None                                           # also of modules saved whole before it existed
+
     def __init__(self, W_q, scales, zeros, mask, scale2=None, bias=None, meta=None):
         super().__init__()
         meta = dict(meta or {})
@@ -65,7 +67,7 @@ class CobaltSparseLinear(nn.Module):
         self._scratch = None
         self._desc = None
         self._desc_key = None
-        self._launch = {}
+        self._launch = None
 
     @classmethod
     def _blank(cls):
@@ -210,6 +212,8 @@ class CobaltSparseLinear(nn.Module):
         bufs = self._buffers
         scale2 = bufs["scale2"]
         key = (bufs["packed"].data_ptr(), None if scale2 is None else scale2.data_ptr())
+        if self._launch is None:
+            self._launch = {}
         args = self._launch.get(kind)
         if args is None or args[0] != key:
             desc = self._descriptor()
@@ -293,7 +297,7 @@ class CobaltSparseLinear(nn.Module):
         out = super()._apply(fn, *a, **k)
         self._desc = None
         self._scratch = None
-        self._launch = {}
+        self._launch = None
         return out
 
     def extra_repr(self) -> str:
@@ -308,6 +312,8 @@ class FusedProjections:
     launch: the decode GEMV for up to 16 tokens (``cobalt_gemv_fused``), the tcgen05 GEMM above that
     (``cobalt_gemm_fused``).  The reference reaches the same goal by concatenating the matrices row-wise at pack time (docs/FORMAT.md:126-151)."""
 
+    _key = _args = None
+
     def __init__(self, mods):
         mods = list(mods)
         if not 1 <= len(mods) <= FUSED_MAX:
@@ -319,7 +325,6 @@ class FusedProjections:
         self._scratch = None
         self._key = None
         self._args = None
-        self._ptrs = ctypes.c_void_p * len(mods)
 
     def _prepare(self, device):
         """``(descriptors, row strides, scratch address, scratch bytes)``, worked out again when a module's image is another one."""
@@ -345,8 +350,8 @@ class FusedProjections:
         flat = x.dim() == 2 and x.shape[1] == N
         x2 = x if flat else x.reshape(-1, N)
         M = x2.shape[0]
-        if M == 0:
-            return [m(x) for m in self.mods]
+        if M == 0 or (M > GEMV_MAX_TOKENS and any(m._forward_hooks or m._forward_pre_hooks for m in self.mods)):
+            return [m(x) for m in self.mods]                 # a prompt runs the hooks of its modules
         if not x2.is_cuda or x2.dtype != torch.bfloat16:
             if M > GEMV_MAX_TOKENS:
                 return [m(x) for m in self.mods]             # raises what a module raises
@@ -356,7 +361,7 @@ class FusedProjections:
         lib = _lib.load()
         descs, ld, sp, sbytes = self._prepare(x2.device)
         ys = [x2.new_empty((M, m.out_features)) for m in self.mods]
-        yp, stream = self._ptrs(*[y.data_ptr() for y in ys]), _raw_stream(x2.get_device())
+        yp, stream = (ctypes.c_void_p * len(ys))(*[y.data_ptr() for y in ys]), _raw_stream(x2.get_device())
         if M <= GEMV_MAX_TOKENS:
             rc = lib.cobalt_gemv_fused(len(ys), descs, x2.data_ptr(), x2.stride(0), yp, ld, None, M, sp, sbytes, stream)
         else:
