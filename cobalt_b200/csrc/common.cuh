@@ -44,9 +44,6 @@ __device__ __forceinline__ int tile_width(const MatView& w, int ct) {
     return rem < TILE_GROUPS ? rem : TILE_GROUPS;
 }
 
-// expansion table, constant-initialised at compile time
-__device__ const LutTable g_lut = make_expand_lut();
-
 // status codes a kernel may leave in the scratch status word
 enum : uint32_t {
     DEV_OK = 0,

@@ -18,8 +18,8 @@
 // both passes (two roundings, scale, maximum, two exponentials, sum, product, packing): about 2300 issue cycles at four
 // warp instructions per cycle, against 1570 cycles of tensor work.  Hence eight softmax warps on one CTA per SM (two per
 // scheduler, 32 independent values each) rather than four, and no third pass.
-// Measured (1965 MHz): 2048 tokens, 32 / 8 heads of 128: 115 us per layer, where batched matmuls with element-wise passes over
-// the scores took 1490 us; 1024 tokens 39 us; 200 tokens, 32 / 16 heads 14.5 us.
+// Measured (1965 MHz): 2048 tokens, 32 / 8 heads of 128: 108 us per layer, where batched matmuls with element-wise passes over
+// the scores took 1490 us; 1024 tokens 37.6 us; 200 tokens, 32 / 16 heads 14.5 us.
 #pragma once
 #include "gemm_kernel.cuh"
 
