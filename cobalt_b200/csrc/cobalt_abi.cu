@@ -152,8 +152,10 @@ int gemv_config(const GemvGeom& g, int N, int M, int num_sms, GemvCfg* c) {
 template <int BITS, int MT, bool XS>
 int launch_gemv(const GemvParams& P, const GemvCfg& c, cudaStream_t st) {
     // kernels per shape class: the common launch, the one that also carries the staged-input and push modes, the one for a column
-    // scale, and the first two for matrices without pruned positions
-    const int kind = P.mode != 0 ? (c.dense ? 4 : 1) : P.col_scale != nullptr ? 2 : c.dense ? 3 : 0;
+    // scale, and the first two for matrices without pruned positions.  A column scale that 16-byte loads cannot read takes the
+    // second kernel, whose literal path reads it one value at a time.
+    const bool odd_scale = ((uintptr_t)P.col_scale & 15) != 0;
+    const int kind = P.mode != 0 || odd_scale ? (c.dense ? 4 : 1) : P.col_scale != nullptr ? 2 : c.dense ? 3 : 0;
     void (*kernel)(const GemvParams) = kind == 1   ? gemv_mma_special_kernel<BITS, MT, XS>
                                        : kind == 2 ? gemv_mma_scaled_kernel<BITS, MT, XS>
                                        : kind == 3 ? gemv_mma_dense_kernel<BITS, MT, XS>
@@ -748,6 +750,7 @@ static int gemm_impl(int n, const CobaltMat* const* w, const GemvOut* out, const
     P.n_mats = n;
     P.G = w[0]->N / GROUP; P.CT = w[0]->n_col_tiles;
     P.col_scale = (const uint16_t*)w[0]->col_scale;
+    P.literal_scale = ((uintptr_t)P.col_scale & 15) != 0;
     P.M = M;
     P.tok_per_cta = c.tok_per_cta; P.acc_tokens = c.acc_tokens; P.splits = c.splits;
     P.a_stages = c.a_stages; P.b_stages = c.b_stages;

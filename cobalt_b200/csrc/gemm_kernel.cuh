@@ -73,6 +73,7 @@ struct GemmParams {
     int n_mats;
     int G, CT;
     const uint16_t* col_scale;  // fp16 bits; the SCALED instantiation only (single-matrix launches)
+    bool literal_scale;         // not on a 16-byte boundary: read one value at a time, by the literal path
     int M;
     int tok_per_cta;            // tokens per token tile
     int acc_tokens;             // tokens per accumulator (tok_per_cta = one or two of these)
@@ -386,7 +387,7 @@ __global__ void __launch_bounds__(gemm_threads(PAIR), PAIR ? 1 : 2) gemm_tcgen05
         for (int g = g_begin + set; g < g_end; g += STEP) {
             GemmFetch<BITS> nxt = {};
             if (g + STEP < g_end) take(nxt, g + STEP);
-            const SegParams sp = make_seg_params(cur.sz, BITS, false);
+            const SegParams sp = make_seg_params(cur.sz, BITS, SCALED && P.literal_scale);
             uint32_t words[4 * GemmFetch<BITS>::NC];
 #pragma unroll
             for (int i = 0; i < GemmFetch<BITS>::NC; ++i) {

@@ -32,6 +32,12 @@ def _scratch_span(buf: torch.Tensor):
     return p, buf.numel() - (p - buf.data_ptr())
 
 
+def _kernel_scale(scale2: torch.Tensor) -> torch.Tensor:
+    """Column scale as the kernels read it fastest: contiguous fp16 on a 16-byte boundary (a slice of a larger buffer may lie anywhere)."""
+    s = scale2.reshape(-1).to(torch.float16).contiguous()
+    return s if s.data_ptr() % 16 == 0 else s.clone()
+
+
 def _ptr(t: Optional[torch.Tensor]) -> Optional[int]:
     return None if t is None else t.data_ptr()
 
@@ -62,7 +68,7 @@ class CobaltSparseLinear(nn.Module):
         self._img_meta = img.meta()
         self.register_buffer("packed", img.blob)
         has_scale2 = scale2 is not None and not bool((scale2.float() == 1).all())
-        self.register_buffer("scale2", scale2.reshape(-1).to(torch.float16).to(img.blob.device) if has_scale2 else None)
+        self.register_buffer("scale2", _kernel_scale(scale2.to(img.blob.device)) if has_scale2 else None)
         self.bias = nn.Parameter(bias.detach().clone(), requires_grad=False) if bias is not None else None
         self._scratch = None
         self._desc = None

@@ -50,7 +50,8 @@ extern "C" {
 typedef struct CobaltMat {
     const void*     tiles;          /* first tile, 16-byte aligned */
     const uint32_t* tile_off;       /* n_row_blocks * n_col_tiles + 1 entries, 16-byte units */
-    const void*     col_scale;      /* optional fp16[N] per-input-column scale (reference `scale2`), or NULL */
+    const void*     col_scale;      /* optional fp16[N] per-input-column scale (reference `scale2`), or NULL; any
+                                       address, but off a 16-byte boundary it takes the kernels' slow path */
     int32_t K, N;                   /* out_features, in_features */
     int32_t bits;                   /* 2, 3 or 4 */
     int32_t group;                  /* 128 */

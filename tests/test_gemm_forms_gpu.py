@@ -60,6 +60,20 @@ def test_column_scale(M, bits):
     check(m, x, m(x))
 
 
+@pytest.mark.parametrize("M", [1, 16, 40, 600])
+@pytest.mark.parametrize("sparsity", [0.5, -1.0])
+def test_column_scale_at_any_address(M, sparsity):
+    """A scale off the 16-byte boundary is read one value at a time: the same arithmetic, hence the same bits."""
+    buf = torch.exp(torch.randn(1153 + 8, generator=torch.Generator(device="cuda").manual_seed(5), device="cuda") * 0.25).half()
+    m, x = module(272, 1152, 4, sparsity=sparsity, scale2=buf[1:1153]), tokens(M, 1152)
+    assert m.scale2.data_ptr() % 16 == 0                          # the module keeps an aligned copy of the slice
+    want = m(x)
+    m.scale2 = buf[1:1153]                                        # a caller's own pointer, as through the C ABI
+    assert m.scale2.data_ptr() % 16 == 2
+    check(m, x, want)
+    assert torch.equal(m(x), want)
+
+
 @pytest.mark.parametrize("M", [2, 40, 600])
 @pytest.mark.parametrize("scaled", [False, True])
 def test_zero_points_off_the_grid(M, scaled):
