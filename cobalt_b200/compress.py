@@ -18,9 +18,10 @@ from __future__ import annotations
 from dataclasses import dataclass
 
 import torch
+import torch.autograd.forward_ad as fwAD
 
 from . import _lib
-from .format import GROUP
+from .format import GROUP, kernels_take
 
 
 @dataclass
@@ -110,7 +111,7 @@ def keep_mask(weight: torch.Tensor, act_norm: torch.Tensor, sparsity: float, bet
     K, N = weight.shape
     if sparsity <= 0.0:
         return torch.ones(K, N, dtype=torch.bool, device=weight.device)
-    if weight.is_cuda and act_norm.is_cuda and N % GROUP == 0 and act_norm.numel() == N and int(K * N * sparsity) >= 1:
+    if kernels_take(weight, act_norm) and N % GROUP == 0 and act_norm.numel() == N and 1 <= int(K * N * sparsity) <= K * N:
         return _keep_mask_cuda(weight, act_norm, sparsity, beta)
     score = weight.float().abs() * act_norm.float().view(1, -1)
     n_row, n_col = int(N * sparsity), int(K * sparsity)
@@ -132,7 +133,9 @@ def quantize_survivors(weight: torch.Tensor, keep: torch.Tensor, bits: int, grou
     if N % group_size:
         raise ValueError(f"in_features {N} is not a multiple of group_size {group_size}")
     G = N // group_size
-    if weight.is_cuda and keep.is_cuda and keep.dtype == torch.bool and keep.shape == weight.shape and group_size == GROUP:
+    differentiated = torch.is_grad_enabled() and weight.requires_grad or fwAD.unpack_dual(weight).tangent is not None
+    if kernels_take(weight, keep) and keep.dtype == torch.bool and keep.shape == weight.shape and group_size == GROUP \
+            and 1 <= bits <= 8 and 0 < K * N < 1 << 34 and not differentiated:
         lib = _lib.load()
         with torch.cuda.device(weight.device):
             w, kb = _dense_for_kernel(weight), keep.contiguous()

@@ -74,6 +74,18 @@ class TileImage:
         return self.K * self.N // 8 + (self.bits * self.nnz + 7) // 8 + self.K * (self.N // GROUP) * 4
 
 
+def _ordinary(t: torch.Tensor) -> bool:
+    """A tensor with memory of its own: no subclass (fake, distributed, ...), not inside ``vmap`` or another function transform."""
+    return type(t) in (torch.Tensor, torch.nn.Parameter) and not torch._C._functorch.is_functorch_wrapped_tensor(t)
+
+
+def kernels_take(*tensors: torch.Tensor) -> bool:
+    """Whether a CUDA kernel may be given these tensors' addresses: ordinary tensors, all on the same GPU.  Anything else takes the
+    torch form, which works on it or says what is wrong (tensors on two devices, above all)."""
+    dev = tensors[0].device
+    return dev.type == "cuda" and all(t.device == dev and _ordinary(t) for t in tensors)
+
+
 def _round_up(x: int, a: int) -> int:
     return (x + a - 1) // a * a
 
@@ -97,7 +109,7 @@ def pack_tiles(keep: torch.Tensor, q: torch.Tensor, scale: torch.Tensor, zero: t
     CT = (G + TILE_GROUPS - 1) // TILE_GROUPS
     Kp, Gp = RB * TILE_ROWS, CT * TILE_GROUPS
 
-    if keep.is_cuda and q.is_cuda and q.shape == keep.shape and RB <= 65535:         # row blocks are a grid dimension there
+    if kernels_take(keep, q) and q.shape == keep.shape and 0 < RB <= 65535:          # row blocks are a grid dimension there
         return _pack_tiles_cuda(keep, q, scale.reshape(K, G), zero.reshape(K, G), bits)
     keep_b = keep != 0
     qi = q.to(torch.int64)

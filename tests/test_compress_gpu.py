@@ -70,3 +70,20 @@ def test_packing_of_empty_and_full_masks(density):
         for form in (q, q.to(torch.uint8)):                  # a surviving code outside the grid is refused
             with pytest.raises(ValueError):
                 F.pack_tiles(keep.cuda(), form.cuda(), sc.cuda(), zr.cuda(), 3)
+
+
+def test_rounding_under_transforms_on_the_gpu():
+    """Derivatives, ``vmap``, empty matrices and wide codes: the torch form, as on the CPU, not a kernel that is handed addresses."""
+    g = torch.Generator().manual_seed(4)
+    W, keep = torch.randn(6, 256, generator=g), torch.rand(6, 256, generator=g) > 0.5
+    Wc, kc = W.cuda(), keep.cuda()
+    q, s, z = C.quantize_survivors(W, keep, 4)
+    leaf = Wc.clone().requires_grad_()
+    q2, s2, z2 = C.quantize_survivors(leaf, kc, 4)
+    assert s2.requires_grad and torch.equal(q2.cpu(), q) and bits_equal(s2.detach(), s)
+    with torch.no_grad():
+        assert not C.quantize_survivors(leaf, kc, 4)[1].requires_grad
+    q3 = torch.vmap(lambda w, k: C.quantize_survivors(w, k, 4)[0])(Wc.view(2, 3, 256), kc.view(2, 3, 256))
+    assert torch.equal(q3.view(6, 256).cpu(), q)
+    assert [tuple(t.shape) for t in C.quantize_survivors(Wc[:0], kc[:0], 4)] == [(0, 256), (0, 2), (0, 2)]
+    assert torch.equal(C.quantize_survivors(Wc, kc, 9)[0].cpu(), C.quantize_survivors(W, keep, 9)[0])

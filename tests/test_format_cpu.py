@@ -98,3 +98,47 @@ def test_linear_tags():
     m.model.add_module("layers", torch.nn.ModuleList([torch.nn.ModuleDict({"q_proj": torch.nn.Linear(128, 16)})]))
     m.add_module("lm_head", torch.nn.Linear(128, 8))
     assert get_linear_tags_from_model(m) == ["q_proj"]
+
+
+def test_compression_kernels_only_take_tensors_of_one_gpu(monkeypatch):
+    """Tensors on two GPUs never reach a kernel: torch's own error names the devices, as on the CPU.  Fake tensors stand in for
+    those of two GPUs; any attempt to launch fails the test."""
+    from torch._subclasses import FakeTensorMode
+    from cobalt_b200 import _lib
+
+    def no_launch():
+        raise AssertionError("a kernel was about to get these tensors")
+
+    monkeypatch.setattr(_lib, "load", no_launch)
+    with FakeTensorMode():
+        def make(device):
+            return (torch.empty(16, 256, device=device), torch.empty(256, device=device), torch.empty(16, 256, dtype=torch.bool, device=device),
+                    torch.empty(16, 256, dtype=torch.uint8, device=device))
+
+        w, norm, keep, q = make("cuda:0")
+        w1, norm1, keep1, q1 = make("cuda:1")
+        sz = torch.empty(16, 2, dtype=torch.float16, device="cuda:0")
+        for args in ((w, norm), (w1, norm1), (keep, q)):          # not ordinary tensors, whatever their device
+            assert not F.kernels_take(*args)
+        monkeypatch.setattr(F, "_ordinary", lambda t: True)
+        assert F.kernels_take(w, norm, keep, q) and F.kernels_take(w1, norm1)
+        for a, b in ((w, norm1), (w1, norm), (w, keep1), (keep, q1), (w, norm.cpu())):
+            assert not F.kernels_take(a, b)
+        for call, what in ((lambda: C.keep_mask(w1, norm, 0.5, 0.5), "device"), (lambda: C.quantize_survivors(w, keep1, 4), "device"),
+                           (lambda: F.pack_tiles(keep, q1, sz, sz, 4), "")):      # a fake mask has no positions to name before that
+            with pytest.raises(RuntimeError, match=what):
+                call()
+
+
+def test_rounding_under_transforms_and_without_rows():
+    """Forms that address-taking kernels cannot serve stay with torch: derivatives, vmap, empty matrices, more than 4 bits."""
+    W = torch.randn(6, 256)
+    keep = torch.rand(6, 256) > 0.5
+    scale = C.quantize_survivors(W.clone().requires_grad_(), keep, 4)[1]
+    assert scale.requires_grad
+    q, s, z = torch.vmap(lambda w, k: C.quantize_survivors(w, k, 4))(W.view(2, 3, 256), keep.view(2, 3, 256))
+    assert torch.equal(q.view(6, 256), C.quantize_survivors(W, keep, 4)[0])
+    assert [tuple(t.shape) for t in C.quantize_survivors(W[:0], keep[:0], 4)] == [(0, 256), (0, 2), (0, 2)]
+    seen = []
+    torch.vmap(lambda w: (seen.append(F._ordinary(w)), w)[1])(W)
+    assert seen == [False] and F._ordinary(W) and F._ordinary(torch.nn.Parameter(W))
