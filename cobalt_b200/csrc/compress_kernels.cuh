@@ -328,17 +328,22 @@ __global__ void __launch_bounds__(256) quantize_groups_kernel(const T* W, const 
     const int lane = threadIdx.x & 31;
     const size_t at = g * GROUP + 4 * lane;
     const uint32_t kp = *reinterpret_cast<const uint32_t*>(keep + at);
-    float w[4], lo = 3.402823466e38f, hi = -3.402823466e38f;
+    constexpr float LIMIT = 3.402823466e38f;                            // what a pruned position counts as
+    float w[4], lo = INFINITY, hi = -INFINITY;
+    bool nan = false;                                                  // fminf and fmaxf drop a NaN; the hull carries it
     load4(W, at / 4, w);
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-        if ((kp >> (8 * i)) & 0xFFu) { lo = fminf(lo, w[i]); hi = fmaxf(hi, w[i]); }
+        const bool kept = ((kp >> (8 * i)) & 0xFFu) != 0u;
+        lo = fminf(lo, kept ? w[i] : LIMIT); hi = fmaxf(hi, kept ? w[i] : -LIMIT);
+        nan = nan || (kept && w[i] != w[i]);
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
         lo = fminf(lo, __shfl_xor_sync(0xFFFFFFFFu, lo, o));
         hi = fmaxf(hi, __shfl_xor_sync(0xFFFFFFFFu, hi, o));
     }
+    if (__any_sync(0xFFFFFFFFu, nan)) lo = hi = __uint_as_float(0x7FC00000u);
     if (!__any_sync(0xFFFFFFFFu, kp != 0u)) { lo = 0.0f; hi = 0.0f; }
     const float top = (float)((1 << bits) - 1);
     float span = __fsub_rn(hi, lo);

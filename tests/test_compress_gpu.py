@@ -87,3 +87,23 @@ def test_rounding_under_transforms_on_the_gpu():
     assert torch.equal(q3.view(6, 256).cpu(), q)
     assert [tuple(t.shape) for t in C.quantize_survivors(Wc[:0], kc[:0], 4)] == [(0, 256), (0, 2), (0, 2)]
     assert torch.equal(C.quantize_survivors(Wc, kc, 9)[0].cpu(), C.quantize_survivors(W, keep, 9)[0])
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_damaged_weights_show_in_scale_and_zero_point(dtype):
+    """A NaN or an infinity among the survivors of a group makes the scale (and zero point) what the torch form makes of it, so that the
+    outputs show the damage; the same value at a pruned position changes nothing."""
+    nan, inf = float("nan"), float("inf")
+    W = (torch.randn(8, 384, generator=torch.Generator().manual_seed(9)) * 0.02).to(dtype)
+    keep = torch.ones(8, 384, dtype=torch.bool)
+    W[0, 5], W[1, 130], W[2, 383], W[3, 0] = nan, inf, -inf, nan
+    keep[3, 0] = False                                       # pruned: harmless
+    W[4, :128], W[5, 128:256], W[6, 256:] = inf, -inf, inf
+    keep[6, 300] = False                                     # an all-infinite group with and without a pruned position
+    W[7, 7], W[7, 8], W[7, 200], keep[7, 200] = inf, -inf, inf, False
+    want = C.quantize_survivors(W, keep, 4)
+    got = [t.cpu() for t in C.quantize_survivors(W.cuda(), keep.cuda(), 4)]
+    assert torch.equal(got[0], want[0])
+    for a, b in zip(got[1:], want[1:]):
+        assert torch.equal(a.isnan(), b.isnan()) and bits_equal(a.nan_to_num(nan=1.5), b.nan_to_num(nan=1.5))
+    assert bool(got[1][0, 0].isnan()) and not bool(got[1][3, 0].isnan())
