@@ -111,7 +111,7 @@ def keep_mask(weight: torch.Tensor, act_norm: torch.Tensor, sparsity: float, bet
     K, N = weight.shape
     if sparsity <= 0.0:
         return torch.ones(K, N, dtype=torch.bool, device=weight.device)
-    if kernels_take(weight, act_norm) and N % GROUP == 0 and act_norm.numel() == N and 1 <= int(K * N * sparsity) <= K * N:
+    if kernels_take(weight, act_norm) and N % GROUP == 0 and act_norm.numel() == N and 1 <= int(K * N * sparsity) <= K * N < 1 << 32:
         return _keep_mask_cuda(weight, act_norm, sparsity, beta)
     score = weight.float().abs() * act_norm.float().view(1, -1)
     n_row, n_col = int(N * sparsity), int(K * sparsity)

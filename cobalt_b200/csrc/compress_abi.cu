@@ -9,6 +9,12 @@ int check_shape(int K, int N) {
     if (K <= 0 || N <= 0 || N % GROUP != 0 || (unsigned long long)K * (unsigned)N >= (1ull << 34)) return COBALT_EINVAL;
     return COBALT_OK;
 }
+// scoring: counts, ranks and the element index of score_columns_kernel are 32-bit words
+int check_scores(int K, int N) {
+    const int rc = check_shape(K, N);
+    if (rc) return rc;
+    return (unsigned long long)K * (unsigned)N < (1ull << 32) ? COBALT_OK : COBALT_ETOOBIG;
+}
 int check_tiling(int K, int N) {
     const int rc = check_shape(K, N);
     if (rc) return rc;
@@ -30,10 +36,10 @@ size_t cobalt_compress_state_bytes(void) { return sizeof(CompressState); }
 
 int cobalt_score_rows(const void* W, int w_type, const float* norm, int K, int N, int n_row, int n_col, uint32_t k_keep, float* scores,
                       float* col_kth, void* state, void* stream) {
-    int rc = check_shape(K, N);
+    int rc = check_scores(K, N);
     if (rc) return rc;
     if (!aligned16(W) || !aligned16(norm) || !aligned16(scores) || !aligned16(state) || w_type < 0 || w_type > 2) return COBALT_EINVAL;
-    if (n_row < 0 || n_row > N || n_col < 0 || n_col > K || (n_col > 0 && !col_kth) || k_keep < 1) return COBALT_EINVAL;
+    if (n_row < 0 || n_row > N || n_col < 0 || n_col > K || (n_col > 0 && !col_kth) || k_keep < 1 || k_keep > (unsigned long long)K * (unsigned)N) return COBALT_EINVAL;
     cudaStream_t st = (cudaStream_t)stream;
     CompressState* S = (CompressState*)state;
     compress_state_init_kernel<<<1, 512, 0, st>>>(S, k_keep);
@@ -48,7 +54,7 @@ int cobalt_score_rows(const void* W, int w_type, const float* norm, int K, int N
 
 int cobalt_keep_from_scores(float* scores, const float* col_div, int K, int N, int rows_normalised, int bracketed, void* state,
                             uint8_t* keep, void* stream) {
-    int rc = check_shape(K, N);
+    int rc = check_scores(K, N);
     if (rc) return rc;
     if (!aligned16(scores) || !aligned16(state) || !aligned16(keep)) return COBALT_EINVAL;
     int sms = 0;

@@ -251,7 +251,7 @@ int cobalt_gemv_fused_host_async(int n_mats, const CobaltMat* const* w, const vo
 
 /* Compression of a dense weight on the GPU (cobalt_b200/compress.py and format.py drive these; every result equals their torch
  * form bit for bit; reference: src/cobaltkernel/cobalt_math.py:15-32, 144-168).  W [K, N] row-major, w_type 0 fp32 / 1 fp16 /
- * 2 bf16, 16-byte aligned; N % 128 == 0, K * N < 2^34.
+ * 2 bf16, 16-byte aligned; N % 128 == 0, K * N < 2^34 (the two scoring calls: < 2^32, else COBALT_ETOOBIG).
  *   cobalt_score_rows        : scores [K, N] fp32 = |W| * norm, with n_row > 0 over the row's n_row-th smallest; with n_col > 0
  *                              also col_kth [N] = the n_col-th smallest of every column (after the division by the maximum).
  *                              `state` (cobalt_compress_state_bytes()) carries what the next call needs; k_keep = the number of

@@ -98,3 +98,12 @@ def test_decoder_refuses_more_tokens_than_cache_slots():
         CobaltDecoder._check_room(d, 33)
     with pytest.raises(ValueError):
         CobaltDecoder._check_room(d, 8, start=30)
+
+
+def test_scoring_refuses_what_32_bit_counts_cannot_hold(lib):
+    """Refused on the host, before any launch: 2^32 elements and more (the caller's torch form takes those), ranks beyond the matrix."""
+    big, odd = (1 << 16, 1 << 16), (1 << 25, 1 << 8)
+    for K, N in (big, odd):
+        assert lib.cobalt_score_rows(4096, 0, 4096, K, N, 1, 0, 5, 4096, None, 4096, None) == -6
+        assert lib.cobalt_keep_from_scores(4096, None, K, N, 0, 0, 4096, 4096, None) == -6
+    assert lib.cobalt_score_rows(4096, 0, 4096, 16, 128, 1, 0, 2049, 4096, None, 4096, None) == -1

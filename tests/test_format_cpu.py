@@ -125,9 +125,11 @@ def test_compression_kernels_only_take_tensors_of_one_gpu(monkeypatch):
         for a, b in ((w, norm1), (w1, norm), (w, keep1), (keep, q1), (w, norm.cpu())):
             assert not F.kernels_take(a, b)
         for call, what in ((lambda: C.keep_mask(w1, norm, 0.5, 0.5), "device"), (lambda: C.quantize_survivors(w, keep1, 4), "device"),
-                           (lambda: F.pack_tiles(keep, q1, sz, sz, 4), "")):      # a fake mask has no positions to name before that
+                           (lambda: F.pack_tiles(keep, q1, sz, sz, 4), "aten")):  # a fake mask has no positions to look at
             with pytest.raises(RuntimeError, match=what):
                 call()
+        with pytest.raises(RuntimeError, match="aten"):           # 2^32 elements: more than the kernels' counts hold
+            C.keep_mask(torch.empty(1 << 16, 1 << 16, device="cuda:0"), torch.empty(1 << 16, device="cuda:0"), 0.5, 0.5)
 
 
 def test_rounding_under_transforms_and_without_rows():
