@@ -14,12 +14,16 @@
 //              the context of tile j, so that the tensor pipe works under the softmax
 // Key tiles outside the causal / sliding range of the CTA's rows are skipped; only tiles that cross its border are masked.
 //
-// Bound: the element-wise work of the softmax warps.  A 128 x 128 tile holds 16384 scores that take about 17 operations over
-// both passes (two roundings, scale, maximum, two exponentials, sum, product, packing): about 2300 issue cycles at four
-// warp instructions per cycle, against 1570 cycles of tensor work.  Hence eight softmax warps on one CTA per SM (two per
-// scheduler, 32 independent values each) rather than four, and no third pass.
-// Measured (1965 MHz): 2048 tokens, 32 / 8 heads of 128: 108 us per layer, where batched matmuls with element-wise passes over
-// the scores took 1490 us; 1024 tokens 37.6 us; 200 tokens, 32 / 16 heads 14.5 us.
+// The softmax is fp32 as in the decode attention: expf, and probabilities that are quotients.  At scores far apart it rounds 17 of
+// a million probabilities to another bf16 value than an exact softmax, torch's fp32 softmax 15; a power of two of the
+// product with log2(e) and a product with the reciprocal were 16 % faster and rounded 144.  The division itself takes
+// 1.8 times as long as quotient() below (2048 tokens: 249 us), for the same bits.
+//
+// Bound: the element-wise work of the softmax warps.  A 128 x 128 tile holds 16384 scores that take about 30 operations over
+// both passes (two roundings, scale, maximum, two exponentials, sum, quotient, packing), against 1570 cycles of tensor work.
+// Hence eight softmax warps on one CTA per SM (two per scheduler, 32 independent values each) rather than four, and no third pass.
+// Measured (1965 MHz, cold L2): 2048 tokens, 32 / 8 heads of 128: 139 us per layer, where batched matmuls with element-wise
+// passes over the scores took 1490 us; 1024 tokens 50 us; 8 x 200 tokens, 32 / 16 heads 56 us.
 #pragma once
 #include "gemm_kernel.cuh"
 
@@ -66,7 +70,13 @@ __device__ __forceinline__ uint64_t umma_smem_desc_mn(uint32_t smem_addr, uint32
     d |= (uint64_t)2 << 61;
     return d;
 }
-__device__ __forceinline__ float exp2_approx(float x) { float y; asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x)); return y; }
+// a / b with inv = 1.0f / b, which every probability of a row shares: the quotient by the reciprocal, put right by its remainder
+// (Markstein, "Computation of elementary functions on the IBM RISC System/6000 processor", 1990).  Equal to the division
+// for the sums met here (1 <= b < 2^25).
+__device__ __forceinline__ float quotient(float a, float b, float inv) {
+    const float q = a * inv;
+    return fmaf(fmaf(-q, b, a), inv, q);
+}
 template <int D>
 __global__ void __launch_bounds__(PA_THREADS, 1) prompt_attn_kernel(const PromptAttnParams P, const __grid_constant__ CUtensorMap qmap,
                                                                     const __grid_constant__ CUtensorMap kmap,
@@ -137,7 +147,6 @@ __global__ void __launch_bounds__(PA_THREADS, 1) prompt_attn_kernel(const Prompt
             if (P.window > 0) lo = (int)max(0ll, min(pl, 0x3FFFFFFFll) - P.window + 1);
         }
         const uint32_t my_lanes = (uint32_t)((warp & 3) * 32) << 16;
-        constexpr float LOG2E = 1.4426950408889634f;
         bool healthy = true;
 
         // scaled, rounded and masked scores of this row's 64 keys of S tile `g` (key tile `jt`); frees the TMEM buffer
@@ -177,9 +186,9 @@ __global__ void __launch_bounds__(PA_THREADS, 1) prompt_attn_kernel(const Prompt
             for (int i = 4; i < 64; ++i) t[i & 3] = fmaxf(t[i & 3], x[i]);
             const float nm = fmaxf(m, fmaxf(fmaxf(t[0], t[1]), fmaxf(t[2], t[3])));
             const float base = nm == -INFINITY ? 0.0f : nm;             // nothing allowed so far: every exponential is zero
-            float s[4] = {l * exp2_approx((m - base) * LOG2E), 0.0f, 0.0f, 0.0f};
+            float s[4] = {l * expf(m - base), 0.0f, 0.0f, 0.0f};
 #pragma unroll
-            for (int i = 0; i < 64; ++i) s[i & 3] += exp2_approx((x[i] - base) * LOG2E);
+            for (int i = 0; i < 64; ++i) s[i & 3] += expf(x[i] - base);
             l = (s[0] + s[1]) + (s[2] + s[3]);
             m = nm;
         }
@@ -190,7 +199,7 @@ __global__ void __launch_bounds__(PA_THREADS, 1) prompt_attn_kernel(const Prompt
         const float gm = fmaxf(m, om);
         const float base = gm == -INFINITY ? 0.0f : gm;
         // (a sum of two: both halves get the same bits)
-        const float inv = 1.0f / (l * exp2_approx((m - base) * LOG2E) + ol * exp2_approx((om - base) * LOG2E));
+        const float tot = l * expf(m - base) + ol * expf(om - base), inv = 1.0f / tot;
 
         for (int j = 0; j < n && healthy; ++j) {                        // pass B
             float x[64];
@@ -199,7 +208,7 @@ __global__ void __launch_bounds__(PA_THREADS, 1) prompt_attn_kernel(const Prompt
             uint32_t p[32];
 #pragma unroll
             for (int i = 0; i < 32; ++i)
-                p[i] = pack_bf16x2(exp2_approx((x[2 * i] - base) * LOG2E) * inv, exp2_approx((x[2 * i + 1] - base) * LOG2E) * inv);
+                p[i] = pack_bf16x2(quotient(expf(x[2 * i] - base), tot, inv), quotient(expf(x[2 * i + 1] - base), tot, inv));
             healthy = __all_sync(full_mask, mbar_wait_bounded(bar_pempty(j & 1), ((uint32_t)(j >> 1) & 1u) ^ 1u, P.status, DEV_TIMEOUT_EMPTY));
             if (!healthy) break;
             const uint32_t row = p_base + (uint32_t)(j & 1) * PA_P_BYTES + (uint32_t)half * PA_SUB + (uint32_t)r * 128u;

@@ -55,6 +55,23 @@ def test_prompt_attention_matches_spec(T, nh, nkv, D, ctx, window, start, gain):
     assert float(d.abs().max()) <= 2.0 ** -6 * float(ref.abs().max())
 
 
+@pytest.mark.parametrize("gain", [1.0, 4.0, 12.0])
+def test_probabilities_are_those_of_an_fp32_softmax(gain):
+    """Unit vectors as keys and values: the scores are exact and the result is the probabilities themselves.  An fp32 softmax is off by
+    about 6e-8 (relative, on average) before the rounding to bf16, whose values lie 2^-8 to 2^-7 apart: about 2e-5 of them round
+    to the other side.  torch's own fp32 softmax: 1.1e-5 at most; a softmax of twice that error exceeds the bound."""
+    T, nh, D = 512, 16, 128
+    g = torch.Generator(device="cuda").manual_seed(2)
+    q = (torch.randn(T, nh * D, generator=g, device="cuda") * gain * D ** 0.5).bfloat16()
+    eye = torch.eye(128, device="cuda").bfloat16().view(1, 128, 128).contiguous()
+    pos = torch.full((T,), 127, device="cuda")
+    rc, out, status = call(q, eye, eye, pos, 128, 0, D ** -0.5, nh, 1, D)
+    scores = (q.float() * D ** -0.5).bfloat16().view(T, nh, 128)
+    want = torch.softmax(scores.double(), -1).bfloat16().view(T, nh * 128)
+    assert rc == 0 and int(status) == 0
+    assert float((out != want).float().mean()) <= 5e-5
+
+
 def test_slots_beyond_the_prompt_are_not_read():
     """What an earlier, longer prompt left in the cache (here: NaN) does not reach the result."""
     g = torch.Generator(device="cuda").manual_seed(3)
