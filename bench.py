@@ -355,7 +355,7 @@ def run_ours(args):
                 run_steps(max(2000, 10 * args.steps))
                 stream.synchronize()
         clocks = sampler.stop() if rank == 0 else None
-        status = max(m.device_status() for b in blocks for m in b.values())
+        status = max(o.device_status() for group in blocks + fuseds for o in group.values())
 
     if dist is not None:
         t = torch.tensor([ms], device=dev)
@@ -578,7 +578,7 @@ def extra_legs(dev, steps=5):
                     "ms_per_token_4_layers": round(ms4, 4), "ms_head_and_embedding": round(ms_head, 4), "ms_per_layer": round(ms_layer, 4),
                     "tokens_per_s_32_layers_extrapolated": round(1e3 / (32 * ms_layer + ms_head), 1),
                     "note": "extrapolated from 4 layers: 32 * ms_per_layer + head; the full-depth run is `--workload model`",
-                    "status": max(m.device_status() for m in dec.lin.values())}
+                    "status": dec.device_status()}
     del dec
     torch.cuda.empty_cache()
     return out
@@ -797,7 +797,7 @@ def run_model(args):
         dist.all_reduce(t, op=dist.ReduceOp.MAX)
         ms = float(t.item())
     wbytes = sum(m.compressed_bytes() for m in dec.lin.values()) * world
-    status = max(m.device_status() for m in dec.lin.values())
+    status = dec.device_status()
     if rank != 0:
         _finish(dist)
         return

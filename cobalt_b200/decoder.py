@@ -30,7 +30,7 @@ import torch.nn.functional as F
 
 from .compress import SparseQuantConfig, compress_weight
 from . import _lib
-from .linear import CobaltSparseLinear, FusedProjections
+from .linear import CobaltSparseLinear, FusedProjections, status_word
 
 PROJ = ("self_attn.q_proj", "self_attn.k_proj", "self_attn.v_proj", "self_attn.o_proj",
         "mlp.gate_proj", "mlp.up_proj", "mlp.down_proj")
@@ -418,6 +418,24 @@ class CobaltDecoder:
         h, x = self._add_rmsnorm(h, self._settled(delta), P["model.norm.weight"], delta_w)
         return self._head_logits(x).unsqueeze(0)                                            # [1, T, V]
 
+    def device_status(self) -> int:
+        """The worst status word of everything this decoder launches (0 = healthy): modules, fused launches, prompt and one-kernel
+        attention, peer all-reduce.  A launch whose bounded wait gave up leaves its output unwritten and its code here."""
+        words = [m.device_status() for m in self.lin.values()] + [int(self.prompt_status.item()), status_word(self.att_fused)]
+        words += [f.device_status() for fs in (self.qkv, self.gate_up, self.o_f, self.down) for f in fs]
+        if self.head_f is not None:
+            words += [self.head.device_status(), self.head_f.device_status()]
+        if self.reducer is not None:
+            words.append(self.reducer.device_status())
+        return max(words)
+
+    def _check_prompt_attention(self):
+        """Raise if a prompt's attention gave up waiting (its context is not written then); the next prompt starts afresh."""
+        word = int(self.prompt_status.item())
+        if word:
+            self.prompt_status.zero_()
+            raise _lib.CobaltError("cobalt_attn_prompt", word, "a bounded wait gave up: the attention of a prompt is incomplete")
+
     @torch.no_grad()
     def time_head_ms(self, reps: int = 20) -> float:
         """Device time of what a decode step spends outside the blocks: embedding lookup, final norm, head, argmax."""
@@ -479,7 +497,8 @@ class CobaltDecoder:
     @torch.no_grad()
     def prefill(self, ids: torch.Tensor) -> torch.Tensor:
         """Run the prompt(s), fill the cache(s), return the logits: ``ids [T]`` -> ``[T, V]`` (sequence 0), or
-        ``ids [B, T]`` (one prompt per sequence, equal lengths) -> ``[B, T, V]``."""
+        ``ids [B, T]`` (one prompt per sequence, equal lengths) -> ``[B, T, V]``.  Waits for nothing; ``device_status()`` says
+        whether the launches were healthy."""
         ids = ids.to(self.dev)
         single = ids.dim() == 1
         ids2 = ids.view(1, -1) if single else ids
@@ -553,6 +572,7 @@ class CobaltDecoder:
             if teacher is not None:
                 self.tok.copy_(teacher[i].reshape(-1).to(self.dev))
         toks = torch.cat(toks).cpu() if single else torch.stack(toks).cpu()
+        self._check_prompt_attention()                       # the tokens are there: costs no further wait
         return toks, torch.stack(all_logits)
 
 

@@ -32,6 +32,15 @@ def _scratch_span(buf: torch.Tensor):
     return p, buf.numel() - (p - buf.data_ptr())
 
 
+def status_word(buf: Optional[torch.Tensor]) -> int:
+    """Status word at the aligned start of a scratch buffer: 0, or the code of the first bounded wait that gave up.  Waits for the
+    current stream."""
+    if buf is None:
+        return 0
+    at = _scratch_span(buf)[0] - buf.data_ptr()
+    return int(buf[at:at + 4].view(torch.int32).item())
+
+
 def _kernel_scale(scale2: torch.Tensor) -> torch.Tensor:
     """Column scale as the kernels read it fastest: contiguous fp16 on a 16-byte boundary (a slice of a larger buffer may lie anywhere)."""
     s = scale2.reshape(-1).to(torch.float16).contiguous()
@@ -375,6 +384,10 @@ class FusedProjections:
         if rc:
             _lib.check("cobalt_gemv_fused" if M <= GEMV_MAX_TOKENS else "cobalt_gemm_fused", rc)
         return ys if flat else [y.reshape(*x.shape[:-1], m.out_features) for y, m in zip(ys, self.mods)]
+
+    def device_status(self) -> int:
+        """Status word of the launches of this object (0 = healthy); its modules' own words do not see them."""
+        return status_word(self._scratch)
 
     def staged(self, kind: int, a: torch.Tensor, b: Optional[torch.Tensor], flavor: int, w: Optional[torch.Tensor] = None,
                w_branch: Optional[torch.Tensor] = None, h_out: Optional[torch.Tensor] = None, eps: float = 0.0,

@@ -97,8 +97,10 @@ def test_infinite_column_scale_leaves_pruned_positions_alone(M):
 def test_fused_launch(M):
     mods = [module(K, 1024, 4, seed=i) for i, K in enumerate((512, 128, 200))]
     x = tokens(M, 1024)
-    for m, y in zip(mods, FusedProjections(mods)(x)):
+    fused = FusedProjections(mods)
+    for m, y in zip(mods, fused(x)):
         check(m, x, y)
+    assert fused._scratch is not None and fused.device_status() == 0        # the launch's own word: the modules were not called
 
 
 @pytest.mark.parametrize("K,N,bits", [(64, 512, 4), (80, 1152, 4), (512, 2048, 3), (48, 640, 2), (2400, 1536, 4)])

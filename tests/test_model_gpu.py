@@ -18,7 +18,8 @@ import pytest
 import torch
 
 from cobalt_b200 import CobaltSparseLinear, SparseQuantConfig
-from cobalt_b200.decoder import CobaltDecoder, compress_head, random_dense_params, random_raw_layer
+from cobalt_b200._lib import CobaltError
+from cobalt_b200.decoder import CobaltDecoder, build_random_decoder, compress_head, random_dense_params, random_raw_layer
 from oracle import cobalt_oracle as O
 from oracle import model_oracle as MO
 
@@ -239,4 +240,25 @@ def test_config3_full_7b_shape():
     g = torch.Generator().manual_seed(2048)
     prompt = torch.randint(0, cfg["vocab_size"], (2048,), generator=g)
     compare(dec, W, cfg, prompt, 256, "cuda")
-    assert max(m.device_status() for m in dec.lin.values()) == 0
+    assert dec.device_status() == 0
+
+
+def test_a_wait_that_gave_up_is_reported():
+    """The status words of every launch of a decoder reach its device_status(), and generate() does not return tokens of a prompt
+    whose attention is incomplete.  (The words are set by hand: no wait is made to run out.)"""
+    cfg = MO.llama_config(hidden=256, layers=1, heads=4, kv_heads=2, head_dim=64, inter=512, vocab=512)
+    dec = build_random_decoder(cfg, SparseQuantConfig(4, 0.5, 0.5), 64, torch.device("cuda"), batch=2, head_bits=4)
+    prompt = torch.randint(0, 512, (2, 20), generator=torch.Generator().manual_seed(1))
+    want, _ = dec.generate(prompt, 4)
+    assert dec.device_status() == 0
+    for fused in (dec.qkv[0], dec.gate_up[0], dec.o_f[0], dec.down[0], dec.head_f):
+        at = (-fused._scratch.data_ptr()) % 256
+        fused._scratch[at] = 5
+        assert fused.device_status() == 5 and dec.device_status() == 5
+        fused._scratch[at] = 0
+    assert dec.device_status() == 0
+    dec.prompt_status.fill_(4)
+    assert dec.device_status() == 4
+    with pytest.raises(CobaltError):
+        dec.generate(prompt, 4)
+    assert torch.equal(dec.generate(prompt, 4)[0], want) and dec.device_status() == 0

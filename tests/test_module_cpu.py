@@ -1,7 +1,12 @@
 """Host side of the module and of its launches: what needs no GPU."""
+from types import SimpleNamespace
+
+import pytest
 import torch
 
-from cobalt_b200 import CobaltSparseLinear
+from cobalt_b200 import CobaltSparseLinear, FusedProjections
+from cobalt_b200._lib import CobaltError
+from cobalt_b200.decoder import CobaltDecoder
 
 
 def small_module(scale2=None, K=16, N=256):
@@ -19,3 +24,26 @@ def test_column_scale_is_kept_where_vector_loads_can_read_it():
         assert torch.equal(m.scale2, scale2.reshape(-1))
         state = m.state_dict()
         assert CobaltSparseLinear.from_state_dict(dict(state, scale2=scale2), device="cpu").scale2.data_ptr() % 16 == 0
+
+
+def test_status_words_of_fused_launches_and_decoders():
+    """A code that a kernel left in the scratch of a fused launch, or for a prompt's attention, is reported."""
+    fused = [FusedProjections([small_module()]) for _ in range(5)]
+    assert [f.device_status() for f in fused] == [0] * 5
+    for f in fused:
+        f._scratch = torch.zeros(1024, dtype=torch.uint8)
+    word = torch.zeros(1, dtype=torch.int32)
+    dec = SimpleNamespace(lin={0: small_module()}, prompt_status=word, att_fused=None, qkv=fused[:1], gate_up=fused[1:2], o_f=fused[2:3],
+                          down=fused[3:4], head=small_module(), head_f=fused[4], reducer=None)
+    assert CobaltDecoder.device_status(dec) == 0
+    for f in fused:
+        at = (-f._scratch.data_ptr()) % 256                 # the kernels' status word: the first aligned byte
+        f._scratch[at] = 3
+        assert f.device_status() == 3 and CobaltDecoder.device_status(dec) == 3
+        f._scratch[at] = 0
+    CobaltDecoder._check_prompt_attention(dec)
+    word.fill_(5)
+    assert CobaltDecoder.device_status(dec) == 5
+    with pytest.raises(CobaltError, match="prompt"):
+        CobaltDecoder._check_prompt_attention(dec)
+    assert int(word) == 0
