@@ -347,9 +347,7 @@ class CobaltDecoder:
         cfg, P = self.cfg, self.P
         nh, nkv, D = self.nh, self.nkv, cfg["head_dim"]                                # heads of this rank
         T, rep, S = ids.shape[0], nh // nkv, attend_len
-        h = P["model.embed_tokens.weight"].index_select(0, ids)                        # [T, H]
-        if self.gemma:
-            h = h * self.embed_scale                                                   # scale rounded to bf16 first
+        h = self._embed(ids)                                                           # [T, H]
         blocked, allowed_of = {}, {}
         if seq is not None and (self.fused_prompt_attention or not self.prompt_kernel) and (T > 1 or self.att_scratch is None):
             causal = self.kv_pos[None, :S] <= positions[:, None]                       # [T, S]
@@ -412,11 +410,27 @@ class CobaltDecoder:
             delta = self._glu_down(i, g, u)
             if self.gemma:
                 delta_w = P[p + "post_feedforward_layernorm.weight"]
+        return self._logits_of(h, delta, delta_w).unsqueeze(0)                              # [1, T, V]
+
+    def _logits_of(self, h, delta, delta_w):
+        """What follows the last block: the branch joins, final norm, head; ``[T, V]``."""
+        w = self.P["model.norm.weight"]
         if self.head_f is not None and self.world == 1:                                # final norm folded into the compressed head
-            h, (lg,) = self._norm_then(self.head_f, h, delta, P["model.norm.weight"], delta_w)
-            return lg.unsqueeze(0)
-        h, x = self._add_rmsnorm(h, self._settled(delta), P["model.norm.weight"], delta_w)
-        return self._head_logits(x).unsqueeze(0)                                            # [1, T, V]
+            return self._norm_then(self.head_f, h, delta, w, delta_w)[1][0]
+        return self._head_logits(self._add_rmsnorm(h, self._settled(delta), w, delta_w)[1])
+
+    def _embed(self, ids: torch.Tensor) -> torch.Tensor:
+        h = self.P["model.embed_tokens.weight"].index_select(0, ids)                   # [T, H]
+        return h * self.embed_scale if self.gemma else h                               # scale rounded to bf16 first
+
+    def _greedy(self, rows: torch.Tensor, out: torch.Tensor):
+        """``out [B]`` = the greedy token of every row of logits."""
+        if rows.dtype == torch.bfloat16 and rows.stride(-1) == 1:
+            rc = self._lib.cobalt_argmax(rows.data_ptr(), rows.stride(0), rows.shape[0], rows.shape[-1], out.data_ptr(),
+                                         torch.cuda.current_stream(self.dev).cuda_stream)
+            _lib.check("cobalt_argmax", rc)
+        else:
+            out.copy_(torch.argmax(rows.float(), dim=-1))
 
     def device_status(self) -> int:
         """The worst status word of everything this decoder launches (0 = healthy): modules, fused launches, prompt and one-kernel
@@ -438,18 +452,29 @@ class CobaltDecoder:
 
     @torch.no_grad()
     def time_head_ms(self, reps: int = 20) -> float:
-        """Device time of what a decode step spends outside the blocks: embedding lookup, final norm, head, argmax."""
-        def once():
-            h = self.P["model.embed_tokens.weight"].index_select(0, self.tok)
-            _, y = self._add_rmsnorm(h, None, self.P["model.norm.weight"])
-            return torch.argmax(self._head_logits(y).float(), dim=-1)
+        """Device time of what a decode step spends outside the blocks - embedding lookup, the last branch joining, final norm,
+        head, greedy token: the code that ``step()`` runs, inside a graph as there."""
+        tok, P = torch.empty_like(self.tok), self.P
+        last = f"model.layers.{self.cfg['num_hidden_layers'] - 1}."
 
-        for _ in range(3):
+        def once():
+            h = self._embed(self.tok)
+            self._greedy(self._logits_of(h, h, P[last + "post_feedforward_layernorm.weight"] if self.gemma else None), tok)
+
+        s = torch.cuda.Stream(self.dev)
+        s.wait_stream(torch.cuda.current_stream(self.dev))
+        with torch.cuda.stream(s):
             once()
+        torch.cuda.current_stream(self.dev).wait_stream(s)
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            once()
+        for _ in range(3):
+            graph.replay()
         e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
         e0.record()
         for _ in range(reps):
-            once()
+            graph.replay()
         e1.record()
         torch.cuda.synchronize()
         return e0.elapsed_time(e1) / reps
@@ -467,9 +492,7 @@ class CobaltDecoder:
         """``ids [n, T]``: the prompts of sequences ``first`` .. ``first + n - 1`` at the same ``positions [T]``; logits ``[n, T, V]``."""
         cfg, P = self.cfg, self.P
         n, T = ids.shape
-        h = P["model.embed_tokens.weight"].index_select(0, ids.reshape(-1))            # [n*T, H]
-        if self.gemma:
-            h = h * self.embed_scale
+        h = self._embed(ids.reshape(-1))                                               # [n*T, H]
         delta, delta_w = None, None
         for i in range(cfg["num_hidden_layers"]):
             p = f"model.layers.{i}."
@@ -522,12 +545,7 @@ class CobaltDecoder:
         """One decode step for the tokens in ``self.tok`` at ``self.pos`` (one per sequence); returns the logits
         (``[V]`` for a single sequence, else ``[B, V]``) and advances ``tok`` (greedy) and ``pos`` on the device."""
         rows = self._forward(self.tok, self.pos, self.max_ctx, seq=0 if self.B == 1 else None)[0]        # [B, V]
-        if rows.dtype == torch.bfloat16 and rows.stride(-1) == 1:
-            rc = self._lib.cobalt_argmax(rows.data_ptr(), rows.stride(0), self.B, rows.shape[-1], self.tok.data_ptr(),
-                                         torch.cuda.current_stream(self.dev).cuda_stream)
-            _lib.check("cobalt_argmax", rc)
-        else:
-            self.tok.copy_(torch.argmax(rows.float(), dim=-1))
+        self._greedy(rows, self.tok)
         self.pos.add_(1)
         return rows[0] if self.B == 1 else rows
 

@@ -262,3 +262,21 @@ def test_a_wait_that_gave_up_is_reported():
     with pytest.raises(CobaltError):
         dec.generate(prompt, 4)
     assert torch.equal(dec.generate(prompt, 4)[0], want) and dec.device_status() == 0
+
+
+@pytest.mark.parametrize("head_bits", [0, 4])
+def test_time_outside_the_blocks_is_that_of_the_step(head_bits, monkeypatch):
+    """time_head_ms() runs the same launches as step() after its last block, and leaves the decoder's tokens alone."""
+    cfg = MO.llama_config(hidden=256, layers=1, heads=4, kv_heads=2, head_dim=64, inter=512, vocab=512)
+    dec = build_random_decoder(cfg, SparseQuantConfig(4, 0.5, 0.5), 64, torch.device("cuda"), head_bits=head_bits)
+    dec.generate(torch.arange(20), 3)
+    seen = []
+    for name in ("_logits_of", "_greedy", "_embed"):
+        inner = getattr(dec, name)
+        monkeypatch.setattr(dec, name, lambda *a, _n=name, _f=inner: (seen.append(_n), _f(*a))[1])
+    tok, pos = dec.tok.clone(), dec.pos.clone()
+    assert dec.time_head_ms(2) > 0
+    assert torch.equal(dec.tok, tok) and torch.equal(dec.pos, pos)
+    timed, seen[:] = seen[:3], []
+    dec.step()
+    assert timed == seen == ["_embed", "_logits_of", "_greedy"]
