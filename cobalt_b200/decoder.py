@@ -30,7 +30,7 @@ import torch.nn.functional as F
 
 from .compress import SparseQuantConfig, compress_weight
 from . import _lib
-from .linear import CobaltSparseLinear, FusedProjections, status_word
+from .linear import CobaltSparseLinear, FusedProjections, called_plainly, status_word
 
 PROJ = ("self_attn.q_proj", "self_attn.k_proj", "self_attn.v_proj", "self_attn.o_proj",
         "mlp.gate_proj", "mlp.up_proj", "mlp.down_proj")
@@ -482,9 +482,11 @@ class CobaltDecoder:
     def _prompts_at_once(self, T: int) -> int:
         """How many sequences' prompts of ``T`` tokens run through the layers together: weights are expanded once for all of them.
         Every row's sums are added as if its sequence ran alone (``sum_tokens``), so the logits do not depend on it.  Up to 8192 rows
-        (activations of a few GB at the widest MLPs); prompts that the decode GEMV takes, tensor parallelism and head
-        widths without the prompt kernel run one by one."""
-        if self.world > 1 or T <= 16 or not self.prompt_kernel or self.fused_prompt_attention:
+        (activations of a few GB at the widest MLPs); prompts that the decode GEMV takes, tensor parallelism, head widths
+        without the prompt kernel and modules whose call runs more than their kernel go one by one."""
+        if self.world > 1 or T <= 16 or not self.prompt_kernel or self.fused_prompt_attention or self.B == 1:
+            return 1
+        if not all(called_plainly(m) for m in list(self.lin.values()) + ([self.head] if self.head is not None else [])):
             return 1
         return max(1, min(self.B, 8192 // T))
 

@@ -322,6 +322,14 @@ class CobaltSparseLinear(nn.Module):
                 f"group_size={GROUP}, density={dens:.3f}, bias={self.bias is not None}")
 
 
+def called_plainly(m: nn.Module) -> bool:
+    """Whether calling ``m`` runs ``CobaltSparseLinear.forward`` and nothing else: no hooks (its own or for all modules), no ``forward``
+    put on the instance (offloading wrappers do that) or on a subclass.  Only then may a launch stand in for the call."""
+    return (type(m).forward is CobaltSparseLinear.forward and type(m).__call__ is nn.Module.__call__ and "forward" not in m.__dict__
+            and m._compiled_call_impl is None and not (m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks)
+            and not torch.nn.modules.module._has_any_global_hook())
+
+
 class FusedProjections:
     """Several ``CobaltSparseLinear`` that read the same activations (q|k|v, gate|up), evaluated with one
     launch: the decode GEMV for up to 16 tokens (``cobalt_gemv_fused``), the tcgen05 GEMM above that
@@ -365,8 +373,8 @@ class FusedProjections:
         flat = x.dim() == 2 and x.shape[1] == N
         x2 = x if flat else x.reshape(-1, N)
         M = x2.shape[0]
-        if M == 0 or (M > GEMV_MAX_TOKENS and any(m._forward_hooks or m._forward_pre_hooks for m in self.mods)):
-            return [m(x) for m in self.mods]                 # a prompt runs the hooks of its modules
+        if M == 0 or (M > GEMV_MAX_TOKENS and not all(called_plainly(m) for m in self.mods)):
+            return [m(x) for m in self.mods]                 # a prompt runs whatever a call of its modules runs
         if not x2.is_cuda or x2.dtype != torch.bfloat16:
             if M > GEMV_MAX_TOKENS:
                 return [m(x) for m in self.mods]             # raises what a module raises

@@ -103,6 +103,39 @@ def test_fused_launch(M):
     assert fused._scratch is not None and fused.device_status() == 0        # the launch's own word: the modules were not called
 
 
+@pytest.mark.parametrize("how", ["hook", "global hook", "replaced", "subclass"])
+def test_fused_launch_does_not_pass_a_module_by(how):
+    """Above 16 tokens whatever a call of a module runs is run, as before there was a launch for several modules."""
+    class Sub(CobaltSparseLinear):
+        def forward(self, x):
+            seen.append(x.shape[0])
+            return super().forward(x)
+
+    seen = []
+    mods = [module(128, 640, 4, seed=i) for i in range(2)]
+    fused, x = FusedProjections(mods), tokens(40, 640)
+    want = fused(x)
+    assert not seen
+    note, handle = lambda m, args, *out: seen.append(args[0].shape[0]), None
+    if how == "hook":
+        handle = mods[1].register_forward_hook(note)
+    elif how == "global hook":
+        handle = torch.nn.modules.module.register_module_forward_pre_hook(note)
+    elif how == "replaced":
+        inner = mods[1].forward
+        mods[1].forward = lambda x: (seen.append(x.shape[0]), inner(x))[1]
+    else:
+        mods[1].__class__ = Sub
+    try:
+        got = fused(x)
+    finally:
+        if handle is not None:
+            handle.remove()
+    assert seen == [40] * (2 if how == "global hook" else 1)
+    for a, b in zip(got, want):
+        assert float((a.double() - b.double()).norm() / b.double().norm()) <= 2.0 ** -8
+
+
 @pytest.mark.parametrize("K,N,bits", [(64, 512, 4), (80, 1152, 4), (512, 2048, 3), (48, 640, 2), (2400, 1536, 4)])
 @pytest.mark.parametrize("M", [1, 5, 8, 16])
 def test_matrix_without_pruned_positions(K, N, bits, M):

@@ -7,6 +7,7 @@ import torch
 from cobalt_b200 import CobaltSparseLinear, FusedProjections
 from cobalt_b200._lib import CobaltError
 from cobalt_b200.decoder import CobaltDecoder
+from cobalt_b200.linear import called_plainly
 
 
 def small_module(scale2=None, K=16, N=256):
@@ -47,3 +48,28 @@ def test_status_words_of_fused_launches_and_decoders():
     with pytest.raises(CobaltError, match="prompt"):
         CobaltDecoder._check_prompt_attention(dec)
     assert int(word) == 0
+
+
+def test_modules_whose_call_runs_more_than_their_kernel():
+    """Hooks, replaced and overridden forwards: a fused launch must not stand in for the call."""
+    class Sub(CobaltSparseLinear):
+        def forward(self, x):
+            return super().forward(x)
+
+    plain = small_module()
+    assert called_plainly(plain)
+    sub = small_module()
+    sub.__class__ = Sub
+    replaced = small_module()
+    replaced.forward = lambda x: x
+    compiled = small_module()
+    compiled._compiled_call_impl = lambda x: x
+    assert not any(called_plainly(m) for m in (sub, replaced, compiled))
+    noop = lambda *a: None
+    for register in (plain.register_forward_hook, plain.register_forward_pre_hook, plain.register_full_backward_hook,
+                     plain.register_full_backward_pre_hook, torch.nn.modules.module.register_module_forward_hook,
+                     torch.nn.modules.module.register_module_forward_pre_hook):
+        handle = register(noop)
+        assert not called_plainly(plain)
+        handle.remove()
+        assert called_plainly(plain)

@@ -114,3 +114,18 @@ def test_prompts_together_equal_prompts_alone(family, batch, T):
         assert torch.equal(dec._forward(ids[b].cuda(), pos, T, seq=b)[0], together[b]), b
     assert torch.equal(dec.k_cache, kc) and torch.equal(dec.v_cache, vc)
     assert int(dec.prompt_status) == 0
+
+
+def test_prompts_of_watched_modules_run_one_by_one():
+    """A hook on o or down sees every prompt by itself, in the order of the sequences, also where prompts could run together."""
+    from cobalt_b200 import SparseQuantConfig
+    from cobalt_b200.decoder import build_random_decoder
+    from oracle import model_oracle as MO
+    cfg = MO.llama_config(hidden=512, layers=2, heads=8, kv_heads=2, head_dim=64, inter=1024, vocab=1008)
+    dec = build_random_decoder(cfg, SparseQuantConfig(4, 0.5, 0.5), 48, torch.device("cuda"), batch=3, head_bits=4)
+    ids = torch.randint(0, 1000, (3, 40), generator=torch.Generator().manual_seed(1))
+    want, seen = dec.prefill(ids), []
+    handle = dec.lin[(1, "mlp.down_proj")].register_forward_hook(lambda m, args, out: seen.append(tuple(args[0].shape)))
+    assert torch.equal(dec.prefill(ids), want) and seen == [(40, 1024)] * 3
+    handle.remove()
+    assert torch.equal(dec.prefill(ids), want) and len(seen) == 3
