@@ -87,10 +87,26 @@ __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
         : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
     return ok != 0;
 }
-// Wait with an iteration limit: returns false (and records `code`) instead of spinning forever.
+// The same for arrivals of other CTAs of the cluster.  Relaxed: enough for completions of tcgen05.commit; what threads of another CTA
+// released is visible after a cluster_acquire()
+__device__ __forceinline__ bool mbar_try_wait_cluster(uint32_t bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.relaxed.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.b32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+    return ok != 0;
+}
+__device__ __forceinline__ void cluster_acquire() {        // of shared memory only; an acquire of all memory costs many times as much
+    asm volatile("fence.acquire.sync_restrict::shared::cluster.cluster;" ::: "memory");
+}
+// Wait with an iteration limit: returns false (and records `code`) instead of spinning forever.  CLUSTER: other CTAs of the
+// cluster, or asynchronous operations of theirs, arrive on this barrier too - the unqualified form orders one CTA only.
+template <bool CLUSTER = false>
 __device__ __forceinline__ bool mbar_wait_bounded(uint32_t bar, uint32_t parity, uint32_t* status, uint32_t code) {
     for (uint32_t it = 0; it < (1u << 18); ++it) {
-        if (mbar_try_wait(bar, parity)) return true;
+        if (CLUSTER ? mbar_try_wait_cluster(bar, parity) : mbar_try_wait(bar, parity)) return true;
         if (it > 64) __nanosleep(128);
     }
     if (status) atomicCAS(status, 0u, code);

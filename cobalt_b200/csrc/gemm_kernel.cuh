@@ -29,8 +29,13 @@
 // 2048 tokens 232 -> 172 us (1.40 PFLOP/s); 4096 x 4096, 2048 tokens 91 -> 68 us; 14336 x 4096, 2048 tokens 317 -> 238 us;
 // 4096 x 4096, 100 tokens 33 -> 26 us; q|k|v of a 7B block (one launch instead of three), 2048 tokens 241 -> 123 us.
 //
-// Generic-proxy writes to A stages are published with fence.proxy.async before the mbarrier arrive.  Every wait on an
-// mbarrier is bounded: on expiry the kernel records a status code, stops issuing work, frees its tensor memory and returns.
+// Generic-proxy writes to A stages are published with fence.proxy.async before the mbarrier arrive.  In a pair the second CTA's half
+// of A is read by MMAs that the first CTA issues: its decode warps release and the issuing warp acquires at cluster scope (an
+// unqualified arrive or wait orders the threads of one CTA only), by the fences that cover shared memory alone: 4096 x
+// 14336, 2048 tokens 169 -> 170.5 us.  release.cluster / acquire.cluster on the barrier operations themselves cover all memory, the
+// decode warps' loads in flight with it, and cost 80 us at 4096 x 4096; the acquire after every wait of a pair cost 3.6 %
+// and is not needed for completions of tcgen05.commit.  Every wait on an mbarrier is bounded: on expiry the kernel records a
+// status code, stops issuing work, frees its tensor memory and returns.
 //
 // Behaviour replaced: cbk::gemm_tile (mma.sync m16n8k16, per-fragment bf16x2 dequantisation,
 // src/cobaltkernel/csrc/cobalt_gemm.cuh:243-609) driven by gemm_phase
@@ -144,8 +149,10 @@ __device__ __forceinline__ float4 ld_cluster_f4(uint32_t addr) {
     asm volatile("ld.shared::cluster.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr) : "memory");
     return v;
 }
+// arrival on a barrier of another CTA of the cluster; releases this thread's (and, after a __syncwarp, its warp's) writes to the shared
+// memory of its own CTA
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
-    asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
+    asm volatile("fence.release.sync_restrict::shared::cta.cluster;\n\tmbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }
 __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&v)[32]) {
     asm volatile(
@@ -395,7 +402,7 @@ __global__ void __launch_bounds__(gemm_threads(PAIR), PAIR ? 1 : 2) gemm_tcgen05
                 words[4 * i + 2] = cur.chunk[i].z; words[4 * i + 3] = cur.chunk[i].w;
             }
             const uint32_t bit1 = cur.bit + (uint32_t)__popc(cur.mask[0]) * (uint32_t)BITS;
-            healthy = __all_sync(full_mask, mbar_wait_bounded(bar_aempty(s), ph ^ 1u, P.status, DEV_TIMEOUT_EMPTY));
+            healthy = __all_sync(full_mask, mbar_wait_bounded<PAIR>(bar_aempty(s), ph ^ 1u, P.status, DEV_TIMEOUT_EMPTY));
             if (!healthy) break;
             const uint32_t dst = rowaddr + s * GEMM_A_BYTES;
             const int col = g * GROUP + (int)half * 64;
@@ -453,14 +460,14 @@ __global__ void __launch_bounds__(gemm_threads(PAIR), PAIR ? 1 : 2) gemm_tcgen05
             if (s >= (uint32_t)P.a_stages) { s -= (uint32_t)P.a_stages; ph ^= 1u; }
             cur = nxt;
         }
-        if (healthy) healthy = __all_sync(full_mask, mbar_wait_bounded(bar_acc, 0u, P.status, DEV_TIMEOUT_ACC));
+        if (healthy) healthy = __all_sync(full_mask, mbar_wait_bounded<PAIR>(bar_acc, 0u, P.status, DEV_TIMEOUT_ACC));
     } else if (warp == DW) {
         // =========================================================== activation loader (TMA)
         bool good = true;
         const uint32_t bytes = P.b_acc_bytes * (n_acc1 > 0 ? 2u : 1u);
         uint32_t s = 0, ph = 0;
         for (uint32_t q = 0; q < (uint32_t)my_stages; ++q) {
-            good = mbar_wait_bounded(bar_bempty(s), ph ^ 1u, P.status, DEV_TIMEOUT_EMPTY);
+            good = mbar_wait_bounded<PAIR>(bar_bempty(s), ph ^ 1u, P.status, DEV_TIMEOUT_EMPTY);
             if (!__all_sync(full_mask, good)) break;
             const int col = g_begin * GROUP + (int)q * GEMM_KS;
             // pair: each CTA loads its half of every accumulator's tokens; both count on the leader's barrier
@@ -483,10 +490,11 @@ __global__ void __launch_bounds__(gemm_threads(PAIR), PAIR ? 1 : 2) gemm_tcgen05
             bool good = true;
             uint32_t sa = 0, pa = 0, sb = 0, pb = 0;
             for (uint32_t q = 0; q < (uint32_t)my_stages; ++q) {
-                good = mbar_wait_bounded(bar_bfull(sb), pb, P.status, DEV_TIMEOUT_STAGE);
-                if (good) good = mbar_wait_bounded(bar_afull(sa), pa, P.status, DEV_TIMEOUT_FULL);
+                good = mbar_wait_bounded<PAIR>(bar_bfull(sb), pb, P.status, DEV_TIMEOUT_STAGE);
+                if (good) good = mbar_wait_bounded<PAIR>(bar_afull(sa), pa, P.status, DEV_TIMEOUT_FULL);
                 good = __all_sync(full_mask, good);
                 if (!good) break;
+                if (PAIR) cluster_acquire();                            // the other CTA's half of A (and of B)
                 tc_fence_after();
                 const uint64_t ad = umma_smem_desc(a_base + sa * GEMM_A_BYTES);
                 const uint64_t bd0 = umma_smem_desc(b_base + sb * P.b_stage_bytes);

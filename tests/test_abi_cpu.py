@@ -107,3 +107,14 @@ def test_scoring_refuses_what_32_bit_counts_cannot_hold(lib):
         assert lib.cobalt_score_rows(4096, 0, 4096, K, N, 1, 0, 5, 4096, None, 4096, None) == -6
         assert lib.cobalt_keep_from_scores(4096, None, K, N, 0, 0, 4096, 4096, None) == -6
     assert lib.cobalt_score_rows(4096, 0, 4096, 16, 128, 1, 0, 2049, 4096, None, 4096, None) == -1
+
+
+def test_arrivals_on_other_ctas_name_the_cluster_scope():
+    """An mbarrier arrive without a scope orders the threads of one CTA; one that goes to another CTA's barrier has to say more."""
+    csrc = os.path.join(ROOT, "cobalt_b200", "csrc")
+    found = []
+    for name in sorted(os.listdir(csrc)):
+        for line in open(os.path.join(csrc, name)):
+            found += re.findall(r"mbarrier\.arrive[.\w:]*shared::cluster[.\w:]*", line.replace("tcgen05.commit", ""))
+    found = [f for f in found if "::arrive::one" not in f]
+    assert found and all(re.match(r"mbarrier\.arrive\.(expect_tx\.)?(relaxed|release)\.cluster\.", f) for f in found), found
