@@ -156,6 +156,9 @@ class CobaltDecoder:
             and max_ctx <= 65536 else None
         # Prompts take the library's tcgen05 attention (128 / 64 wide heads), other head widths batched matmuls
         self.prompt_kernel = D in (64, 128) and self.nh // self.nkv <= 128 and max_ctx <= 1 << 24
+        # Rows (tokens of all prompts) that go through the layers together when several sequences are prefilled: the activations of
+        # 8192 are a GB or more at the widest MLPs.  The caller may lower it; 0 = one prompt at a time.
+        self.prompt_rows = 8192
         self.prompt_status = torch.zeros(1, dtype=torch.int32, device=device)          # non-zero: a bounded wait gave up
         # One-kernel attention (cooperative launch; its scratch starts zeroed; only while its whole grid fits on the GPU).
         # Off by default: bit-identical to the three kernels but slower inside the decode graph (4-layer 7B-shaped step
@@ -481,14 +484,14 @@ class CobaltDecoder:
 
     def _prompts_at_once(self, T: int) -> int:
         """How many sequences' prompts of ``T`` tokens run through the layers together: weights are expanded once for all of them.
-        Every row's sums are added as if its sequence ran alone (``sum_tokens``), so the logits do not depend on it.  Up to 8192 rows
-        (activations of a few GB at the widest MLPs); prompts that the decode GEMV takes, tensor parallelism, head widths
-        without the prompt kernel and modules whose call runs more than their kernel go one by one."""
+        Every row's sums are added as if its sequence ran alone (``sum_tokens``), so the logits do not depend on it.  Up to
+        ``prompt_rows`` rows; prompts that the decode GEMV takes, tensor parallelism, head widths without the prompt kernel
+        and modules whose call runs more than their kernel go one by one."""
         if self.world > 1 or T <= 16 or not self.prompt_kernel or self.fused_prompt_attention or self.B == 1:
             return 1
         if not all(called_plainly(m) for m in list(self.lin.values()) + ([self.head] if self.head is not None else [])):
             return 1
-        return max(1, min(self.B, 8192 // T))
+        return max(1, min(self.B, self.prompt_rows // T))
 
     def _forward_prompts(self, ids: torch.Tensor, positions: torch.Tensor, first: int) -> torch.Tensor:
         """``ids [n, T]``: the prompts of sequences ``first`` .. ``first + n - 1`` at the same ``positions [T]``; logits ``[n, T, V]``."""
@@ -533,10 +536,14 @@ class CobaltDecoder:
         self._check_room(T)
         pos = torch.arange(T, device=self.dev)
         n, at_once = ids2.shape[0], self._prompts_at_once(T)
+        logits = None
         if at_once > 1 and n > 1:
-            parts = [self._forward_prompts(ids2[b:b + at_once], pos, b) for b in range(0, n, at_once)]
-            logits = parts[0] if len(parts) == 1 else torch.cat(parts)
-        else:
+            try:
+                parts = [self._forward_prompts(ids2[b:b + at_once], pos, b) for b in range(0, n, at_once)]
+                logits = parts[0] if len(parts) == 1 else torch.cat(parts)
+            except torch.cuda.OutOfMemoryError:              # one at a time needs less, and writes the same bits over what is in the caches
+                parts = None
+        if logits is None:
             parts = [self._forward(ids2[b], pos, T, seq=b) for b in range(n)]              # [1, T, V] each
             logits = parts[0] if n == 1 else torch.cat(parts)
         self.pos.fill_(T)

@@ -73,3 +73,18 @@ def test_modules_whose_call_runs_more_than_their_kernel():
         assert not called_plainly(plain)
         handle.remove()
         assert called_plainly(plain)
+
+
+def test_how_many_prompts_run_together():
+    """As many as fit the rows that the caller allows; one by one where it says so, and where a module's call runs more than its kernel."""
+    dec = SimpleNamespace(world=1, prompt_kernel=True, fused_prompt_attention=False, B=8, prompt_rows=8192, lin={0: small_module()}, head=None)
+    at_once = lambda T: CobaltDecoder._prompts_at_once(dec, T)
+    assert [at_once(T) for T in (16, 17, 1000, 1024, 1025, 4096, 4097, 20000)] == [1, 8, 8, 8, 7, 2, 1, 1]
+    dec.prompt_rows = 400
+    assert [at_once(T) for T in (100, 133, 201)] == [4, 3, 1]
+    dec.prompt_rows = 0
+    assert at_once(100) == 1
+    dec.prompt_rows = 8192
+    dec.head = small_module()
+    dec.head.register_forward_hook(lambda *a: None)
+    assert at_once(100) == 1

@@ -129,3 +129,31 @@ def test_prompts_of_watched_modules_run_one_by_one():
     assert torch.equal(dec.prefill(ids), want) and seen == [(40, 1024)] * 3
     handle.remove()
     assert torch.equal(dec.prefill(ids), want) and len(seen) == 3
+
+
+def test_prompts_together_give_way_to_memory(monkeypatch):
+    """Where the activations of all prompts at once do not fit, or the caller wants less, the prompts run in smaller parts: same bits."""
+    from cobalt_b200 import SparseQuantConfig
+    from cobalt_b200.decoder import build_random_decoder
+    from oracle import model_oracle as MO
+    cfg = MO.llama_config(hidden=512, layers=2, heads=8, kv_heads=2, head_dim=64, inter=1024, vocab=1008)
+    dec = build_random_decoder(cfg, SparseQuantConfig(4, 0.5, 0.5), 48, torch.device("cuda"), batch=5, head_bits=4)
+    ids = torch.randint(0, 1000, (5, 40), generator=torch.Generator().manual_seed(1))
+    want = dec.prefill(ids)
+    caches = dec.k_cache.clone(), dec.v_cache.clone()
+    parts, inner = [], dec._forward_prompts
+
+    def forward_prompts(ids, positions, first):
+        parts.append(ids.shape[0])
+        if dec.prompt_rows == 199:                            # no allocation is made to fail: the error alone matters
+            raise torch.cuda.OutOfMemoryError("no room")
+        return inner(ids, positions, first)
+
+    monkeypatch.setattr(dec, "_forward_prompts", forward_prompts)
+    for rows, expect in ((8192, [5]), (100, [2, 2, 1]), (0, []), (199, [4])):
+        dec.prompt_rows = rows
+        dec.k_cache.zero_()
+        dec.v_cache.zero_()
+        del parts[:]
+        assert torch.equal(dec.prefill(ids), want) and parts == expect
+        assert torch.equal(dec.k_cache, caches[0]) and torch.equal(dec.v_cache, caches[1])
