@@ -359,7 +359,13 @@ int launch_prompt_attn(const PromptAttnParams& P, dim3 grid, const CUtensorMap& 
     return cudaGetLastError() == cudaSuccess ? COBALT_OK : COBALT_ELAUNCH;
 }
 
-constexpr int ROPE_MIN_ROWS = 32;
+// Rotation with a block per token, against a thread per value (a warp per head with the norm).  A block costs about 0.7 us at least,
+// and pays once the values (tokens x (query + KV heads) x width) are many: 32 / 8 heads of 128, 48 tokens 3.2 us against 3.0, 64 tokens
+// 3.2 / 3.4, 2048 tokens 10 / 47; 4 / 1 heads of 128, 384 tokens 2.8 / 2.9; 16 / 4 heads of 64, 192 tokens 2.8 / 2.9.  With the norm
+// the heads of a token follow each other, eight at a time: 256 tokens equal at 32 / 16, 16 / 8 (heads of 128) and 8 / 4 (256),
+// 192 tokens of 32 / 16 heads 8.4 / 6.6, 384 tokens 9.9 / 11.1, 2048 tokens 33 / 47; heads of 64 never gained.
+constexpr long long ROPE_ROWS_MIN_VALUES = 1 << 18;
+constexpr int ROPE_NORM_ROWS_MIN_TOKENS = 288, ROPE_NORM_ROWS_MIN_DIM = 128;
 constexpr long STAGED_NORM_MAX_VALUES = 8192, STAGED_GLU_MAX_VALUES = 32768;     // M * in_features a staged input may compute
 constexpr size_t SCRATCH_PUSH_DONE_OFF = 128;            // CTA arrival counter of pushing launches, inside the status block
 
@@ -888,8 +894,9 @@ int cobalt_rope_kv(void* q, const void* k, const void* v, const int64_t* positio
     int sms = 0;
     int rc = device_info(&sms);
     if (rc) return rc;
-    // a block per token once that fills a good part of the GPU; fewer tokens (a decode step) spread every head instead
-    const bool rows = T >= ROPE_MIN_ROWS && head_dim % 16 == 0 && head_dim <= 2 * ROPE_MAX_HALF && cache_seq_stride % 8 == 0 &&
+    const bool many = q_norm_w ? T >= ROPE_NORM_ROWS_MIN_TOKENS && head_dim >= ROPE_NORM_ROWS_MIN_DIM
+                               : (long long)T * (n_heads + n_kv_heads) * head_dim >= ROPE_ROWS_MIN_VALUES;
+    const bool rows = many && head_dim % 16 == 0 && head_dim <= 2 * ROPE_MAX_HALF && cache_seq_stride % 8 == 0 &&
                       !(((uintptr_t)q | (uintptr_t)k | (uintptr_t)v | (uintptr_t)k_cache | (uintptr_t)v_cache) & 15);
     if (rows) {
         if (q_norm_w)

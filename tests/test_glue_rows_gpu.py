@@ -15,15 +15,16 @@ def rand(*shape, seed=0, gain=1.0):
     return (torch.randn(*shape, generator=torch.Generator(device="cuda").manual_seed(seed + sum(shape)), device="cuda") * gain).bfloat16()
 
 
-# one block per token (32 tokens on) against the same tokens in calls of 16, which take the kernels that spread every head: same bits
-@pytest.mark.parametrize("T,nh,nkv,D", [(32, 8, 2, 128), (77, 6, 2, 64), (48, 4, 1, 256), (33, 3, 3, 16)])
+# one block per token (2^18 values on; with the norm 288 tokens and heads of 128 on) against the same tokens in calls of 16, which
+# take the kernels that spread every head: same bits.  The first four stay below the line, the others lie on or beyond it.
+@pytest.mark.parametrize("T,nh,nkv,D", [(32, 8, 2, 128), (77, 6, 2, 64), (48, 4, 1, 256), (33, 3, 3, 16), (288, 8, 2, 128), (300, 4, 1, 256),
+                                        (331, 5, 1, 144), (2731, 3, 3, 16), (700, 6, 2, 64)])
 @pytest.mark.parametrize("norm", [False, True])
 def test_rope_of_many_tokens_equals_few(T, nh, nkv, D, norm):
     lib, ctx = _lib.load(), T + 7
     k, v, pos = rand(T, nkv * D, seed=1), rand(T, nkv * D, seed=2), torch.arange(3, 3 + T, device="cuda")
     pos[5], pos[6] = -1, ctx                                     # outside the cache: not stored
     inv = 1.0 / (1e4 ** (torch.arange(0, D, 2, device="cuda").float() / D))
-    w = [rand(D, seed=s, gain=0.1).data_ptr() if norm else None for s in (3, 4)]
     keep = [rand(D, seed=s, gain=0.1) for s in (3, 4)]           # owns the norm weights
     w = [t.data_ptr() if norm else None for t in keep]
     res = []
