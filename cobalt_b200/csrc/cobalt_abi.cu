@@ -79,7 +79,7 @@ struct GemvCfg {
     int stages, mt, grid;
     bool xs;                           // activations staged in shared memory
     bool aligned;                      // every CTA holds whole row blocks
-    bool dense;                        // nothing pruned: tiles are copied row by row, 16 bytes apart
+    bool dense;                        // nothing pruned, 4 bit: tiles are copied row by row, 16 bytes apart
     uint32_t slot, xs_bytes, total_warps, part_q, part_r;
     size_t smem, counters_off, partials_off, xperm_off, total;
 };
@@ -98,8 +98,8 @@ GemvGeom geom_of(const CobaltMat* w) {
 int gemv_config(const GemvGeom& g, int N, int M, int num_sms, GemvCfg* c) {
     const int RB = g.RB, CT = g.CT;
     c->mt = M > 8 ? 2 : 1;
-    c->dense = g.dense;
-    c->slot = (uint32_t)round_up((size_t)g.max_tile_bytes + 32 + (g.dense ? TILE_ROWS * 16 : 0), 128);
+    c->dense = g.dense && g.bits == GEMV_DENSE_BITS;
+    c->slot = (uint32_t)round_up((size_t)g.max_tile_bytes + 32 + (c->dense ? TILE_ROWS * 16 : 0), 128);
     const size_t fixed = GEMV_LUT_BYTES + GEMV_BAR_BYTES + GEMV_REDCNT_BYTES + gemv_red_bytes(c->mt) + 64;
     // Two ring slots per warp keep one tile in flight behind the one being decoded.  The activations are staged in
     // shared memory when they fit beside such a ring (always for one token); what is left goes to deeper rings.
@@ -158,9 +158,11 @@ int launch_gemv(const GemvParams& P, const GemvCfg& c, cudaStream_t st) {
     const int kind = P.mode != 0 || odd_scale ? (c.dense ? 4 : 1) : P.col_scale != nullptr ? 2 : c.dense ? 3 : 0;
     void (*kernel)(const GemvParams) = kind == 1   ? gemv_mma_special_kernel<BITS, MT, XS>
                                        : kind == 2 ? gemv_mma_scaled_kernel<BITS, MT, XS>
-                                       : kind == 3 ? gemv_mma_dense_kernel<BITS, MT, XS>
-                                       : kind == 4 ? gemv_mma_dense_special_kernel<BITS, MT, XS>
                                                    : gemv_mma_kernel<BITS, MT, XS>;
+    if constexpr (BITS == GEMV_DENSE_BITS) {
+        if (kind == 3) kernel = gemv_mma_dense_kernel<BITS, MT, XS>;
+        if (kind == 4) kernel = gemv_mma_dense_special_kernel<BITS, MT, XS>;
+    }
     static bool configured[MAX_DEVICES][5];
     int dev = 0;
     cudaGetDevice(&dev);

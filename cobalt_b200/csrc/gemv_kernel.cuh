@@ -406,9 +406,12 @@ struct GemvUnit {
 // (GemvParams::mode != 0).  The common launch is a kernel of its own without any of that code, so that the
 // less common modes cost it neither a start-up test nor a register.  SCALED = the matrix has a column scale: its weights
 // are expanded like the others and finished in fp32 (decode8_scaled), a kernel of its own for the same reason.
-// DENSE = nothing is pruned (a compressed head).  Every row of a tile then has the same number of code bytes, a multiple of the 128
-// bytes of all banks at 4 bit: the code words of the 8 rows and 4 groups of a warp fall into two banks.  Full tiles are
-// copied row by row, 16 bytes apart, which spreads the rows over the banks: 32000 x 5376, 4 bit, 8 tokens 92 -> 56 us
+// DENSE = nothing is pruned (a compressed head), 4 bit.  Every row of a tile then has the same number of code bytes, a multiple of
+// the 128 bytes of all banks: the code words of the 8 rows and 4 groups of a warp fall into two banks.  Full tiles are
+// copied row by row, 16 bytes apart, which spreads the rows over the banks: 32000 x 5376, 8 tokens 92 -> 59 us.  At 3 bit (192
+// bytes a row) the sixteen copies cost more than the conflicts: 53.3 us whole, 59.9 row by row; at 2 bit they cost about as
+// much: 50.7 / 54.8, but 40.1 / 39.9 at 32000 x 4096.
+constexpr int GEMV_DENSE_BITS = 4;
 template <int BITS, int MT, bool XS, bool SPECIAL, bool SCALED, bool DENSE>
 __device__ __forceinline__ void gemv_mma_body(const GemvParams& P) {
     extern __shared__ __align__(1024) uint8_t smem[];
@@ -952,7 +955,7 @@ template <int BITS, int MT, bool XS>
 __global__ void __launch_bounds__(GEMV_THREADS, 1) gemv_mma_special_kernel(const __grid_constant__ GemvParams P) {
     gemv_mma_body<BITS, MT, XS, true, false, false>(P);
 }
-// matrices without pruned positions, plain and staged
+// matrices without pruned positions (GEMV_DENSE_BITS only), plain and staged
 template <int BITS, int MT, bool XS>
 __global__ void __launch_bounds__(GEMV_THREADS, 1) gemv_mma_dense_kernel(const GemvParams P) {
     gemv_mma_body<BITS, MT, XS, false, false, true>(P);
