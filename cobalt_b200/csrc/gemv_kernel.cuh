@@ -844,9 +844,11 @@ __device__ __forceinline__ void gemv_mma_body(const GemvParams& P) {
 
             // one word (two units) of both rows; `cur` arrives requested, the first unit of the next word leaves requested
             auto do_word = [&](GemvUnit<MT, SCALED>& cur, uint32_t mAj, uint32_t mBj, uint32_t mAn, uint32_t mBn, int j) {
-                // The table entries know how many bits their survivors take: no population count per unit (two 7B blocks, one
-                // token 148.8 -> 147.0 us).  With two accumulator sets the wait for the entries shows (182.1 -> 182.5 us).
-                constexpr bool FROM_TABLE = MT == 1;
+                // The table entries know how many bits their survivors take: no population count per unit.  One accumulator set, one
+                // token: 14336 x 4096 19.97 -> 19.70 us (4 bit), 20.99 both (3 bit), 19.35 -> 19.18 (2 bit).  With two sets the wait
+                // for the entries shows at 4 bit (14336 x 4096, 16 tokens 24.45 with counts, 24.54 from the table; 41.8 / 41.6 at
+                // 21504 x 5376 with 30 % pruned), not below: 3 bit 25.8 -> 25.4, 2 bit 24.2 -> 23.9.
+                constexpr bool FROM_TABLE = MT == 1 || BITS < 4;
                 const uint32_t bitA1 = FROM_TABLE ? bitA + cur.ea0.w + cur.ea1.w : bitA + BITS * __popc(mAj & 0xFFFFu);
                 const uint32_t bitB1 = FROM_TABLE ? bitB + cur.eb0.w + cur.eb1.w : bitB + BITS * __popc(mBj & 0xFFFFu);
                 const GemvUnit<MT, SCALED> nxt = load_unit(mAj >> 16, mBj >> 16, bitA1, bitB1, j, 1);
