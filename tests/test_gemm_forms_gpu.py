@@ -5,6 +5,8 @@ bf16 spacing (2^-7 of the magnitude at most) for every rounding - of the product
 magnitudes differ when the bias cancels the product - plus 1e-4 of the largest value for fp32 sums in another order (5e-5
 seen over 14336 columns).
 """
+import re
+
 import pytest
 import torch
 
@@ -101,6 +103,27 @@ def test_fused_launch(M):
     for m, y in zip(mods, fused(x)):
         check(m, x, y)
     assert fused._scratch is not None and fused.device_status() == 0        # the launch's own word: the modules were not called
+
+
+def launched_form(call):
+    """Template arguments of the prompt GEMM's kernel in one call: <bits, CTA pairs, column scale>."""
+    from torch.profiler import ProfilerActivity, profile
+    with profile(activities=[ProfilerActivity.CUDA]) as prof:
+        call()
+        torch.cuda.synchronize()
+    (form,) = {re.search("<(.*?)>", e.key).group(1) for e in prof.key_averages() if "gemm_tcgen05_kernel" in e.key}
+    return form
+
+
+@pytest.mark.parametrize("K,N,T,n", [(512, 512, 150, 5), (2048, 1024, 200, 8), (6144, 1024, 100, 8), (1024, 1024, 40, 8)])
+def test_sums_do_not_depend_on_the_form(K, N, T, n):
+    """``sum_tokens``: the rows of n prompts in one launch get the bits that each prompt gets alone, also where one launch takes CTA
+    pairs and the other single CTAs (all but the last case)."""
+    fused, x = FusedProjections([module(K, N, 4)]), tokens(n * T, N)
+    first = x[:T].contiguous()
+    alone = torch.cat([fused(x[i * T:(i + 1) * T].contiguous())[0] for i in range(n)])
+    assert torch.equal(fused(x, T)[0], alone)
+    assert (launched_form(lambda: fused(x, T)) != launched_form(lambda: fused(first))) == (K != 1024)
 
 
 @pytest.mark.parametrize("how", ["hook", "global hook", "replaced", "subclass"])
