@@ -197,15 +197,22 @@ struct GemmCfg {
 };
 
 // Form (single CTAs, two per SM, or CTA pairs), token tile and split of one launch of `row_tiles` 128-row tiles: the cheapest
-// of all under a cost model in SM clocks, fitted to 770 timed launches (512 .. 28672 rows, 1024 .. 14336 columns, 20 .. 2048 tokens,
-// every form, one to four more token tiles than needed, 1 .. 8 splits; 8 % rms).  Over those shapes its choice is 2.5 % slower
-// than the best launch on average, 20 % at worst (1024 x 4096, 64 tokens: 22.5 us against 18.4).
+// of all under a cost model in SM clocks, fitted to timed launches (512 .. 28672 rows, 1024 .. 14336 columns, 20 .. 2048 tokens, every
+// form, one to four more token tiles than needed, 1 .. 8 splits; 8 % rms with cold weights).  How good its choice is, from a build
+// with -DCOBALT_TUNING_HOOKS, whose keys 2, 4 and 5 name split, form and token tiles: over 25 matrices of 64 x 512 to 28672 x 4096 and
+// 21504 x 5376, 17 .. 2048 tokens (616 cases, warm weights, launches in a graph) it is 5.8 % slower than the best of all on
+// average, 37 % at worst: narrow matrices at few tokens, which one token tile in eight splits does faster (1024 x 4096, 64
+// tokens 17.2 us against 12.8).
 //   per 64-column stage, the largest of: expanding its weights (a CTA that has its SM to itself, one of two, a pair's); MMA
 //   per token; operands through shared memory (A written once and read once per accumulator, B written and read, half of it
 //   per SM in a pair; 128 bytes per clock)
 //   per tile: first loads, drain and epilogue, with the tokens;  split columns: cluster barriers and reduction
 //   clusters of many CTAs do not fill every SM of a GPC: the share that does
+//   singles two to an SM that come in more than one round: the CTAs of a part-filled round start as others end, so such a round
+//   counts by its share as well.  Counted in full, 5376 x 21504 took four splits, which leave most SMs one CTA: 17
+//   tokens, 4 bit 95.9 us, eight splits 82.1; slower in none of the 616 cases.
 constexpr double GEMM_CLK_ALONE = 1280, GEMM_CLK_SHARED = 990, GEMM_CLK_PAIR = 1150, GEMM_CLK_MMA_TOKEN = 2.74, GEMM_CLK_SMEM = 1.56 / 128;
+constexpr double GEMM_FULL_ROUND = 0.6;
 constexpr double GEMM_CLK_TILE = 12000, GEMM_CLK_TILE_TOKEN = 47, GEMM_CLK_SPLIT = 1700, GEMM_CLK_SPLIT_TOKEN = 9.5;
 
 // `only_splits` > 0: that split, whatever it costs (the order of the sums is the caller's choice)
@@ -244,7 +251,8 @@ int gemm_config(int row_tiles, int G, int M, int num_sms, GemmCfg* c, int only_s
                 if (clk < GEMM_CLK_MMA_TOKEN * tpc) clk = GEMM_CLK_MMA_TOKEN * tpc;
                 if (clk < smem) clk = smem;
                 const double stages = 2.0 * ((G + splits - 1) / splits), tile = GEMM_CLK_TILE + GEMM_CLK_TILE_TOKEN * tpc;
-                double cost = alone ? ceil(ctas / sms) * (stages * clk + tile) : ceil(ctas / (2.0 * sms)) * (2.0 * stages * clk + tile);
+                const double rounds = ctas / (2.0 * sms), paired = GEMM_FULL_ROUND * ceil(rounds) + (1.0 - GEMM_FULL_ROUND) * rounds;
+                double cost = alone ? ceil(ctas / sms) * (stages * clk + tile) : (paired > 1.0 ? paired : 1.0) * (2.0 * stages * clk + tile);
                 if (splits > 1) cost += GEMM_CLK_SPLIT * splits + GEMM_CLK_SPLIT_TOKEN * tpc;
                 if (c->tok_per_cta == 0 || cost < best) {
                     best = cost;
