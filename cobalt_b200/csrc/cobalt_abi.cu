@@ -138,9 +138,9 @@ int gemv_config(const GemvGeom& g, int N, int M, int num_sms, GemvCfg* c) {
     c->total_warps = (uint32_t)(grid * GEMV_WARPS);
     if ((unsigned long long)(tiles + 1) * TILE_WORDS * (unsigned long long)grid >= (1ull << 32)) return COBALT_ETOOBIG;   // 32-bit partition arithmetic
     c->counters_off = SCRATCH_STATUS_BYTES;
-    // the counters of both kernels live in the first 64 KB behind the status word and their partial sums behind
-    // that, so that one zero-initialised buffer can serve GEMV and GEMM calls in any order (each kernel returns
-    // its counters to zero; neither ever sees the other's partial sums where it expects counters)
+    // the counters live in the first 64 KB behind the status word and the partial sums behind that, so that one
+    // zero-initialised buffer can serve GEMV calls of any shape and GEMM calls in any order (the GEMV returns its counters to zero and
+    // never sees partial sums where it expects counters; the GEMM uses the status word only)
     c->partials_off = c->counters_off + round_up((size_t)RB * 4, 256);
     if (c->partials_off < SCRATCH_STATUS_BYTES + SCRATCH_COUNTER_BYTES) c->partials_off = SCRATCH_STATUS_BYTES + SCRATCH_COUNTER_BYTES;
     c->xperm_off = c->partials_off + round_up((size_t)grid * 2 * 4 * c->mt * 32 * sizeof(float), 256);    // one subtotal per CTA and side

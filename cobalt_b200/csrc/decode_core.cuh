@@ -346,6 +346,8 @@ CB_HD void decode16_fast(uint32_t m16, uint32_t& w0, uint32_t& w1, uint32_t& w2,
     }
 }
 
+// 32 positions of a fast segment, by way of nibbles: no kernel's path any more (they use decode8), a second derivation of the same
+// weights that the host test (tests/cpp/test_decode_core.cpp) holds against the literal one.
 template <class LutFn>
 CB_HD void decode32_fast(uint32_t m, uint32_t w0, uint32_t w1, uint32_t w2, uint32_t w3, const SegParams& p,
                          LutFn lut, uint32_t out[16]) {

@@ -378,7 +378,8 @@ class CobaltDecoder:
                 # opt-in for prompts: the library's fused attention (fp32 scores and softmax inside; no [T, S] score
                 # tensor in memory).  It skips the spec's bf16 rounding of scores and probabilities; on a small model the
                 # prefill logits then sit 7e-3 (rel-L2) from the spec against 2e-3 for a change of accumulation order,
-                # which is why it is off by default.
+                # which is why it is off by default.  Nor is it faster where the prompt kernel serves: 2048 tokens through two
+                # 7B-shaped layers take 2405 us with it, 2381 us without.
                 ctx = F.scaled_dot_product_attention(q.view(1, T, nh, D).transpose(1, 2), Kc.unsqueeze(0), Vc.unsqueeze(0),
                                                      attn_mask=allowed_of[self.types[i]], scale=scale, enable_gqa=True)
                 ctx = ctx.transpose(1, 2).reshape(T, nh * D)

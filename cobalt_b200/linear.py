@@ -166,7 +166,7 @@ class CobaltSparseLinear(nn.Module):
             need = lib.cobalt_gemm_scratch_bytes(ctypes.byref(d), M)
         if need == 0:
             raise _lib.CobaltError("cobalt_*_scratch_bytes", -1, "could not size the scratch buffer")
-        # one buffer per kernel kind: the GEMV buffer has a fixed size (see above), the GEMM buffer grows with M
+        # one buffer per kernel kind, each of a fixed size (the GEMM's is its status word, whatever M): _launch_args keeps the addresses
         kind = "gemv" if M <= GEMV_MAX_TOKENS else "gemm"
         cur = self._scratch.get(kind) if isinstance(self._scratch, dict) else None
         if cur is None or cur.numel() < need + 256 or cur.device != self.packed.device:
@@ -364,7 +364,7 @@ class FusedProjections:
         if self._scratch is None or self._scratch.numel() < need + 256 or self._scratch.device != device:
             self._scratch = torch.zeros(need + 256, dtype=torch.uint8, device=device)
         self._args = (descs, (ctypes.c_int64 * n)(*[m.out_features for m in self.mods]), *_scratch_span(self._scratch))
-        self._key = [(m._img_meta, m._buffers["packed"].data_ptr()) for m in self.mods]      # held, so that neither can be reused
+        self._key = [(m._img_meta, m._buffers["packed"].data_ptr()) for m in self.mods]      # every image comes with a new _img_meta
         return self._args
 
     def __call__(self, x: torch.Tensor, sum_tokens: int = 0):
