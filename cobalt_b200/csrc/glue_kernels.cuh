@@ -323,11 +323,11 @@ __global__ void swiglu_kernel(const uint16_t* g, const uint16_t* u, uint16_t* ou
 
 // the same over 16-byte chunks (n a multiple of 8, everything 16-byte aligned): value by value the loads and stores were the cost,
 // 2048 x 14336 values 120 -> 67 us, and the one-conversion rounding of staged_input.cuh took it from there
-__global__ void __launch_bounds__(256) swiglu_chunks_kernel(const uint4* __restrict__ g, const uint4* __restrict__ u, uint4* __restrict__ out,
-                                                            long long chunks, int act) {
+// (out may be gate or up: a thread reads its chunk before it writes it)
+__global__ void __launch_bounds__(256) swiglu_chunks_kernel(const uint4* g, const uint4* u, uint4* out, long long chunks, int act) {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < chunks) out[i] = glu_chunk(__ldg(g + i), __ldg(u + i), act);
+    if (i < chunks) out[i] = glu_chunk(g[i], u[i], act);
 }
 
 // ----------------------------------------------------------------------------- greedy token

@@ -292,7 +292,7 @@ int cobalt_pack_tiles(const uint8_t* keep, const uint8_t* q, const void* scale, 
  *                        bf16(x * rsqrt(mean_D(x^2) + eps) * (1 + w)) (src/cobaltkernel/ref_gemma3.py:181-185).
  *                        cache_seq_stride (elements): token t writes at cache + t * cache_seq_stride - 0 when the T tokens
  *                        belong to one sequence, the size of one sequence's cache when T sequences decode one token each.
- *   cobalt_swiglu      : out = act(gate) * up over n elements; act 0 = SiLU, act 1 = GELU (tanh approximation).
+ *   cobalt_swiglu      : out = act(gate) * up over n elements; act 0 = SiLU, act 1 = GELU (tanh approximation); out may be gate or up.
  *   cobalt_attn_decode : grouped-query attention of one new token (q [n_heads*D], already rotated) over the caches
  *                        [n_kv_heads][max_ctx][D]; slots 0..positions[0] are attended (positions[0] is read on the device;
  *                        window > 0 keeps only the last `window` slots); out [n_heads*D].  Rounding points of

@@ -56,6 +56,17 @@ def test_gated_activation_in_chunks_equals_value_by_value(n, act):
     assert torch.equal(outs[0].view(torch.int16), outs[1].view(torch.int16))
 
 
+@pytest.mark.parametrize("n", [8000, 8001])
+@pytest.mark.parametrize("target", [0, 1])
+def test_gated_activation_in_place(n, target):
+    """The result may take the place of either input, whichever kernel runs."""
+    lib = _lib.load()
+    g, u, out = rand(n, seed=1, gain=3.0), rand(n, seed=2), torch.empty(n, dtype=torch.bfloat16, device="cuda")
+    assert lib.cobalt_swiglu(g.data_ptr(), u.data_ptr(), out.data_ptr(), n, 0, stream()) == 0
+    assert lib.cobalt_swiglu(g.data_ptr(), u.data_ptr(), (g, u)[target].data_ptr(), n, 0, stream()) == 0
+    assert torch.equal((g, u)[target], out)
+
+
 @pytest.mark.parametrize("rows,V", [(1, 1), (1, 7), (3, 8), (2, 4095), (1, 32000), (16, 32000), (2, 262144), (5, 1001)])
 def test_argmax_matches_torch(rows, V):
     lib = _lib.load()
