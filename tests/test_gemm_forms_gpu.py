@@ -183,3 +183,35 @@ def test_almost_full_tile_in_a_launch_for_full_ones(missing):
     m._desc = None
     exact = x.double() @ W64.double().t()
     assert bool(((m(x).double() - exact).abs() <= exact.abs() * 2.0 ** -7 + exact.abs().max() * 1e-4).all())
+
+
+def test_modules_saved_whole_before_launches_were_kept():
+    """Objects of an earlier version, restored with the attributes they had then, run and report their status."""
+    import io
+    m, x = module(128, 640, 4), tokens(40, 640)
+    want = m(x), m(x[:3])
+    old = module(128, 640, 4)
+    for name in ("_launch",):
+        del old.__dict__[name]
+    buf = io.BytesIO()
+    torch.save(old, buf)
+    buf.seek(0)
+    again = torch.load(buf, weights_only=False)
+    assert torch.equal(again(x), want[0]) and torch.equal(again(x[:3]), want[1]) and again.device_status() == 0
+    fused = FusedProjections.__new__(FusedProjections)
+    fused.__dict__.update(mods=[again], _scratch=None, _arrays=None)
+    assert fused.device_status() == 0
+    assert torch.equal(fused(x[:3])[0], want[1]) and torch.equal(fused(x)[0], want[0]) and fused.device_status() == 0
+
+
+def test_very_many_tokens():
+    """More token tiles of the single form than a grid has rows: the pair form takes them.  (4.3 GB of activations.)"""
+    M, N, K = 65535 * 256 + 300, 128, 16
+    m, few = module(K, N, 4), tokens(300, N)
+    x = torch.zeros(M, N, dtype=torch.bfloat16, device="cuda")
+    x[:300], x[-300:] = few, few
+    y = m(x)
+    assert m.device_status() == 0 and y.shape == (M, K)
+    check(m, few, y[:300])
+    check(m, few, y[-300:])
+    assert not bool(y[300:-300].any())
