@@ -208,9 +208,12 @@ struct GemmCfg {
 //   per SM in a pair; 128 bytes per clock)
 //   per tile: first loads, drain and epilogue, with the tokens;  split columns: cluster barriers and reduction
 //   clusters of many CTAs do not fill every SM of a GPC: the share that does
-//   singles two to an SM that come in more than one round: the CTAs of a part-filled round start as others end, so such a round
-//   counts by its share as well.  Counted in full, 5376 x 21504 took four splits, which leave most SMs one CTA: 17
-//   tokens, 4 bit 95.9 us, eight splits 82.1; slower in none of the 616 cases.
+//   singles two to an SM, all tokens in one tile, columns split, that come in one round and part of a second: the CTAs of the second
+//   start as others end, so it counts by its share as well.  Counted in full, 5376 x 21504 took four splits, which leave most
+//   SMs one CTA: 17 tokens, 4 bit 97.1 us, eight splits 82.3.  Of 3000 matrices and token counts drawn over 64 .. 21504 rows, 512
+//   .. 21504 columns and 17 .. 2048 tokens this moves 47, by 8 % to the faster side on average; one got slower (19126 x 5632, 70
+//   tokens 85.2 -> 89.1).  Without the limit to one tile and split columns it took others from the pairs, which were the
+//   faster: 15596 x 1024, 789 tokens 52.7 -> 64.2.
 constexpr double GEMM_CLK_ALONE = 1280, GEMM_CLK_SHARED = 990, GEMM_CLK_PAIR = 1150, GEMM_CLK_MMA_TOKEN = 2.74, GEMM_CLK_SMEM = 1.56 / 128;
 constexpr double GEMM_FULL_ROUND = 0.6;
 constexpr double GEMM_CLK_TILE = 12000, GEMM_CLK_TILE_TOKEN = 47, GEMM_CLK_SPLIT = 1700, GEMM_CLK_SPLIT_TOKEN = 9.5;
@@ -251,8 +254,9 @@ int gemm_config(int row_tiles, int G, int M, int num_sms, GemmCfg* c, int only_s
                 if (clk < GEMM_CLK_MMA_TOKEN * tpc) clk = GEMM_CLK_MMA_TOKEN * tpc;
                 if (clk < smem) clk = smem;
                 const double stages = 2.0 * ((G + splits - 1) / splits), tile = GEMM_CLK_TILE + GEMM_CLK_TILE_TOKEN * tpc;
-                const double rounds = ctas / (2.0 * sms), paired = GEMM_FULL_ROUND * ceil(rounds) + (1.0 - GEMM_FULL_ROUND) * rounds;
-                double cost = alone ? ceil(ctas / sms) * (stages * clk + tile) : (paired > 1.0 ? paired : 1.0) * (2.0 * stages * clk + tile);
+                const double rounds = ctas / (2.0 * sms);
+                const double paired = tok_tiles == 1 && splits > 1 && rounds > 1.0 && rounds < 2.0 ? 2.0 * GEMM_FULL_ROUND + (1.0 - GEMM_FULL_ROUND) * rounds : ceil(rounds);
+                double cost = alone ? ceil(ctas / sms) * (stages * clk + tile) : paired * (2.0 * stages * clk + tile);
                 if (splits > 1) cost += GEMM_CLK_SPLIT * splits + GEMM_CLK_SPLIT_TOKEN * tpc;
                 if (c->tok_per_cta == 0 || cost < best) {
                     best = cost;
